@@ -194,8 +194,9 @@ void porsol_transport::capillary_solve(porsol_solver* P, double* sat, const doub
     cap_bcv.alloc(nhf);
     if (tab) PORSOL_LAUNCH(k_cap_mob<true><<<div_up(nc, TB), TB, 0, s>>>(nc, d_sat, p, rock, cap_mob.p));
     else PORSOL_LAUNCH(k_cap_mob<false><<<div_up(nc, TB), TB, 0, s>>>(nc, d_sat, p, rock, cap_mob.p));
-    const int nfe = int(fe_h.size());
-    if (nfe) launch_face_dS(s, nfe, fe.p, d_sat, d_flux, p, rock, dS.p, status.p);
+    cstate.alloc(size_t(nc) + faces.nbc);
+    launch_cell_state(s, faces, d_sat, p, rtab, cstate.p);
+    launch_face_dS(s, faces, d_flux, cstate.p, p, rtab, dS.p, status.p);
     if (tab)
         PORSOL_LAUNCH(k_cap_source<true><<<div_up(nc, TB), TB, 0, s>>>(nc, cptr.p, cent.p, dS.p, d_inj, d_sat, p, rock,
                                                                      cap_src.p));

@@ -15,7 +15,7 @@
 // geometry factor, n.n) are computed once per transportSolve.  A sub-step with gravity or
 // capillarity is two kernels: face entries compute dS, then each cell gathers its entries' dS
 // in a fixed order (no atomics, deterministic) and updates its saturation with the range check.
-// A viscous-only sub-step is one cell kernel that evaluates its entries' terms itself.
+// A viscous-only sub-step is one cell kernel over inflow lists built once per call.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -33,138 +33,285 @@ namespace {
 
 constexpr int TB = 256;
 
-// UpdateForCell::operator() for one face (EulerUpstreamResidual_impl.hpp:101-291), scalar
-// mobilities evaluated in the upstream cell (the boundary cell on Dirichlet faces)
+// x >= 0 and the range test of an updated saturation on the integer pipe: GB300 issues two FP64
+// operations a clock and SM, so a sub-step's FP64 instructions, comparisons included, set its time.
+__device__ __forceinline__ bool not_negative(double x)
+{
+    const long long b = __double_as_longlong(x);
+    return b >= 0 || (b << 1) == 0;   // +x, +0, -0
+}
+
+// checkAndPossiblyClampSat of one cell; saturations in [0, 1] (one unsigned comparison) need nothing
+__device__ __forceinline__ double checked_sat(double sn, int check, int clamp, int* status)
+{
+    if ((unsigned long long)__double_as_longlong(sn) > 0x3FF0000000000000ull) {
+        if (check || clamp) {
+            if (sn > 1.0 || sn < 0.0) {
+                if (clamp) sn = fmax(fmin(sn, 1.0), 0.0);
+                else if (sn > 1.001 || sn < -0.001) atomicOr(status, ST_SAT_RANGE);
+            }
+        }
+        if (!isfinite(sn)) atomicOr(status, ST_NONFINITE);
+    }
+    return sn;
+}
+
+// Mobilities, capillary pressure and saturation of every cell, and of every Dirichlet entry's boundary
+// saturation in its cell's rock (records nc ..): one table search per cell and sub-step instead of
+// up to four per face, and one 32-byte record per gather of the face kernel.
 template <bool TAB>
-__global__ void k_face_dS(int nfe, const FaceEntry* __restrict__ fe, const double* __restrict__ sat,
-                          const double* __restrict__ flux, TrParams p, RockView R, double* __restrict__ dS,
+__device__ __forceinline__ CellState cell_state(int c, double s, const TrParams& p, const RockTab& R)
+{
+    CellState v;
+    v.s = s;
+    if (TAB) {
+        double dx;
+        const int r = R.cell[c];
+        const double* node = tab_row(R, r, s, dx);
+        v.m0 = fma(node[2], dx, node[1]);
+        v.m1 = fma(node[4], dx, node[3]);
+        v.pc = fma(node[6], dx, node[5]) * R.pcs[c];
+    } else {
+        v.m0 = mob1(s, p.mu1);
+        v.m1 = mob2(s, p.mu2);
+        v.pc = 1e5 * (1.0 - s);
+    }
+    return v;
+}
+
+template <bool TAB>
+__global__ void k_cell_state(int nc, int nbc, const double* __restrict__ sat, const int* __restrict__ bc_cell,
+                             const double* __restrict__ bc_sat, TrParams p, RockTab R, CellState* __restrict__ cs)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < nc) cs[i] = cell_state<TAB>(i, sat[i], p, R);
+    else if (i < nc + nbc) cs[i] = cell_state<TAB>(bc_cell[i - nc], bc_sat[i - nc], p, R);
+}
+
+// UpdateForCell::operator() for one face (EulerUpstreamResidual_impl.hpp:101-291), scalar
+// mobilities evaluated in the upstream cell (the boundary cell on Dirichlet faces, c1 >= nc).
+// FP64-issue bound.  The cells' mobilities come from their records, the mean saturation takes one table
+// search (two where the cells' rocks differ) and a quotient five FP64 operations: a host call of 12
+// sub-steps on 167k cells (500k faces, two rocks, gravity and capillarity) takes 0.91 ms, and took
+// 2.93 ms (211 us per launch of this kernel) with up to eight table values and two divisions per face.
+template <bool TAB>
+__global__ void k_face_dS(int nc, int nfe, const int* __restrict__ fc0, const int* __restrict__ fc1,
+                          const int* __restrict__ fhf, const double* __restrict__ fG, const double* __restrict__ fcapf,
+                          const double* __restrict__ fnn, const double* __restrict__ flux,
+                          const CellState* __restrict__ cs, TrParams p, RockTab R, double* __restrict__ dS,
                           const int* __restrict__ status)
 {
+    chain_wait();
     if (*status) return;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nfe) return;
-    const FaceEntry e = fe[k];
-    const double s0 = sat[e.c0];
-    const double s1 = e.dirichlet ? e.satbc : sat[e.c1];
-    const double q = flux[e.hf];
-    const double G = p.grav ? e.G : 0.0;
-    const int triv = G >= 0.0 ? 0 : 1;
-    const double sup = (q >= 0.0) ? s0 : s1;
-    const int cup = (q >= 0.0) ? e.c0 : e.c1;
-    double m[2];
-    m[triv] = mobp<TAB>(triv, cup, sup, p, R);
-    const double signG = triv == 0 ? -1.0 : 1.0;
-    const double gnt = signG * m[triv] * G;
-    const double supn = (q + gnt >= 0.0) ? s0 : s1;
-    const int cupn = (q + gnt >= 0.0) ? e.c0 : e.c1;
-    const int nt = 1 - triv;
-    m[nt] = mobp<TAB>(nt, cupn, supn, p, R);
-    const double mtinv = 1.0 / (m[0] + m[1]);
-    double d = 0.0;
-    if (p.visc) d += m[0] * mtinv * q * e.nn;
-    if (p.grav && !e.dirichlet) d += m[0] * mtinv * m[1] * G;
-    if (p.cap && e.capf != 0.0) {
-        const double as = 0.5 * (s0 + s1);
-        double a1, a2, cp0, cp1;
+    const int c0 = fc0[k], c1 = fc1[k];
+    const CellState a = cs[c0], b = cs[c1];
+    const double q = flux[fhf[k]];
+    const double G = p.grav ? fG[k] : 0.0;
+    const bool triv0 = not_negative(G);
+    const bool up = not_negative(q);
+    const double mt = triv0 ? (up ? a.m0 : b.m0) : (up ? a.m1 : b.m1);
+    const double shift = mt * G;
+    const bool upn = not_negative(triv0 ? q - shift : q + shift);
+    const double mn = triv0 ? (upn ? a.m1 : b.m1) : (upn ? a.m0 : b.m0);
+    const double m0 = triv0 ? mt : mn, m1 = triv0 ? mn : mt;
+    double drive = p.visc ? q * fnn[k] : 0.0;
+    if (p.grav && c1 < nc) drive = fma(m1, G, drive);
+    double d = quotient(m0, m0 + m1) * drive;
+    const double capf = p.cap ? fcapf[k] : 0.0;
+    if (capf != 0.0) {
+        const double as = 0.5 * (a.s + b.s);
+        double a1, a2;
         if (TAB) {
             // mobilities at the mean saturation averaged over both cells' rocks (:226-236)
-            a1 = 0.5 * (mobp<TAB>(0, e.c0, as, p, R) + mobp<TAB>(0, e.c1, as, p, R));
-            a2 = 0.5 * (mobp<TAB>(1, e.c0, as, p, R) + mobp<TAB>(1, e.c1, as, p, R));
-            cp0 = rock_pc(R, e.c0, s0);
-            cp1 = rock_pc(R, e.c1, s1);
+            const int r0 = R.cell[c0], r1 = R.cell[c1];
+            double dx;
+            const double* node = tab_row(R, r0, as, dx);
+            a1 = fma(node[2], dx, node[1]);
+            a2 = fma(node[4], dx, node[3]);
+            if (r1 != r0) {
+                node = tab_row(R, r1, as, dx);
+                a1 = 0.5 * (a1 + fma(node[2], dx, node[1]));
+                a2 = 0.5 * (a2 + fma(node[4], dx, node[3]));
+            }
         } else {
             a1 = mob1(as, p.mu1);
             a2 = mob2(as, p.mu2);
-            cp0 = 1e5 * (1.0 - s0);
-            cp1 = 1e5 * (1.0 - s1);
         }
-        d += a1 * (1.0 / (a1 + a2)) * a2 * e.capf * (cp1 - cp0);
+        d = fma(quotient(a1 * a2, a1 + a2) * capf, b.pc - a.pc, d);
     }
     dS[k] = d;
 }
 
-// Fractional flow lambda_1 / (lambda_1 + lambda_2), evaluated with the same operations as the
-// viscous term of k_face_dS (m1 * (1 / (m1 + m2))), so the viscous-only sub-step is bitwise equal.
+// Fractional flow lambda_1 / (lambda_1 + lambda_2)
 template <bool TAB>
-__device__ __forceinline__ double frac1(int c, double s, const TrParams& p, const RockView& R)
+__device__ __forceinline__ double frac1(int c, double s, const TrParams& p, const RockTab& R)
 {
-    const double m0 = mobp<TAB>(0, c, s, p, R), m1 = mobp<TAB>(1, c, s, p, R);
-    return m0 * (1.0 / (m0 + m1));
+    if (TAB) {
+        double dx;
+        const double* node = tab_row(R, R.cell[c], s, dx);
+        const double m0 = fma(node[2], dx, node[1]);
+        return quotient(m0, m0 + fma(node[4], dx, node[3]));
+    }
+    // both mobilities times mu2: s^2 mu2 / mu1 and (1 - s)^2
+    const double m0 = (s * s) * p.mratio, u = 1.0 - s;
+    return quotient(m0, fma(u, u, m0));
 }
 
+// fractional flows of the cells and of the Dirichlet entries' boundary saturations (nc ..)
 template <bool TAB>
-__global__ void k_frac_init(int nc, const double* __restrict__ sat, TrParams p, RockView R, double* __restrict__ frac)
+__global__ void k_frac_init(int nc, int nbc, const double* __restrict__ sat, const int* __restrict__ bc_cell,
+                            const double* __restrict__ bc_sat, TrParams p, RockTab R, double* __restrict__ frac,
+                            double* __restrict__ frac2)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < nc) {
+        frac[i] = frac1<TAB>(i, sat[i], p, R);
+    } else if (i < nc + nbc) {
+        const double f = frac1<TAB>(bc_cell[i - nc], bc_sat[i - nc], p, R);
+        frac[i] = f;
+        frac2[i] = f;
+    }
+}
+
+// Position of the t-th inflow entry of this lane's cell among its warp's: entry t of all 32 cells that
+// have one lie next to each other (no padding), so the loads of a warp stay coalesced.
+__device__ __forceinline__ int packed_slot(unsigned mask, int base)
+{
+    return base + __popc(mask & ((1u << (threadIdx.x & 31)) - 1u));
+}
+
+// The fluxes of a transportSolve are fixed, and so is every face's upstream cell without gravity and
+// capillarity: with the rates divided by the pore volume and scaled by dt, a sub-step is
+//   s_c += out_c f(s_c) + sum over the inflow faces of coef f(s_upstream).
+// This kernel splits each cell's entries once per call: out[c] sums the faces whose upstream cell is c,
+// the others (about half) become (upstream record, coefficient) pairs, cnt[c] of them, packed per warp
+// from the first entry of the warp's 32 cells on (the entry range is an upper bound, so no scan).
+__global__ void k_inflow_build(int nc, const int* __restrict__ cptr, const int* __restrict__ cent,
+                               const int* __restrict__ fc0, const int* __restrict__ fc1, const int* __restrict__ fhf,
+                               const double* __restrict__ fnn, const double* __restrict__ flux,
+                               const double* __restrict__ ipv, double dt, double* __restrict__ out,
+                               int* __restrict__ cnt, int* __restrict__ src, double* __restrict__ coef)
 {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < nc) frac[c] = frac1<TAB>(c, sat[c], p, R);
+    const bool row = c < nc;
+    const int first = min(c & ~31, nc - 1);
+    int pos = cptr[first];
+    const int b = row ? cptr[c] : 0, e = row ? cptr[c + 1] : 0;
+    const double scale = row ? dt * ipv[c] : 0.0;
+    // upstream record of entry x as seen from this cell: the face's c0 for q >= 0, its c1 otherwise
+    // (a face whose two cells are this one is an outflow face)
+    double own = 0.0;
+    int n = 0;
+    for (int q = b; q < e; ++q) {
+        const int x = cent[q], k = x >= 0 ? x : ~x;
+        const double qf = flux[fhf[k]];
+        const int up = qf >= 0.0 ? fc0[k] : fc1[k];
+        if (up == c) own += x >= 0 ? qf * fnn[k] : -(qf * fnn[k]);
+        else ++n;
+    }
+    if (row) {
+        out[c] = own * scale;
+        cnt[c] = n;
+    }
+    int q = b;
+    for (int t = 0;; ++t) {
+        const unsigned m = __ballot_sync(0xffffffffu, n > t);
+        if (m == 0u) break;
+        if (n > t) {
+            for (;; ++q) {   // the next inflow entry: there are n of them
+                const int x = cent[q], k = x >= 0 ? x : ~x;
+                const double qf = flux[fhf[k]];
+                const int up = qf >= 0.0 ? fc0[k] : fc1[k];
+                if (up == c) continue;
+                const int at = packed_slot(m, pos);
+                src[at] = up;
+                coef[at] = (x >= 0 ? qf * fnn[k] : -(qf * fnn[k])) * scale;
+                ++q;
+                break;
+            }
+        }
+        pos += __popc(m);
+    }
 }
 
-// Fractional flow of each Dirichlet entry's boundary saturation, in its cell's rock
+// One viscous-only sub-step (no gravity driving force, no capillary term) over the inflow lists.
+// FP64-issue bound (two FP64 operations a clock and SM): per cell one product per inflow face, one for
+// the outflow, four for the two mobilities and five for their quotient; the comparisons are integer.
+// Fractional flows are read from frac_in and the updated cell's written to frac_out (a neighbour may
+// still read the old value); the boundary records behind the cells' never change.  A 1M-cell sub-step
+// takes 34.5 us (FP64 pipe 83 % busy, DRAM 2.1 TB/s); evaluating every face from its flux and normal in
+// both its cells, with a division per cell, took 73 us.
+constexpr int INFLOW_UNROLL = 6;
 template <bool TAB>
-__global__ void k_frac_bc(int nfe, const FaceEntry* __restrict__ fe, TrParams p, RockView R, double* __restrict__ fbc)
+__global__ void __launch_bounds__(TB) k_visc_substep(int nc, const int* __restrict__ cptr,
+                                                     const int* __restrict__ cnt, const int* __restrict__ src,
+                                                     const double* __restrict__ coef,
+                                                     const double* __restrict__ out,
+                                                     const double* __restrict__ frac_in,
+                                                     const double* __restrict__ inj, const double* __restrict__ ipv,
+                                                     TrParams p, RockTab R, double dt, int check, int clamp,
+                                                     double* __restrict__ sat, double* __restrict__ frac_out,
+                                                     int* status)
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < nfe && fe[k].dirichlet) fbc[k] = frac1<TAB>(fe[k].c0, fe[k].satbc, p, R);
-}
-
-// One viscous-only sub-step (no gravity driving force, no capillary term) as a single cell
-// kernel.  Both phase mobilities of a face come from the same upstream cell, so its term is
-// f(s_up) q n.n with the fractional flow f precomputed per cell (one FP64 division per cell, not
-// per face), q the flux of the lower cell's half-face.  Every cell evaluates the terms of its own
-// entries in its gather order, then updates as k_cell_update; an entry's term is evaluated by
-// both its cells with the same operations, (f q) (+-n.n) = +-(f q n.n) exactly, so each cell
-// sums exactly what a face-entry pass followed by the gather would give, without the per-entry
-// array written and read back or a second launch per sub-step.  Fractional flows are read from
-// frac_in and the updated cell's written to frac_out (a neighbour may still read the old value).
-template <bool TAB>
-__global__ void k_visc_substep(int nc, const int* __restrict__ cptr, const int* __restrict__ va,
-                               const int* __restrict__ vb, const int* __restrict__ vhf,
-                               const double* __restrict__ vcoef, const double* __restrict__ flux,
-                               const double* __restrict__ frac_in, const double* __restrict__ fbc,
-                               const double* __restrict__ inj, const double* __restrict__ ipv, TrParams p, RockView R,
-                               double dt, int check, int clamp, double* __restrict__ sat,
-                               double* __restrict__ frac_out, int* status)
-{
+    chain_wait();
     if (*status) return;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nc) return;
-    double r = 0.0;
-    for (int q = cptr[c]; q < cptr[c + 1]; ++q) {
-        const double qf = flux[vhf[q]];
-        const int b = vb[q];
-        double f;
-        if (qf >= 0.0) f = frac_in[va[q]];
-        else f = b >= 0 ? frac_in[b] : fbc[~b];
-        r += (f * qf) * vcoef[q];
+    const bool row = c < nc;
+    const int cc = min(c, nc - 1);
+    const int n = row ? cnt[cc] : 0;
+    int pos = cptr[min(c & ~31, nc - 1)];
+    const double s = sat[cc], fo = frac_in[cc], oc = out[cc];
+    int at[INFLOW_UNROLL];
+#pragma unroll
+    for (int t = 0; t < INFLOW_UNROLL; ++t) {
+        const unsigned m = __ballot_sync(0xffffffffu, n > t);
+        at[t] = packed_slot(m, pos);
+        pos += __popc(m);
     }
-    const double s = sat[c];
+    double k[INFLOW_UNROLL], f[INFLOW_UNROLL];
+#pragma unroll
+    for (int t = 0; t < INFLOW_UNROLL; ++t) {
+        k[t] = f[t] = 0.0;
+        if (n > t) {
+            k[t] = coef[at[t]];
+            f[t] = frac_in[src[at[t]]];
+        }
+    }
+    double r = fma(oc, fo, s);
+#pragma unroll
+    for (int t = 0; t < INFLOW_UNROLL; ++t)
+        if (n > t) r = fma(k[t], f[t], r);
+    for (int t = INFLOW_UNROLL;; ++t) {   // cells of many faces
+        const unsigned m = __ballot_sync(0xffffffffu, n > t);
+        if (m == 0u) break;
+        if (n > t) {
+            const int a = packed_slot(m, pos);
+            r = fma(coef[a], frac_in[src[a]], r);
+        }
+        pos += __popc(m);
+    }
+    if (!row) return;
     if (inj) {
         double rate = inj[c];
-        if (rate < 0.0) {
-            const double l1 = mobp<TAB>(0, c, s, p, R), l2 = mobp<TAB>(1, c, s, p, R);
-            rate *= l1 / (l1 + l2);
-        }
-        r += rate;
+        if (rate < 0.0) rate *= fo;
+        r = fma(dt * rate, ipv[c], r);
     }
-    double sn = s + (dt * r) * ipv[c];
-    if (check || clamp) {
-        if (sn > 1.0 || sn < 0.0) {
-            if (clamp) sn = fmax(fmin(sn, 1.0), 0.0);
-            else if (sn > 1.001 || sn < -0.001) atomicOr(status, ST_SAT_RANGE);
-        }
-    }
-    if (!isfinite(sn)) atomicOr(status, ST_NONFINITE);
+    const double sn = checked_sat(r, check, clamp, status);
     sat[c] = sn;
     frac_out[c] = frac1<TAB>(c, sn, p, R);
 }
 
-// residual gather + smallTimeStep update + checkAndPossiblyClampSat
+// residual gather + smallTimeStep update + checkAndPossiblyClampSat, and the cell's record for the
+// next sub-step
 template <bool TAB>
 __global__ void k_cell_update(int nc, const int* __restrict__ cptr, const int* __restrict__ cent,
                               const double* __restrict__ dS, const double* __restrict__ inj,
-                              const double* __restrict__ ipv, TrParams p, RockView R, double dt, int check,
-                              int clamp, double* __restrict__ sat, int* status)
+                              const double* __restrict__ ipv, TrParams p, RockTab R, double dt, int check,
+                              int clamp, double* __restrict__ sat, CellState* __restrict__ cs, int* status)
 {
+    chain_wait();
     if (*status) return;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= nc) return;
@@ -173,26 +320,16 @@ __global__ void k_cell_update(int nc, const int* __restrict__ cptr, const int* _
         const int x = cent[q];
         r += x >= 0 ? dS[x] : -dS[~x];
     }
-    const double s = sat[c];
     if (inj) {
         double rate = inj[c];
-        if (rate < 0.0) {
-            const double l1 = mobp<TAB>(0, c, s, p, R), l2 = mobp<TAB>(1, c, s, p, R);
-            rate *= l1 / (l1 + l2);
-        }
+        if (rate < 0.0) rate *= quotient(cs[c].m0, cs[c].m0 + cs[c].m1);
         r += rate;
     }
     // ipv = 1 / pore volume, precomputed at init: one FP64 division per cell and sub-step saved
     // (the update differs from s + dt r / pv by at most one rounding of the increment)
-    double sn = s + (dt * r) * ipv[c];
-    if (check || clamp) {
-        if (sn > 1.0 || sn < 0.0) {
-            if (clamp) sn = fmax(fmin(sn, 1.0), 0.0);
-            else if (sn > 1.001 || sn < -0.001) atomicOr(status, ST_SAT_RANGE);
-        }
-    }
-    if (!isfinite(sn)) atomicOr(status, ST_NONFINITE);
+    const double sn = checked_sat(sat[c] + (dt * r) * ipv[c], check, clamp, status);
     sat[c] = sn;
+    cs[c] = cell_state<TAB>(c, sn, p, R);
 }
 
 // findCFLtimeVelocity (CflCalculator.hpp:55-88) and findCFLtimeGravity (:91-139) per cell
@@ -333,11 +470,27 @@ void single_rock_cfl(double mu1, double mu2, const RockView* R, int rock, double
 
 namespace porsol {
 
-void launch_face_dS(cudaStream_t s, int nfe, const FaceEntry* fe, const double* sat, const double* flux,
-                    const TrParams& p, const RockView& R, double* dS, const int* status)
+void launch_cell_state(cudaStream_t s, const FaceTables& f, const double* sat, const TrParams& p, const RockTab& R,
+                       CellState* cs)
 {
-    if (R.nrock > 0) PORSOL_LAUNCH(k_face_dS<true><<<div_up(nfe, TB), TB, 0, s>>>(nfe, fe, sat, flux, p, R, dS, status));
-    else PORSOL_LAUNCH(k_face_dS<false><<<div_up(nfe, TB), TB, 0, s>>>(nfe, fe, sat, flux, p, R, dS, status));
+    const int nb = div_up((long long)f.nc + f.nbc, TB);
+    if (R.nrock > 0)
+        PORSOL_LAUNCH(k_cell_state<true><<<nb, TB, 0, s>>>(f.nc, f.nbc, sat, f.bc_cell, f.bc_sat, p, R, cs));
+    else
+        PORSOL_LAUNCH(k_cell_state<false><<<nb, TB, 0, s>>>(f.nc, f.nbc, sat, f.bc_cell, f.bc_sat, p, R, cs));
+    PORSOL_CUDA(cudaGetLastError());
+}
+
+void launch_face_dS(cudaStream_t s, const FaceTables& f, const double* flux, const CellState* cs, const TrParams& p,
+                    const RockTab& R, double* dS, const int* status)
+{
+    if (f.nfe == 0) return;
+    if (R.nrock > 0)
+        chain(k_face_dS<true>, div_up(f.nfe, TB), TB, 0, s, f.nc, f.nfe, f.c0, f.c1, f.hf, f.G, f.capf, f.nn, flux, cs,
+              p, R, dS, status);
+    else
+        chain(k_face_dS<false>, div_up(f.nfe, TB), TB, 0, s, f.nc, f.nfe, f.c0, f.c1, f.hf, f.G, f.capf, f.nn, flux, cs,
+              p, R, dS, status);
 }
 
 }  // namespace porsol
@@ -408,6 +561,7 @@ void porsol_transport::set_rock_tables(const porsol_rock_tables* rt)
     if (!rt) {
         rock = RockView{};
         rock_h = RockView{};
+        rtab = RockTab{};
         compute_cfl_factors();
         return;
     }
@@ -456,7 +610,33 @@ void porsol_transport::set_rock_tables(const porsol_rock_tables* rt)
         const double* K = &perm[9 * size_t(c)];
         rk_skp_h[c] = std::sqrt((K[0] + K[4] + K[8]) / (3 * poro[c]));
     }
+    // the rows as the sub-step kernels read them: ordered keys for the search, and per row its
+    // saturation, the phase mobilities and J with the slopes to the next row (0 in the last row)
+    std::vector<long long> key(m);
+    std::vector<double> node(8 * size_t(m), 0.0);
+    const double iv[2] = {1.0 / fluid.viscosity1, 1.0 / fluid.viscosity2};
+    for (int r = 0; r < nr; ++r)
+        for (int k = rk_pos_h[r]; k < rk_pos_h[r + 1]; ++k) {
+            key[k] = tab_key(rk_s_h[k]);
+            double* d = &node[8 * size_t(k)];
+            const bool last = k + 1 == rk_pos_h[r + 1];
+            const double w = last ? 0.0 : rk_s_h[k + 1] - rk_s_h[k];
+            d[0] = rk_s_h[k];
+            d[1] = rk_krw_h[k] * iv[0];
+            d[3] = rk_kro_h[k] * iv[1];
+            d[5] = rk_J_h[k];
+            if (w > 0.0) {   // equal saturations leave an interval that no search returns
+                d[2] = (rk_krw_h[k + 1] - rk_krw_h[k]) / w * iv[0];
+                d[4] = (rk_kro_h[k + 1] - rk_kro_h[k]) / w * iv[1];
+                d[6] = (rk_J_h[k + 1] - rk_J_h[k]) / w;
+            }
+        }
+    std::vector<double> pcs(nc);
+    for (int c = 0; c < nc; ++c) pcs[c] = rt->use_jfunction_scaling ? rt->sigma_cos_theta / rk_skp_h[c] : 1.0;
     cudaStream_t s = stream;
+    rk_key.upload(key, s);
+    rk_node.upload(node, s);
+    rk_pcs.upload(pcs, s);
     rk_pos.upload(rk_pos_h, s);
     rk_s.upload(rk_s_h, s);
     rk_krw.upload(rk_krw_h, s);
@@ -485,6 +665,7 @@ void porsol_transport::set_rock_tables(const porsol_rock_tables* rt)
     };
     rock = view(true);
     rock_h = view(false);
+    rtab = RockTab{nr, rk_pos.p, rk_key.p, rk_node.p, rk_cell.p, rk_pcs.p};
     compute_cfl_factors();
 }
 
@@ -510,6 +691,7 @@ void porsol_transport::init(const porsol_grid* grid, const double* K, const doub
     if (opts) o = *opts;
     rock = RockView{};   // a new grid drops earlier rock tables
     rock_h = RockView{};
+    rtab = RockTab{};
     compute_cfl_factors();
     hf_cell.resize(nhf);
     int maxbid = 0;
@@ -633,27 +815,38 @@ void porsol_transport::build_entries(const double* grav)
     for (int c = 0; c < nc; ++c) cp[c + 1] = cp[c] + int(cl[c].size());
     ce.reserve(cp[nc]);
     for (int c = 0; c < nc; ++c) ce.insert(ce.end(), cl[c].begin(), cl[c].end());
-    // the same entries seen from each cell, for the single-kernel viscous sub-step
-    std::vector<int> va(ce.size()), vb(ce.size()), vh(ce.size());
-    std::vector<double> vc(ce.size());
-    for (size_t q = 0; q < ce.size(); ++q) {
-        const int x = ce[q], k = x >= 0 ? x : ~x;
-        const FaceEntry& e = fe_h[size_t(k)];
-        va[q] = e.c0;
-        vb[q] = e.dirichlet ? ~k : e.c1;
-        vh[q] = e.hf;
-        vc[q] = x >= 0 ? e.nn : -e.nn;
+    // the faces' factors side by side; a Dirichlet face's second record is its boundary saturation's
+    const size_t nfe = fe_h.size();
+    std::vector<int> f0(nfe), f1(nfe), fh(nfe), bcc;
+    std::vector<double> fg(nfe), fcap(nfe), fn(nfe), bcs;
+    for (size_t k = 0; k < nfe; ++k) {
+        const FaceEntry& e = fe_h[k];
+        f0[k] = e.c0;
+        f1[k] = e.dirichlet ? nc + int(bcc.size()) : e.c1;
+        fh[k] = e.hf;
+        fg[k] = e.G;
+        fcap[k] = e.capf;
+        fn[k] = e.nn;
+        if (e.dirichlet) {
+            bcc.push_back(e.c0);
+            bcs.push_back(e.satbc);
+        }
     }
     any_gravity = false;
     for (const FaceEntry& e : fe_h) any_gravity = any_gravity || e.G != 0.0;
     cudaStream_t s = stream;
-    fe.upload(fe_h, s);
     cptr.upload(cp, s);
     cent.upload(ce, s);
-    ve_a.upload(va, s);
-    ve_b.upload(vb, s);
-    ve_hf.upload(vh, s);
-    ve_coef.upload(vc, s);
+    fe_c0.upload(f0, s);
+    fe_c1.upload(f1, s);
+    fe_hf.upload(fh, s);
+    fe_G.upload(fg, s);
+    fe_capf.upload(fcap, s);
+    fe_nn.upload(fn, s);
+    bc_cell.upload(bcc, s);
+    bc_sat.upload(bcs, s);
+    faces = FaceTables{nc,     int(bcc.size()), int(nfe),  fe_c0.p,   fe_c1.p,  fe_hf.p,
+                       fe_G.p, fe_capf.p,       fe_nn.p,   bc_cell.p, bc_sat.p};
     gflux_hf.upload(ghf, s);
     dS.alloc(std::max<size_t>(fe_h.size(), 1));
     PORSOL_CUDA(cudaStreamSynchronize(s));
@@ -736,47 +929,53 @@ void porsol_transport::solve(double* sat, double time, const double* grav, const
     PORSOL_CUDA(cudaMemcpyAsync(sat0.p, d_sat, nc * sizeof(double), cudaMemcpyDeviceToDevice, s));
     const TrParams p = params(o.method_viscous, o.method_gravity, o.method_capillary);
     const bool tab = rock.nrock > 0;
-    const int nfe = int(fe_h.size());
-    // viscous-only sub-steps use the per-cell fractional flow (same arithmetic, fewer FP64 ops)
+    const int nb = div_up(nc, TB), nbx = div_up((long long)nc + faces.nbc, TB);
+    // without gravity and capillarity every face's upstream cell is fixed by the fluxes
     const bool visc_only = o.method_viscous && !o.method_capillary && (!o.method_gravity || !any_gravity);
     if (visc_only) {
-        frac.alloc(nc);
-        frac2.alloc(nc);
-        fbc.alloc(std::max(nfe, 1));
-        if (nfe) {
-            if (tab) PORSOL_LAUNCH(k_frac_bc<true><<<div_up(nfe, TB), TB, 0, s>>>(nfe, fe.p, p, rock, fbc.p));
-            else PORSOL_LAUNCH(k_frac_bc<false><<<div_up(nfe, TB), TB, 0, s>>>(nfe, fe.p, p, rock, fbc.p));
-        }
+        frac.alloc(size_t(nc) + faces.nbc);
+        frac2.alloc(size_t(nc) + faces.nbc);
+        in_out.alloc(nc);
+        in_cnt.alloc(nc);
+        in_src.alloc(std::max<size_t>(cent.n, 1));
+        in_coef.alloc(std::max<size_t>(cent.n, 1));
+    } else {
+        cstate.alloc(size_t(nc) + faces.nbc);
     }
     int repeats = 0;
     const int max_repeats = 10;
     while (true) {
         if (visc_only) {
-            if (tab) PORSOL_LAUNCH(k_frac_init<true><<<div_up(nc, TB), TB, 0, s>>>(nc, d_sat, p, rock, frac.p));
-            else PORSOL_LAUNCH(k_frac_init<false><<<div_up(nc, TB), TB, 0, s>>>(nc, d_sat, p, rock, frac.p));
+            PORSOL_LAUNCH(k_inflow_build<<<nb, TB, 0, s>>>(nc, cptr.p, cent.p, faces.c0, faces.c1, faces.hf, faces.nn,
+                                                           d_flux, ipv.p, dt, in_out.p, in_cnt.p, in_src.p, in_coef.p));
+            if (tab)
+                PORSOL_LAUNCH(k_frac_init<true><<<nbx, TB, 0, s>>>(nc, faces.nbc, d_sat, faces.bc_cell, faces.bc_sat, p,
+                                                                   rtab, frac.p, frac2.p));
+            else
+                PORSOL_LAUNCH(k_frac_init<false><<<nbx, TB, 0, s>>>(nc, faces.nbc, d_sat, faces.bc_cell, faces.bc_sat, p,
+                                                                    rtab, frac.p, frac2.p));
+            PORSOL_CUDA(cudaGetLastError());
             for (int q = 0; q < n; ++q) {
                 const double* fin = (q & 1) ? frac2.p : frac.p;
                 double* fout = (q & 1) ? frac.p : frac2.p;
                 if (tab)
-                    PORSOL_LAUNCH(k_visc_substep<true><<<div_up(nc, TB), TB, 0, s>>>(
-                        nc, cptr.p, ve_a.p, ve_b.p, ve_hf.p, ve_coef.p, d_flux, fin, fbc.p, d_inj, ipv.p, p, rock, dt,
-                        o.check_sat, o.clamp_sat, d_sat, fout, status.p));
+                    chain(k_visc_substep<true>, nb, TB, 0, s, nc, cptr.p, in_cnt.p, in_src.p, in_coef.p, in_out.p, fin,
+                          d_inj, ipv.p, p, rtab, dt, o.check_sat, o.clamp_sat, d_sat, fout, status.p);
                 else
-                    PORSOL_LAUNCH(k_visc_substep<false><<<div_up(nc, TB), TB, 0, s>>>(
-                        nc, cptr.p, ve_a.p, ve_b.p, ve_hf.p, ve_coef.p, d_flux, fin, fbc.p, d_inj, ipv.p, p, rock, dt,
-                        o.check_sat, o.clamp_sat, d_sat, fout, status.p));
-                if ((q & 255) == 255) PORSOL_CUDA(cudaGetLastError());
+                    chain(k_visc_substep<false>, nb, TB, 0, s, nc, cptr.p, in_cnt.p, in_src.p, in_coef.p, in_out.p, fin,
+                          d_inj, ipv.p, p, rtab, dt, o.check_sat, o.clamp_sat, d_sat, fout, status.p);
             }
-        }
-        for (int q = 0; q < (visc_only ? 0 : n); ++q) {
-            if (nfe) launch_face_dS(s, nfe, fe.p, d_sat, d_flux, p, rock, dS.p, status.p);
-            if (tab)
-                PORSOL_LAUNCH(k_cell_update<true><<<div_up(nc, TB), TB, 0, s>>>(
-                    nc, cptr.p, cent.p, dS.p, d_inj, ipv.p, p, rock, dt, o.check_sat, o.clamp_sat, d_sat, status.p));
-            else
-                PORSOL_LAUNCH(k_cell_update<false><<<div_up(nc, TB), TB, 0, s>>>(
-                    nc, cptr.p, cent.p, dS.p, d_inj, ipv.p, p, rock, dt, o.check_sat, o.clamp_sat, d_sat, status.p));
-            if ((q & 255) == 255) PORSOL_CUDA(cudaGetLastError());
+        } else {
+            launch_cell_state(s, faces, d_sat, p, rtab, cstate.p);
+            for (int q = 0; q < n; ++q) {
+                launch_face_dS(s, faces, d_flux, cstate.p, p, rtab, dS.p, status.p);
+                if (tab)
+                    chain(k_cell_update<true>, nb, TB, 0, s, nc, cptr.p, cent.p, dS.p, d_inj, ipv.p, p, rtab, dt,
+                          o.check_sat, o.clamp_sat, d_sat, cstate.p, status.p);
+                else
+                    chain(k_cell_update<false>, nb, TB, 0, s, nc, cptr.p, cent.p, dS.p, d_inj, ipv.p, p, rtab, dt,
+                          o.check_sat, o.clamp_sat, d_sat, cstate.p, status.p);
+            }
         }
         PORSOL_CUDA(cudaGetLastError());
         int stt = 0;

@@ -10,6 +10,7 @@
 #pragma once
 
 #include <cmath>
+#include <cstring>
 
 namespace porsol {
 
@@ -80,5 +81,68 @@ __host__ __device__ inline double rock_sat(const RockView& R, int c, double pc)
     const double s = tab_value(R.Jx + a, R.sy + a, n, v);
     return fmin(R.s[a + n - 1], fmax(R.s[a], s));
 }
+
+// ---- the tables as the transport sub-steps read them ----
+// GB300 issues two FP64 operations a clock and SM, so these kernels search the rows on the integer pipe
+// and keep one subtraction and one FMA per value: saturations as ordered 64-bit keys, and 8 doubles per
+// row: s, krw / mu1 and its slope to the next row, kro / mu2 and its slope, J and its slope, unused.
+// The mobilities and pressures differ from rock_kr / rock_pc by rounding only.
+struct RockTab {
+    int nrock = 0;                    // 0: no tables
+    const int* pos = nullptr;         // [nrock + 1]
+    const long long* key = nullptr;   // tab_key(s) per row
+    const double* node = nullptr;     // 8 per row
+    const int* cell = nullptr;        // rock of each cell
+    const double* pcs = nullptr;      // per cell factor from J to the capillary pressure
+};
+
+// 64-bit integers in the order of the doubles (-0 before +0, NaN outside)
+__host__ __device__ inline long long tab_key(double v)
+{
+    long long b;
+#ifdef __CUDA_ARCH__
+    b = __double_as_longlong(v);
+#else
+    memcpy(&b, &v, sizeof(b));
+#endif
+    return b ^ ((b >> 63) & 0x7FFFFFFFFFFFFFFFll);
+}
+
+#ifdef __CUDACC__
+// Row of rock r whose interval holds v, and v's distance from its start: 0 outside the table, where the
+// end value holds (NaN for a NaN, which then reaches every value).
+__device__ __forceinline__ const double* tab_row(const RockTab& R, int r, double v, double& dx)
+{
+    const int a = R.pos[r], e = R.pos[r + 1] - 1;
+    const long long k = tab_key(v);
+    int lo = a;
+    const bool nan = ((unsigned long long)__double_as_longlong(v) << 1) > 0xFFE0000000000000ull;
+    dx = nan ? v : 0.0;
+    if (k >= R.key[e]) {
+        lo = e;
+        if (k <= R.key[a]) lo = a;
+    } else if (k > R.key[a]) {
+        int hi = e;
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (R.key[mid] <= k) lo = mid;
+            else hi = mid;
+        }
+        dx = v - R.node[8 * size_t(lo)];
+    }
+    return R.node + 8 * size_t(lo);
+}
+
+// num / den in five FP64 operations: the hardware's reciprocal estimate, one Newton step, and the
+// quotient corrected once by its remainder (Markstein, IBM J. Res. Dev. 34, 1990).
+__device__ __forceinline__ double quotient(double num, double den)
+{
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(den));
+    r = fma(r, fma(-den, r, 1.0), r);
+    const double q = num * r;
+    return fma(fma(-den, q, num), r, q);
+}
+#endif
 
 }  // namespace porsol

@@ -22,6 +22,7 @@ struct FaceEntry {
 struct TrParams {
     double mu1, mu2;   // reciprocal viscosities 1/mu1, 1/mu2
     int visc, grav, cap;
+    double mratio;     // mu2 / mu1 (of the viscosities)
 };
 
 // kr_i / mu_i with the reciprocal viscosities precomputed (FP64 division is a multi-FMA
@@ -37,9 +38,25 @@ __device__ __forceinline__ double mobp(int phase, int c, double s, const TrParam
     return phase == 0 ? mob1(s, p.mu1) : mob2(s, p.mu2);
 }
 
+// the face entries on the device, factor by factor; c1 of a Dirichlet face is its boundary record nc + i
+struct FaceTables {
+    int nc = 0, nbc = 0, nfe = 0;
+    const int *c0 = nullptr, *c1 = nullptr, *hf = nullptr;
+    const double *G = nullptr, *capf = nullptr, *nn = nullptr;
+    const int* bc_cell = nullptr;      // [nbc] cell and saturation of the boundary records
+    const double* bc_sat = nullptr;
+};
+
+// what a face needs of a cell: phase mobilities, capillary pressure, saturation
+struct __align__(32) CellState {
+    double m0, m1, pc, s;
+};
+
+void launch_cell_state(cudaStream_t s, const FaceTables& f, const double* sat, const TrParams& p, const RockTab& R,
+                       CellState* cs);
 // dS of every face entry (UpdateForCell::operator(), EulerUpstreamResidual_impl.hpp:101-291)
-void launch_face_dS(cudaStream_t s, int nfe, const FaceEntry* fe, const double* sat, const double* flux,
-                    const TrParams& p, const RockView& R, double* dS, const int* status);
+void launch_face_dS(cudaStream_t s, const FaceTables& f, const double* flux, const CellState* cs, const TrParams& p,
+                    const RockTab& R, double* dS, const int* status);
 
 }  // namespace porsol
 
@@ -60,14 +77,16 @@ struct porsol_transport {
     std::vector<int> hf_cell;
     std::vector<porsol::FaceEntry> fe_h;
     double grav_cached[3] = {NAN, NAN, NAN};
-    porsol::DBuf<porsol::FaceEntry> fe;
     porsol::DBuf<int> cptr, cent, facepos, status;
-    porsol::DBuf<double> ipv, vol, poro_d, dS, sat0, gflux_hf, in_sat, in_flux, in_inj, frac;
-    // the viscous-only sub-step as one cell kernel: each cell's entries in its gather order (lower
-    // cell, other cell or ~entry for Dirichlet faces, flux half-face, +-n.n), the fractional flow
-    // of the Dirichlet entries, and a second fractional-flow buffer (read one, write the other)
-    porsol::DBuf<int> ve_a, ve_b, ve_hf;
-    porsol::DBuf<double> ve_coef, fbc, frac2;
+    porsol::DBuf<double> ipv, vol, poro_d, dS, sat0, gflux_hf, in_sat, in_flux, in_inj;
+    porsol::FaceTables faces;         // views of the arrays below
+    porsol::DBuf<int> fe_c0, fe_c1, fe_hf, bc_cell;
+    porsol::DBuf<double> fe_G, fe_capf, fe_nn, bc_sat;
+    porsol::DBuf<porsol::CellState> cstate;
+    // the viscous-only sub-step: outflow coefficient and inflow list of each cell (written once per
+    // call), and two fractional-flow buffers (read one, write the other)
+    porsol::DBuf<int> in_cnt, in_src;
+    porsol::DBuf<double> in_out, in_coef, frac, frac2;
     bool any_gravity = false;   // some face entry has a non-zero gravity driving force
     porsol::DBuf<unsigned long long> red;
     porsol::DBuf<double> cfl_part;   // per-block minima of the CFL bounds
@@ -75,6 +94,9 @@ struct porsol_transport {
     // rock tables (porsol_transport_set_rock_tables); rock.nrock == 0 without
     porsol::RockView rock;            // device pointers
     porsol::RockView rock_h;          // the same tables on the host (CFL factors)
+    porsol::RockTab rtab;             // the rows as the sub-step kernels read them
+    porsol::DBuf<long long> rk_key;
+    porsol::DBuf<double> rk_node, rk_pcs;
     std::vector<int> rk_pos_h, rk_cell_h;
     std::vector<double> rk_s_h, rk_krw_h, rk_kro_h, rk_J_h, rk_Jx_h, rk_sy_h, rk_skp_h;
     porsol::DBuf<int> rk_pos, rk_cell;
@@ -93,7 +115,8 @@ struct porsol_transport {
     void build_entries(const double* grav);
     porsol::TrParams params(int visc, int grav, int cap) const
     {
-        return porsol::TrParams{1.0 / fluid.viscosity1, 1.0 / fluid.viscosity2, visc, grav, cap};
+        return porsol::TrParams{1.0 / fluid.viscosity1, 1.0 / fluid.viscosity2, visc, grav, cap,
+                                fluid.viscosity2 / fluid.viscosity1};
     }
     void solve(double* sat, double time, const double* grav, const double* flux, const double* inj,
                porsol_transport_stats* stats, bool dev);
