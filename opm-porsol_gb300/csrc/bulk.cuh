@@ -1,0 +1,62 @@
+// bulk.cuh -- bulk copies into shared memory (cp.async.bulk) completing on an mbarrier, with bounded waits.
+#pragma once
+
+#include "porsol_internal.h"
+
+namespace porsol {
+
+constexpr unsigned long long BULK_WAIT_NS = 20000000ull;  // 20 ms: a copy of a few KB takes microseconds
+constexpr long long BULK_WAIT_TRIES = 1LL << 26;          // backstop should the timer not advance
+
+__device__ __forceinline__ unsigned smem_u32(const void* p) { return unsigned(__cvta_generic_to_shared(p)); }
+
+__device__ __forceinline__ unsigned long long global_ns()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// wait for the barrier's phase of this parity; false when it has not completed within limit_ns
+__device__ __forceinline__ bool mbar_wait_bounded(unsigned bar, unsigned parity, unsigned long long limit_ns)
+{
+    unsigned long long t0 = 0;
+    for (long long it = 0; it < BULK_WAIT_TRIES; ++it) {
+        unsigned ok;
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (ok) return true;
+        const unsigned long long t = global_ns();
+        if (it == 0) t0 = t;
+        else if (t - t0 > limit_ns) return false;
+    }
+    return false;
+}
+
+__device__ __forceinline__ void mbar_init(unsigned bar)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+}
+
+__device__ __forceinline__ void mbar_init_fence()
+{
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+
+__device__ __forceinline__ void mbar_expect(unsigned bar, unsigned bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+
+// both addresses 16-byte aligned, bytes a multiple of 16
+__device__ __forceinline__ void bulk_copy(unsigned dst, const void* src, unsigned bytes, unsigned bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+
+}  // namespace porsol

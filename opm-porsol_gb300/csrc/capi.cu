@@ -354,6 +354,7 @@ void porsol_solver::linear_solve(const porsol_solve_opts& o, porsol_solve_stats&
         st.ms_precond_setup = now_ms() - t_begin;
         x.zero(stream);
         CgResult r = cg64.solve(stream, P, val.p, ilu, rhs.p, x.p, o.residual_tolerance, maxit, &prof, PK_SPMV64);
+        check_ilu_status();
         st.iterations = r.iterations;
         st.reduction = r.reduction;
         count_krylov_bytes(o, r.iterations, 0);
@@ -425,6 +426,12 @@ void porsol_solver::linear_solve(const porsol_solve_opts& o, porsol_solve_stats&
     if (!r.converged) fail(r.iterations, r.reduction);
 }
 
+void porsol_solver::check_ilu_status()
+{
+    if (ilu.solve_status(stream) & ST_TIMEOUT)
+        throw Error(PORSOL_ERR_TIMEOUT, "ILU0 sweep: bulk copy of a step record failed (wait gave up)");
+}
+
 // ILU0-CG (solveLinearSystem, :1387-1420) of a structure whose device numbering differs from the
 // reference's: ILU(0) depends on the order of the unknowns, so the factorisation and the CG run on
 // the system gathered into the reference numbering (same factors, iterates and iteration counts as
@@ -454,6 +461,7 @@ void porsol_solver::ilu_solve_reference_order(const porsol_solve_opts& o, porsol
     x_ref.zero(stream);
     CgResult r = cg64.solve(stream, P, val_ref.p, ilu, rhs_ref.p, x_ref.p, o.residual_tolerance, maxit, &prof,
                             PK_SPMV64);
+    check_ilu_status();
     launch_permute(stream, n, dof_perm_d.p, x_ref.p, x.p, false);
     st.iterations = r.iterations;
     st.reduction = r.reduction;
@@ -520,6 +528,7 @@ void porsol_solver::batched_solve(const porsol_solve_opts& o, porsol_solve_stats
         std::fill(h.begin(), h.end(), o.residual_tolerance);
         upload(btol, h);
         CgResult r = bcg64.solve(stream, P, val.p, *M, batch, rhs.p, x.p, btol.p, maxit);
+        if (o.linsolver_type == 0) check_ilu_status();
         st.iterations = r.iterations;
         st.reduction = r.reduction;
         if (r.breakdown) throw Error(PORSOL_ERR_NONFINITE, "CG breakdown (non-positive curvature)");

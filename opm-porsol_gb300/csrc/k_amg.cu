@@ -13,6 +13,7 @@
 #include <unordered_map>
 
 #include "amg.h"
+#include "bulk.cuh"
 #include "sell.cuh"
 
 namespace porsol {
@@ -891,34 +892,6 @@ __global__ void k_cheb_step(int n, const int* __restrict__ sp, const CI* __restr
 // those of k_cheb_step<T, 0, __half, true> in the same order.  Every wait is bounded: on a timeout
 // the warp sets ST_TIMEOUT, waits once more (bounded) for its copies and returns without writing.
 constexpr int BULK_SLICES = 8;
-constexpr unsigned long long BULK_WAIT_NS = 20000000ull;  // 20 ms: a copy of a few KB takes microseconds
-constexpr long long BULK_WAIT_TRIES = 1LL << 26;          // backstop should the timer not advance
-
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return unsigned(__cvta_generic_to_shared(p)); }
-
-__device__ __forceinline__ unsigned long long global_ns()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// wait for phase 0 of the barrier; false when it has not completed within limit_ns
-__device__ __forceinline__ bool mbar_wait_bounded(unsigned bar, unsigned long long limit_ns)
-{
-    const unsigned long long t0 = global_ns();
-    for (long long it = 0; it < BULK_WAIT_TRIES; ++it) {
-        unsigned ok;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n selp.u32 %0, 1, 0, p;\n}"
-            : "=r"(ok)
-            : "r"(bar)
-            : "memory");
-        if (ok) return true;
-        if (global_ns() - t0 > limit_ns) return false;
-    }
-    return false;
-}
 
 // Dynamic shared memory: 128 bytes for the warps' barriers (per warp one the copies complete on,
 // and one gate used only by the self-test), then BULK_SLICES column areas of cap entries
@@ -965,27 +938,18 @@ __global__ void __launch_bounds__(BULK_SLICES * 32)
     CI* scol = reinterpret_cast<CI*>(smem + 128) + size_t(w) * cap;
     __half* sval = reinterpret_cast<__half*>(smem + 128 + size_t(BULK_SLICES) * cap * CB) + size_t(w) * cap;
     if (lane == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-        if (extra_tx) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gate) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(unsigned(ne) * (CB + 2u))
-                     : "memory");
-        if (extra_tx)
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(gate), "r"(extra_tx)
-                         : "memory");
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                         smem_u32(scol)),
-                     "l"(col4 + e0), "r"(unsigned(ne) * CB), "r"(bar)
-                     : "memory");
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                         smem_u32(sval)),
-                     "l"(a4 + e0), "r"(unsigned(ne) * 2u), "r"(bar)
-                     : "memory");
+        mbar_init(bar);
+        if (extra_tx) mbar_init(gate);
+        mbar_init_fence();
+        mbar_expect(bar, unsigned(ne) * (CB + 2u));
+        if (extra_tx) mbar_expect(gate, extra_tx);
+        bulk_copy(smem_u32(scol), col4 + e0, unsigned(ne) * CB, bar);
+        bulk_copy(smem_u32(sval), a4 + e0, unsigned(ne) * 2u, bar);
     }
     __syncwarp();
-    if (!((extra_tx == 0 || mbar_wait_bounded(gate, BULK_WAIT_NS)) && mbar_wait_bounded(bar, BULK_WAIT_NS))) {
+    if (!((extra_tx == 0 || mbar_wait_bounded(gate, 0, BULK_WAIT_NS)) && mbar_wait_bounded(bar, 0, BULK_WAIT_NS))) {
         if (lane == 0) atomicOr(status, ST_TIMEOUT);
-        mbar_wait_bounded(bar, BULK_WAIT_NS);  // the copies themselves may still be in flight
+        mbar_wait_bounded(bar, 0, BULK_WAIT_NS);  // the copies themselves may still be in flight
         return;
     }
     const int i = s * 32 + lane;

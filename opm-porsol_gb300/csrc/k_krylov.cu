@@ -5,8 +5,11 @@
 // counter + threadfence) adds the partials in block order and updates the CG scalars in
 // device memory.  The summation order is fixed, so results are run-to-run reproducible.
 #include <algorithm>
+#include <climits>
 #include <cmath>
+#include <cstring>
 
+#include "bulk.cuh"
 #include "krylov.h"
 #include "sell.cuh"
 
@@ -500,6 +503,187 @@ __global__ void k_ilu_factor_level(int nrows, const int* __restrict__ rows, cons
     lu[d] = 1.0 / piv;
 }
 
+// The same factorisation of one level with a warp per row (every row at most 32 entries): lane t holds
+// entry t of row i.  The finished rows j < i it needs are read lane by entry, two at a time ahead of
+// their use, and lane t finds its column in row j among the lanes.  Each entry takes the updates of the
+// serial walk in its order.  A level of the 10^3 cube takes about a launch latency instead of the 27 us
+// of one thread walking its row's merges load by load.
+__global__ void __launch_bounds__(128) k_ilu_factor_warp(int nrows, const int* __restrict__ rows,
+                                                         const int* __restrict__ sp, const int* __restrict__ col,
+                                                         const int* __restrict__ rowlen,
+                                                         const int* __restrict__ diag, double* lu, int* status)
+{
+    chain_wait();
+    const int q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (q >= nrows) return;   // whole warps
+    const int lane = threadIdx.x & 31;
+    const int i = rows[q], len = rowlen[i];
+    const int k = sell_slot(sp, i, lane);
+    const int ci = lane < len ? col[k] : INT_MAX;
+    double a = lane < len ? lu[k] : 0.0;
+    const int nl = __popc(__ballot_sync(0xffffffffu, ci < i));   // entries are sorted: the first nl are lower
+    auto fetch = [&](int t, int& cj, double& aj, double& pj) {
+        const int j = __shfl_sync(0xffffffffu, ci, t);
+        const int kj = sell_slot(sp, j, lane);
+        const bool in = lane < rowlen[j];
+        cj = in ? col[kj] : INT_MAX;
+        aj = in ? lu[kj] : 0.0;
+        pj = lu[diag[j]];
+    };
+    int cj = INT_MAX, cn = INT_MAX;
+    double aj = 0.0, an = 0.0, pj = 0.0, pn = 0.0;
+    if (nl > 0) fetch(0, cj, aj, pj);
+    for (int t = 0; t < nl; ++t) {
+        if (t + 1 < nl) fetch(t + 1, cn, an, pn);
+        if (lane == t) a *= pj;                     // L_ij = a_ij * inv(a_jj)
+        const double lij = __shfl_sync(0xffffffffu, a, t);
+        // a_ik -= L_ij a_jk for k > j present in both rows
+        const int lj = __popc(__ballot_sync(0xffffffffu, cj != INT_MAX));
+        for (int u = 0; u < lj; ++u) {
+            const int c = __shfl_sync(0xffffffffu, cj, u);
+            const double v = __shfl_sync(0xffffffffu, aj, u);
+            if (lane > t && lane < len && c == ci) a -= lij * v;
+        }
+        cj = cn;
+        aj = an;
+        pj = pn;
+    }
+    if (ci == i) {
+        if (!(fabs(a) > 0.0) || !isfinite(a)) atomicOr(status, ST_NONFINITE);
+        a = 1.0 / a;
+    }
+    if (lane < len) lu[k] = a;
+}
+
+// the factor's values into the sweep's step records
+__global__ void k_ilu_pack(int nval, const int* __restrict__ pos, const int* __restrict__ slot,
+                           const double* __restrict__ lu, double* __restrict__ blob)
+{
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < nval) blob[pos[e]] = lu[slot[e]];
+}
+
+// Steps [s0, s1) of the sweep by one block: a step is (part of) a level, a thread a row, a barrier ends the
+// step.  What bounds it is the chain from level to level: the operands from shared memory, the row's five
+// dependent FP64 products (a warp's FP64 instruction takes 64 clocks, also when predicated off) and the
+// barrier, 0.57 us in all.  The step records do not depend on the sweep, so a warp of its own brings them
+// into a ring of nst stages by bulk copies ahead of their use.  With SZ the whole vector lives in shared
+// memory, copied in from r and out to z; without, z holds the right-hand side on entry.  The products are
+// added in the row's order, as the per-level kernels do; a padding entry multiplies the 0 behind the
+// vector.  10^3 cube (3300 rows, 84 + 84 levels): one application takes 99 us in one launch, and took 510 us in
+// 168 launches.  Measured and not kept: the records prefetched into registers (130 us), one of the row
+// threads issuing the copies (163 us), each row's operands loaded a step ahead by its own thread (117 us).
+// Every wait is bounded; on a timeout the block sets ST_TIMEOUT, waits (bounded) for its copies and returns.
+constexpr int ILU_ROWS = 256;              // rows of a step at most: a thread each, and one warp that copies
+constexpr int ILU_TB = ILU_ROWS + 32;
+constexpr int ILU_AHEAD = 8;               // products of a row whose operands are loaded before the first sum
+constexpr unsigned ILU_STAGE = 12 * 1024;  // bytes of a stage: the largest step record
+constexpr int ILU_STAGES = 8;
+constexpr size_t ILU_SMEM = 220 * 1024;
+
+// acc - sum over the first W columns of v[k] z[c[k]] for one row (operands cp apart), in column order.  W is
+// the same for the whole step, so the unused products of shorter bodies are not issued at all.
+template <int W, class CI, class Z>
+__device__ __forceinline__ double ilu_row(double acc, const double* v, const CI* c, int cp, Z z)
+{
+    double a[W > 0 ? W : 1], x[W > 0 ? W : 1];
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+        a[k] = v[k * cp];
+        x[k] = z(int(c[k * cp]));
+    }
+#pragma unroll
+    for (int k = 0; k < W; ++k) acc -= a[k] * x[k];
+    return acc;
+}
+
+// Step record: a header (rows, W, upper, -), W columns of cp doubles (cp: rows rounded up to 8), for the
+// upper triangle cp inverted pivots, cp row numbers, W columns of cp column numbers.
+// steps: (offset in the records / 16, bytes).
+template <class CI, bool SZ>
+__global__ void __launch_bounds__(ILU_TB) k_ilu_steps(int s0, int s1, const int2* __restrict__ steps,
+                                                      const unsigned char* __restrict__ blob,
+                                                      const double* __restrict__ r, double* z, int n, int nst,
+                                                      const int* stop, int* status)
+{
+    chain_wait();
+    if (*stop) return;
+    extern __shared__ __align__(128) unsigned char sm[];
+    unsigned char* ring = sm + 128;
+    double* zs = reinterpret_cast<double*>(ring + size_t(nst) * ILU_STAGE);
+    const int i = threadIdx.x;
+    const bool copier = i == ILU_ROWS;
+    const unsigned bars = smem_u32(sm);
+    auto issue = [&](const int2& t, int stage) {
+        mbar_expect(bars + 8 * stage, unsigned(t.y));
+        bulk_copy(smem_u32(ring + size_t(stage) * ILU_STAGE), blob + 16 * size_t(t.x), unsigned(t.y), bars + 8 * stage);
+    };
+    const int2 none = make_int2(0, 0);
+    int2 next = none;
+    if (copier) {
+        for (int k = 0; k < nst; ++k) mbar_init(bars + 8 * k);
+        mbar_init_fence();
+        for (int k = 0; k < nst && s0 + k < s1; ++k) issue(steps[s0 + k], k);
+        next = s0 + nst < s1 ? steps[s0 + nst] : none;
+    }
+    if (SZ) {
+        for (int k = i; k < n; k += ILU_TB) zs[k] = r[k];
+        if (i == 0) zs[n] = 0.0;
+    }
+    auto value = [&](int j) { return SZ ? zs[j] : (j < n ? z[j] : 0.0); };
+    int stage = 0;
+    unsigned parity = 0;
+    __syncthreads();   // barriers initialised, vector in place
+    for (int s = s0; s < s1; ++s) {
+        if (!mbar_wait_bounded(bars + 8 * stage, parity, BULK_WAIT_NS)) {
+            if (copier) {
+                atomicOr(status, ST_TIMEOUT);
+                for (int k = 0; k < nst && s + k < s1; ++k) {   // the copies still in flight
+                    const int g = stage + k;
+                    mbar_wait_bounded(bars + 8 * (g < nst ? g : g - nst), g < nst ? parity : parity ^ 1u, BULK_WAIT_NS);
+                }
+            }
+            return;
+        }
+        const unsigned char* rec = ring + size_t(stage) * ILU_STAGE;
+        const int4 h = *reinterpret_cast<const int4*>(rec);
+        if (i < h.x) {
+            const int W = h.y, up = h.z, cp = (h.x + 7) & ~7;
+            const double* v = reinterpret_cast<const double*>(rec + 16) + i;
+            const CI* rows = reinterpret_cast<const CI*>(rec + 16 + size_t(W + up) * cp * sizeof(double)) + i;
+            const CI* c = rows + cp;
+            const int row = int(*rows);
+            double acc = SZ ? zs[row] : z[row];
+            switch (min(W, ILU_AHEAD)) {
+            case 0: break;
+            case 1: acc = ilu_row<1>(acc, v, c, cp, value); break;
+            case 2: acc = ilu_row<2>(acc, v, c, cp, value); break;
+            case 3: acc = ilu_row<3>(acc, v, c, cp, value); break;
+            case 4: acc = ilu_row<4>(acc, v, c, cp, value); break;
+            case 5: acc = ilu_row<5>(acc, v, c, cp, value); break;
+            case 6: acc = ilu_row<6>(acc, v, c, cp, value); break;
+            case 7: acc = ilu_row<7>(acc, v, c, cp, value); break;
+            default: acc = ilu_row<8>(acc, v, c, cp, value); break;
+            }
+            for (int k = ILU_AHEAD; k < W; ++k) acc -= v[k * cp] * value(int(c[k * cp]));
+            if (up) acc = v[W * cp] * acc;
+            if (SZ) zs[row] = acc;
+            else z[row] = acc;
+        }
+        __syncthreads();
+        if (copier && s + nst < s1) {   // every thread is done with this stage
+            issue(next, stage);
+            next = s + nst + 1 < s1 ? steps[s + nst + 1] : none;
+        }
+        if (++stage == nst) {
+            stage = 0;
+            parity ^= 1u;
+        }
+    }
+    if (SZ)
+        for (int k = i; k < n; k += ILU_TB) z[k] = zs[k];
+}
+
 __global__ void k_ilu_lower_level(int nrows, const int* __restrict__ rows, const int* __restrict__ sp,
                                   const int* __restrict__ col, const int* __restrict__ diag,
                                   const double* __restrict__ lu, const double* __restrict__ r, double* __restrict__ z,
@@ -911,6 +1095,99 @@ void Ilu0::build_levels(const SellPattern& P, cudaStream_t s)
     bucket(ulev, nu, h_uptr_, urows, true);
     lrows_.upload(lrows, s);
     urows_.upload(urows, s);
+    warp_rows_ = true;
+    for (int i = 0; i < n; ++i) warp_rows_ = warp_rows_ && P.h_rowlen[i] <= 32;
+    // The fused sweep: step records of at most ILU_ROWS rows of one level and ILU_STAGE bytes.  The vector
+    // goes to shared memory (16-bit row and column numbers) when all levels are fused and it fits beside
+    // two stages.
+    bool all = true;
+    for (const std::vector<int>* ptr : {&h_lptr_, &h_uptr_})
+        for (size_t l = 0; l + 1 < ptr->size(); ++l) all = all && (*ptr)[l + 1] - (*ptr)[l] <= FUSE_ROWS;
+    const size_t zbytes = (size_t(n) + 1) * sizeof(double);
+    shared_z_ = all && n < 65535 && 128 + zbytes + 2 * size_t(ILU_STAGE) <= ILU_SMEM;
+    stages_ = shared_z_ ? std::min<int>(ILU_STAGES, int((ILU_SMEM - 128 - zbytes) / ILU_STAGE)) : ILU_STAGES;
+    const size_t ib = shared_z_ ? 2 : 4;
+    std::vector<int2> steps;
+    std::vector<unsigned char> blob;
+    std::vector<int> pos, from;
+    runs_.clear();
+    auto bytes_of = [&](int cnt, int w, int up) {
+        const size_t cp = size_t(cnt + 7) / 8 * 8;
+        return 16 + ((w + up) * sizeof(double) + (w + 1) * ib) * cp;
+    };
+    auto add = [&](const std::vector<int>& ptr, const std::vector<int>& rows, int up) {
+        auto in = [&](int i, int j) { return up ? j > i : j < i; };
+        auto length = [&](int i) {
+            int m = 0;
+            for (int t = 0; t < P.h_rowlen[i]; ++t) m += in(i, P.h_col[slot(i, t)]);
+            return m;
+        };
+        for (int l = 0; l + 1 < int(ptr.size()); ++l) {
+            if (ptr[l + 1] - ptr[l] > FUSE_ROWS) {
+                runs_.push_back({false, l, up});
+                continue;
+            }
+            if (runs_.empty() || !runs_.back().fused) runs_.push_back({true, int(steps.size()), int(steps.size())});
+            for (int b = ptr[l]; b < ptr[l + 1];) {
+                int cnt = 0, w = 0;
+                while (b + cnt < ptr[l + 1] && cnt < ILU_ROWS) {
+                    const int w1 = std::max(w, length(rows[b + cnt]));
+                    if (cnt > 0 && bytes_of(cnt + 1, w1, up) > ILU_STAGE) break;
+                    w = w1;
+                    ++cnt;
+                }
+                const size_t cp = size_t(cnt + 7) / 8 * 8, at = blob.size(), sz = bytes_of(cnt, w, up);
+                PORSOL_REQUIRE(sz <= ILU_STAGE && at / 16 < (1u << 31), PORSOL_ERR_BAD_ARG, "ILU0: row too long");
+                blob.resize(at + sz, 0);
+                const int head[4] = {cnt, w, up, 0};
+                std::memcpy(blob.data() + at, head, 16);
+                auto number = [&](size_t q, int v) {   // q-th row or column number of the record
+                    unsigned char* d = blob.data() + at + 16 + (w + up) * cp * sizeof(double) + q * ib;
+                    if (ib == 2) {
+                        const unsigned short h = (unsigned short)v;
+                        std::memcpy(d, &h, 2);
+                    } else {
+                        std::memcpy(d, &v, 4);
+                    }
+                };
+                for (size_t q = 0; q < cp; ++q) {
+                    const int i = q < size_t(cnt) ? rows[b + q] : n;
+                    number(q, i);
+                    int m = 0;
+                    if (i < n)
+                        for (int t = 0; t < P.h_rowlen[i]; ++t) {
+                            const int k = int(slot(i, t)), j = P.h_col[k];
+                            if (!in(i, j)) continue;
+                            number(cp + m * cp + q, j);
+                            pos.push_back(int(at / 8 + 2 + m * cp + q));
+                            from.push_back(k);
+                            ++m;
+                        }
+                    for (; m < w; ++m) number(cp + m * cp + q, n);
+                    if (up && i < n) {
+                        pos.push_back(int(at / 8 + 2 + w * cp + q));
+                        from.push_back(-1 - i);   // the diagonal's slot
+                    }
+                }
+                steps.push_back(make_int2(int(at / 16), int(sz)));
+                runs_.back().b = int(steps.size());
+                b += cnt;
+            }
+        }
+    };
+    add(h_lptr_, lrows, 0);
+    add(h_uptr_, urows, 1);
+    for (int& k : from)
+        if (k < 0) {
+            const int i = -1 - k;
+            for (int t = 0; t < P.h_rowlen[i]; ++t)
+                if (P.h_col[slot(i, t)] == i) k = int(slot(i, t));
+            PORSOL_REQUIRE(k >= 0, PORSOL_ERR_BAD_ARG, "ILU0: missing diagonal");
+        }
+    steps_.upload(steps, s);
+    blob_.upload(blob, s);
+    pos_.upload(pos, s);
+    from_.upload(from, s);
     PORSOL_CUDA(cudaStreamSynchronize(s));
 }
 
@@ -924,9 +1201,18 @@ void Ilu0::factor(cudaStream_t s, const SellPattern& P, const double* val)
     DBuf<int>& status = status_;
     for (size_t l = 0; l + 1 < h_lptr_.size(); ++l) {
         const int cnt = h_lptr_[l + 1] - h_lptr_[l];
-        PORSOL_LAUNCH(k_ilu_factor_level<<<div_up(cnt, 128), 128, 0, s>>>(cnt, lrows_.p + h_lptr_[l], P.slice_ptr.p, P.col.p,
-                                                            P.rowlen.p, P.diag.p, lu_.p, status.p));
+        if (warp_rows_)
+            chain(k_ilu_factor_warp, div_up(cnt, 4), 128, 0, s, cnt, lrows_.p + h_lptr_[l], P.slice_ptr.p, P.col.p,
+                  P.rowlen.p, P.diag.p, lu_.p, status.p);
+        else
+            PORSOL_LAUNCH(k_ilu_factor_level<<<div_up(cnt, 128), 128, 0, s>>>(cnt, lrows_.p + h_lptr_[l],
+                                                                              P.slice_ptr.p, P.col.p, P.rowlen.p,
+                                                                              P.diag.p, lu_.p, status.p));
     }
+    PORSOL_CUDA(cudaGetLastError());
+    if (pos_.n)
+        PORSOL_LAUNCH(k_ilu_pack<<<div_up((long long)pos_.n, RB), RB, 0, s>>>(int(pos_.n), pos_.p, from_.p, lu_.p,
+                                                                             reinterpret_cast<double*>(blob_.p)));
     PORSOL_CUDA(cudaGetLastError());
     int st = 0;
     PORSOL_CUDA(cudaMemcpyAsync(&st, status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -934,18 +1220,40 @@ void Ilu0::factor(cudaStream_t s, const SellPattern& P, const double* val)
     PORSOL_REQUIRE(st == 0, PORSOL_ERR_NONFINITE, "ILU0: zero or non-finite pivot");
 }
 
+int Ilu0::solve_status(cudaStream_t s) const
+{
+    int st = 0;
+    PORSOL_CUDA(cudaMemcpyAsync(&st, status_.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    PORSOL_CUDA(cudaStreamSynchronize(s));
+    return st;
+}
+
 void Ilu0::apply(cudaStream_t s, const double* r, double* z, const int* stop)
 {
     const SellPattern& P = *P_;
-    for (size_t l = 0; l + 1 < h_lptr_.size(); ++l) {
-        const int cnt = h_lptr_[l + 1] - h_lptr_[l];
-        chain(k_ilu_lower_level, div_up(cnt, 128), 128, 0, s, cnt, lrows_.p + h_lptr_[l], P.slice_ptr.p, P.col.p,
-            P.diag.p, lu_.p, r, z, stop);
-    }
-    for (size_t l = 0; l + 1 < h_uptr_.size(); ++l) {
-        const int cnt = h_uptr_[l + 1] - h_uptr_[l];
-        chain(k_ilu_upper_level, div_up(cnt, 128), 128, 0, s, cnt, urows_.p + h_uptr_[l], P.slice_ptr.p, P.col.p,
-            P.rowlen.p, P.diag.p, lu_.p, z, stop);
+    const size_t zbytes = size_t(P.n) * sizeof(double);
+    const size_t shm = 128 + size_t(stages_) * ILU_STAGE + (shared_z_ ? zbytes + sizeof(double) : 0);
+    if (!shared_z_) PORSOL_CUDA(cudaMemcpyAsync(z, r, zbytes, cudaMemcpyDeviceToDevice, s));   // the fused steps start from z
+    for (const Run& u : runs_) {
+        if (u.fused && shared_z_) {
+            PORSOL_CUDA(cudaFuncSetAttribute(k_ilu_steps<unsigned short, true>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, int(ILU_SMEM)));
+            chain(k_ilu_steps<unsigned short, true>, 1, ILU_TB, shm, s, u.a, u.b, steps_.p, blob_.p, r, z, P.n, stages_,
+                  stop, status_.p);
+        } else if (u.fused) {
+            PORSOL_CUDA(cudaFuncSetAttribute(k_ilu_steps<int, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             int(ILU_SMEM)));
+            chain(k_ilu_steps<int, false>, 1, ILU_TB, shm, s, u.a, u.b, steps_.p, blob_.p, r, z, P.n, stages_, stop,
+                  status_.p);
+        } else if (u.b == 0) {
+            const int b = h_lptr_[u.a], cnt = h_lptr_[u.a + 1] - b;
+            chain(k_ilu_lower_level, div_up(cnt, 128), 128, 0, s, cnt, lrows_.p + b, P.slice_ptr.p, P.col.p, P.diag.p,
+                  lu_.p, r, z, stop);
+        } else {
+            const int b = h_uptr_[u.a], cnt = h_uptr_[u.a + 1] - b;
+            chain(k_ilu_upper_level, div_up(cnt, 128), 128, 0, s, cnt, urows_.p + b, P.slice_ptr.p, P.col.p, P.rowlen.p,
+                  P.diag.p, lu_.p, z, stop);
+        }
     }
     PORSOL_CUDA(cudaGetLastError());
 }

@@ -130,20 +130,41 @@ private:
 // ILU(0) with the pivots stored inverted, factor and triangular solves level-scheduled
 // (rows of one level are independent).  The algorithm of dune-istl's SeqILU0 with
 // relaxation 1 (IncompFlowSolverHybrid.hpp:1404).
+//
+// The levels of a mid-size grid hold tens of rows and a sweep has a hundred levels, so a launch per
+// level costs a launch latency per handful of rows.  Runs of levels of at most FUSE_ROWS rows are swept
+// by one block in one launch (k_ilu_steps), from records of the two triangles in sweep order;
+// wider levels, which would wait for one SM's FP64 pipe, keep a launch of their own.
 class Ilu0 : public Precond<double> {
 public:
     void build_levels(const SellPattern& P, cudaStream_t s);   // structure only
     void factor(cudaStream_t s, const SellPattern& P, const double* val);
     void apply(cudaStream_t s, const double* r, double* z, const int* stop) override;
+    // error bits set by apply() (ST_TIMEOUT: a bounded wait for a bulk copy gave up); synchronises the stream
+    int solve_status(cudaStream_t s) const;
     int num_levels_lower() const { return int(h_lptr_.size()) - 1; }
     int num_levels_upper() const { return int(h_uptr_.size()) - 1; }
 
 private:
+    static constexpr int FUSE_ROWS = 1024;
     const SellPattern* P_ = nullptr;
     DBuf<double> lu_;
     std::vector<int> h_lptr_, h_uptr_;
     DBuf<int> lrows_, urows_;
     DBuf<int> status_;
+    bool warp_rows_ = false;   // every row fits a warp (the factorisation then takes one warp per row)
+    // a launch of apply(): steps [a, b) of the fused sweep, or (fused false) level a of the lower (b = 0)
+    // or upper (b = 1) triangle
+    struct Run {
+        bool fused;
+        int a, b;
+    };
+    std::vector<Run> runs_;
+    DBuf<int2> steps_;             // the fused sweep's steps and their records (k_ilu_steps)
+    DBuf<unsigned char> blob_;
+    DBuf<int> pos_, from_;         // value pos_[e] of the records is the factor's slot from_[e]
+    bool shared_z_ = false;        // the sweep's vector lives in shared memory
+    int stages_ = 2;
 };
 
 // Helpers used by the solver front end.

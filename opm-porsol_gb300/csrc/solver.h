@@ -67,6 +67,7 @@ struct porsol_solver {
     // dof permutation, slot sources, values, right-hand side and solution
     porsol::DBuf<int> dof_perm_d, ref_slot_src_d;
     porsol::DBuf<double> val_ref, rhs_ref, x_ref, pi_ref;
+    void check_ilu_status();
     void ilu_solve_reference_order(const porsol_solve_opts& o, porsol_solve_stats& st, int maxit);
     porsol::RedScratch red;
 
