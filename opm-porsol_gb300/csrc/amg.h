@@ -20,6 +20,7 @@
 #include <cuda_fp16.h>
 
 #include "krylov.h"
+#include "tail.h"
 
 namespace porsol {
 
@@ -142,6 +143,14 @@ private:
     double cycle_bytes(int l, std::vector<double>* per_level, bool started = false) const;
     // 1 / theta of the level's Chebyshev interval [lmax / 30, lmax]
     static double cheb_inv_theta(const Level& L) { return 1.0 / (0.5 * (L.lmax + L.lmax / 30.0)); }
+    // The smallest levels as one cluster launch (tail.h): levels tail_ .. nlev_ - 1, -1: none.
+    void choose_tail(cudaStream_t s);
+    void finish_tail(const std::vector<int>& bytes);
+    int tail_ = -1, tail_first_ = -1, tail_shm_ = 0;
+    TailArgs<T> targs_{};
+    DBuf<unsigned char> tail_blob_;
+    // interval of a level's Chebyshev polynomial: 1 / theta and the coefficients of its two steps
+    static void cheb_coefficients(const Level& L, T& inv_theta, T (&c1)[2], T (&c2)[2]);
     DBuf<double> kpart_, kcoef_;   // K-cycle dot partials and coefficients (8 per level)
 
     AmgOpts o_;

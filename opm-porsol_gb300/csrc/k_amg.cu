@@ -1411,6 +1411,7 @@ int read_int(cudaStream_t s, const int* d)
 // keeping at least five entries per lane.  At 121k rows of 42 entries the one-thread-per-row
 // SELL-32x4 step was faster than 4 lanes (13.8 against 15.0 us).
 constexpr long long LANES_FILL_THREADS = 1LL << 18;
+constexpr long long TAIL_ENTRIES_FP16 = 128 * 1024, TAIL_ENTRIES_FP64 = 64 * 1024;   // choose_tail()
 int lanes_for(int n, long long nent)
 {
     const double avg = n > 0 ? double(nent) / n : 0.0;
@@ -1909,11 +1910,16 @@ void Amg<T>::setup(cudaStream_t s, const SellPattern& P0, const T* A0, const Amg
         PORSOL_CUDA(cudaMemsetAsync(L.act.p, 1, L.act.n, s));
     }
     PORSOL_CUDA(cudaGetLastError());
-    // Chebyshev intervals of the smoothed levels and the x4 copies' largest column offsets (one
-    // copy each for all levels)
+    // Chebyshev intervals of the smoothed levels, the x4 copies' largest column offsets and the sizes of
+    // the tail's parts (one copy each for all levels)
+    choose_tail(s);
     {
         std::vector<unsigned long long> gb(size_t(nlev_), 0ULL);
         std::vector<int> mo(size_t(nlev_), 0);
+        std::vector<int> tb(tail_first_ < 0 ? 0 : size_t(nlev_ - 1 - tail_first_) * TAIL_CTAS);
+        if (!tb.empty())
+            PORSOL_CUDA(cudaMemcpy2DAsync(tb.data(), sizeof(int), tail_blob_.p, TAIL_BLOB, sizeof(int), tb.size(),
+                                          cudaMemcpyDeviceToHost, s));
         PORSOL_CUDA(cudaMemcpyAsync(gb.data(), s_gmax_.p, sizeof(unsigned long long) * gb.size(),
                                     cudaMemcpyDeviceToHost, s));
         PORSOL_CUDA(cudaMemcpyAsync(mo.data(), s_maxoff_.p, sizeof(int) * mo.size(), cudaMemcpyDeviceToHost, s));
@@ -1935,6 +1941,7 @@ void Amg<T>::setup(cudaStream_t s, const SellPattern& P0, const T* A0, const Amg
                 L.c16 = false;
             }
         }
+        finish_tail(tb);
     }
     // K-cycle vectors and scalars
     kcoef_.alloc(8 * size_t(std::max(nlev_, 1)));
@@ -1948,8 +1955,91 @@ void Amg<T>::setup(cudaStream_t s, const SellPattern& P0, const T* A0, const Amg
     Level& C = *lv_[nlev_ - 1];
     PORSOL_REQUIRE(C.n <= 2048, PORSOL_ERR_BAD_ARG, "AMG: coarsening stalled above the dense-solve limit");
     build_coarse_solver(s, *C.P, C.A, C.n);
+    targs_.cinv = cinv_.p;
     const int st = read_int(s, status_.p);
     PORSOL_REQUIRE(st == 0, PORSOL_ERR_NONFINITE, "AMG setup: non-positive diagonal or missing diagonal entry");
+}
+
+// Levels a tail may start at: from the last smoothed one up, while rows and entries stay within what the
+// cluster does faster than a launch per phase, never the finest or a K-cycle level.  Eight SMs gather
+// about 8 FP16 entries a clock each: 128k entries are 1 us a phase beside the 1.3 us of its barrier and
+// latencies, against 3 us per launch on a level of that size.  In FP64 (two operations a clock and SM)
+// 64k entries are 2.1 us, against 6 us per launch.  Their parts are written here; finish_tail() keeps as
+// many as the blocks' shared memory holds.  Batched solves keep the launches, which skip converged blocks.
+template <class T>
+void Amg<T>::choose_tail(cudaStream_t s)
+{
+    tail_ = tail_first_ = -1;
+    const int last = nlev_ - 2;
+    if (blk0_ || o_.smooth_steps != 1 || o_.cheb_degree != 2 || last < 1 || lv_[nlev_ - 1]->n > TAIL_DENSE ||
+        lv_[nlev_ - 1]->n < 1 || !tail_fits<T>(lv_[last]->half, TAIL_SMEM))
+        return;
+    const long long most = sizeof(T) == 8 ? TAIL_ENTRIES_FP64 : TAIL_ENTRIES_FP16;
+    int first = nlev_ - 1;
+    while (first - 1 >= 1 && first - 1 > o_.kcycle_levels && last - (first - 1) < TAIL_LEVELS) {
+        const Level& L = *lv_[size_t(first - 1)];
+        if (L.n > TAIL_ROWS || L.P->nent > most || L.v4 || L.half != lv_[size_t(last)]->half) break;
+        --first;
+    }
+    if (first > last) return;
+    tail_first_ = first;
+    tail_blob_.alloc(size_t(last - first + 1) * TAIL_CTAS * TAIL_BLOB);
+    for (int l = first; l <= last; ++l) {
+        const Level& L = *lv_[size_t(l)];
+        const int nn = lv_[size_t(l + 1)]->n;
+        tail_pack<T>(s, L.n, L.P->slice_ptr.p, L.P->col.p, L.P->rowlen.p, L.half ? L.ah.p : nullptr, L.A, L.dinv.p,
+                     L.half ? L.diagv.p : nullptr, L.agg.agg.p, nn, L.agg.ptr.p, L.agg.idx.p, l == last,
+                     tail_blob_.p + size_t(l - first) * TAIL_CTAS * TAIL_BLOB);
+    }
+}
+
+template <class T>
+void Amg<T>::finish_tail(const std::vector<int>& bytes)
+{
+    if (bytes.empty()) return;
+    const int last = nlev_ - 2;
+    for (int first = tail_first_; first <= last && tail_ < 0; ++first) {
+        TailArgs<T> a{};
+        a.levels = last - first + 1;
+        bool fit = true;
+        for (int k = 0; k < a.levels; ++k) {
+            const Level& L = *lv_[size_t(first + k)];
+            a.lv[k].n = L.n;
+            a.lv[k].lanes = tail_lanes(L.n);
+            cheb_coefficients(L, a.lv[k].inv_theta, a.lv[k].c1, a.lv[k].c2);
+            for (int r = 0; r < TAIL_CTAS; ++r)
+                a.part_bytes[k] = std::max(a.part_bytes[k], bytes[size_t(first + k - tail_first_) * TAIL_CTAS + r]);
+            fit = fit && a.part_bytes[k] <= TAIL_BLOB;
+        }
+        a.nd = lv_[size_t(nlev_ - 1)]->n;
+        if (!fit) continue;
+        tail_shm_ = tail_layout(a);
+        if (tail_shm_ > TAIL_SMEM) continue;
+        const Level& F = *lv_[size_t(first - 1)];
+        a.blob = tail_blob_.p + size_t(first - tail_first_) * TAIL_CTAS * TAIL_BLOB;
+        a.rptr = F.agg.ptr.p;
+        a.ridx = F.agg.idx.p;
+        a.rfine = F.r.p;
+        a.x = lv_[size_t(first)]->x.p;
+        a.wp = T(o_.prolong);
+        targs_ = a;
+        tail_ = first;
+    }
+}
+
+template <class T>
+void Amg<T>::cheb_coefficients(const Level& L, T& inv_theta, T (&c1)[2], T (&c2)[2])
+{
+    const double theta = 0.5 * (L.lmax + L.lmax / 30.0), delta = 0.5 * (L.lmax - L.lmax / 30.0);
+    const double sigma = theta / delta;
+    double rho = 1.0 / sigma;
+    inv_theta = T(1.0 / theta);
+    for (int k = 0; k < 2; ++k) {
+        const double rho1 = 1.0 / (2.0 * sigma - rho);
+        c1[k] = T(rho1 * rho);
+        c2[k] = T(2.0 * rho1 / delta);
+        rho = rho1;
+    }
 }
 
 template <class T>
@@ -2090,13 +2180,17 @@ void Amg<T>::vcycle(cudaStream_t s, int l, const T* b, T* x, const int* stop, bo
     // the coarse level's cycle starts with a Chebyshev start from zero on Nx.b (its first cycle
     // under a K-cycle): done here, in the restriction; the coarsest level solves directly
     const bool fuse = l + 1 < nlev_ - 1;
-    if (fuse)
+    if (l + 1 == tail_) {   // the levels below in one launch, their restriction included
+        targs_.stop = stop;
+        tail_launch<T>(s, lv_[size_t(tail_)]->half, targs_, tail_shm_);
+    } else if (fuse)
         chain(k_restrict_start0<T>, div_up(Nx.n, TB), TB, 0, s, Nx.n, L.agg.ptr.p, L.agg.idx.p, L.r.p, Nx.b.p,
             Nx.dinv.p, Nx.r.p, Nx.d0.p, T(cheb_inv_theta(Nx)), stop, level_act(Nx));
     else
         chain(k_restrict<T>, div_up(Nx.n, TB), TB, 0, s, Nx.n, L.agg.ptr.p, L.agg.idx.p, L.r.p, Nx.b.p, stop,
             level_act(Nx));
-    if (k_level(l + 1)) kcycle(s, l + 1, Nx.b.p, Nx.x.p, stop, fuse);
+    if (l + 1 == tail_) {
+    } else if (k_level(l + 1)) kcycle(s, l + 1, Nx.b.p, Nx.x.p, stop, fuse);
     else vcycle(s, l + 1, Nx.b.p, Nx.x.p, stop, fuse);
     // post-smoothing from t + w P xc
     chebyshev(s, L, b, x, false, Nx.x.p, L.agg.agg.p, stop);
@@ -2151,6 +2245,12 @@ double Amg<T>::cycle_bytes(int l, std::vector<double>* per_level, bool started) 
     }
     const Level& L = *lv_[l];
     const double n = L.n, nc = lv_[l + 1]->n;
+    if (tail_ >= 0 && l >= tail_) {   // entries with 16-bit columns once; the first level's restriction and result
+        b = double(L.P->nent) * ((L.half ? 2.0 : sx) + 2.0) + 2.0 * n * sx +
+            (l == tail_ ? n * (4.0 + sx) + lv_[size_t(l - 1)]->n * (4.0 + sx) : 0.0);
+        if (per_level) (*per_level)[size_t(l)] += b;
+        return b + cycle_bytes(l + 1, per_level, false);
+    }
     const double vb = L.half ? 2.0 : sx, cb = ((L.v4 && L.c16) || plain16(L)) ? 2.0 : 4.0;
     const double mat = double(L.P->nent) * (vb + cb);
     const int deg = std::max(1, o_.cheb_degree);
@@ -2168,7 +2268,7 @@ double Amg<T>::cycle_bytes(int l, std::vector<double>* per_level, bool started) 
     b += (started ? 3.0 : 4.0) * n * sx + steps(true);
     b += (o_.smooth_steps - 1) * (start + steps(false));
     b += mat + n * sx * (L.half ? 4.0 : 3.0);            // residual
-    b += n * (sx + 4.0) + nc * (4.0 + sx);               // restriction
+    if (l + 1 != tail_) b += n * (sx + 4.0) + nc * (4.0 + sx);   // restriction
     const bool fuse = l + 1 < nlev_ - 1;                 // the coarse start is done by the restriction
     if (L.lanes == 1)                                    // post-smoothing from t + w P xc
         b += n * (2.0 * sx + 4.0) + nc * sx + start;
