@@ -19,6 +19,7 @@
 
 #include <cuda_fp16.h>
 
+#include "aggregate.h"
 #include "krylov.h"
 #include "tail.h"
 
@@ -55,6 +56,10 @@ int bulk_step_selftest(bool expire, float* r, float* d, float* x);
 struct Aggregates {
     int n = 0, nc = 0;
     DBuf<int> agg, ptr, idx;
+    // set by the round that wrote the Galerkin candidate offsets too: candidates in all, and of one
+    // aggregate at most
+    bool offsets = false;
+    int total = 0, bound = 0;
 };
 
 template <class T>
@@ -123,6 +128,8 @@ private:
     void aggregate_round(cudaStream_t s, const SellPattern& P, const T* A, int n, bool neg_first, Aggregates& out);
     void pairwise(cudaStream_t s, const SellPattern& P, const T* A, int n, bool neg, double theta, bool join,
                   Aggregates& out);
+    void aggregate_small(cudaStream_t s, const SellPattern& P, const T* A, int n, bool neg_first, Aggregates& out);
+    void compose(cudaStream_t s, Aggregates& first, const Aggregates& second);
     void members(cudaStream_t s, Aggregates& a);
     void galerkin(cudaStream_t s, const SellPattern& P, const T* A, const Aggregates& a, SellPattern& Pc,
                   DBuf<T>& Ac);

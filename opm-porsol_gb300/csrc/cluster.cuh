@@ -1,0 +1,64 @@
+// cluster.cuh -- thread-block clusters: barriers and stores into the other blocks' shared memory.
+#pragma once
+
+#include "porsol_internal.h"
+
+namespace porsol {
+
+__device__ __forceinline__ unsigned cluster_rank()
+{
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// hardware barrier over all threads of the cluster: remote stores before it are visible after it
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ void cluster_sync()
+{
+    cluster_arrive();
+    cluster_wait();
+}
+// address of this block's shared location `a` in the block of rank r
+__device__ __forceinline__ unsigned map_rank(unsigned a, unsigned r)
+{
+    unsigned d;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(r));
+    return d;
+}
+__device__ __forceinline__ void put(unsigned a, float v)
+{
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+__device__ __forceinline__ void put(unsigned a, double v)
+{
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+
+__device__ __forceinline__ void put(unsigned a, int v)
+{
+    asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+
+// Launch of one cluster of `ctas` blocks, chained (chain()) when pdl.
+template <class... KA, class... A>
+inline void launch_cluster(void (*kernel)(KA...), int ctas, int threads, size_t shm, cudaStream_t s, bool pdl, A&&... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = ctas;
+    cfg.blockDim = threads;
+    cfg.dynamicSmemBytes = shm;
+    cfg.stream = s;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = ctas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = pdl ? 2 : 1;
+    PORSOL_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...));
+    PORSOL_COUNT_LAUNCH();
+}
+
+}  // namespace porsol

@@ -14,6 +14,8 @@
 
 #include "amg.h"
 #include "bulk.cuh"
+#include "cluster.cuh"
+#include "match.cuh"
 #include "sell.cuh"
 
 namespace porsol {
@@ -150,44 +152,6 @@ __global__ void k_diag_rsqrt(int n, const int* __restrict__ diag, const T* __res
     if (i < n) rs[i] = rsqrtf(fabsf(float(A[diag[i]])));
 }
 
-// Symmetric 32-bit hash of an edge {i, j}: equal strengths (common on uniform grids) are
-// ordered by this pseudo-random priority, the same from both endpoints, so locally
-// dominant edges are unique and mutual-best matching pairs most rows in a few sweeps.
-__device__ __forceinline__ unsigned edge_hash(int i, int j)
-{
-    const unsigned lo = unsigned(min(i, j)), hi = unsigned(max(i, j));
-    unsigned x = lo * 0x9E3779B1u + hi * 0x85EBCA77u;
-    x ^= x >> 15;
-    x *= 0x2C1B3C6Du;
-    x ^= x >> 12;
-    x *= 0x297A2D39u;
-    x ^= x >> 15;
-    return x;
-}
-
-// (s, hash) lexicographic comparison with the column as the last key
-__device__ __forceinline__ bool stronger(float s, unsigned h, int j, float bs, unsigned bh, int bj)
-{
-    return s > bs || (s == bs && (h > bh || (h == bh && j < bj)));
-}
-
-// Entry (j, a) of row i as a candidate: kept when its neighbour has the wanted state, its strength
-// s = a' rs_i rs_j (a' = -a for negative couplings, |a| otherwise) passes the floor, and it beats the
-// best so far.  stronger() is a total order, so the best is the same whatever the order of the entries.
-__device__ __forceinline__ void consider(int i, int j, float a, int stj, float rsj, float ri, int want_state,
-                                         bool neg, float floor_s, float& bs, unsigned& bh, int& bj)
-{
-    if (j == i || stj != want_state) return;
-    const float s = (neg ? -a : fabsf(a)) * ri * rsj;
-    if (!(s > 0.0f && s >= floor_s)) return;
-    const unsigned h = edge_hash(i, j);
-    if (bj < 0 || stronger(s, h, j, bs, bh, bj)) {
-        bs = s;
-        bh = h;
-        bj = j;
-    }
-}
-
 // The best candidate over this lane's entries q, q + K, ... of row i.  With one or two lanes per row
 // (long walks per lane) the columns and values of four entries are loaded before their four state
 // and scale gathers: one dependent load chain per four entries instead of one per entry.  More lanes
@@ -243,24 +207,6 @@ __global__ void k_isolated(int n, const int* __restrict__ sp, const int* __restr
     state[i] = iso ? 2 : 0;
     partner[i] = -1;
     join[i] = -1;
-}
-
-// best candidate of K lanes: (strength, hash, column) is a strict total order over the distinct
-// columns of a row, so the reduction gives the one-lane scan's answer in any lane order
-template <int K>
-__device__ __forceinline__ void best_of_lanes(float& bs, unsigned& bh, int& bj)
-{
-#pragma unroll
-    for (int o = K >> 1; o > 0; o >>= 1) {
-        const float s2 = __shfl_xor_sync(0xffffffffu, bs, o);
-        const unsigned h2 = __shfl_xor_sync(0xffffffffu, bh, o);
-        const int j2 = __shfl_xor_sync(0xffffffffu, bj, o);
-        if (j2 >= 0 && (bj < 0 || stronger(s2, h2, j2, bs, bh, bj))) {
-            bs = s2;
-            bh = h2;
-            bj = j2;
-        }
-    }
 }
 
 // Block-aggregated append of row i (when take) to a worklist: one atomic per block, the rows of
@@ -660,12 +606,12 @@ __global__ void __launch_bounds__(GD_WARPS * 32) k_gal_dedup(int nc, int cap, co
 
 // One warp per slice of the coarse matrix (lane = row): copy each row from the temporary
 // buffer, pad past the row length (col = row, value 0; rows past nc get col = 0) and record
-// the diagonal's slot (-1 if the row has none; k_check_diag reports it).
+// the diagonal's slot (-1 and ST_BAD_INDEX if the row has none).
 template <class T>
 __global__ void k_gal_scatter(int nc, int nslices, const int* __restrict__ sp_c, const int* __restrict__ off,
                               const int* __restrict__ tcol, const T* __restrict__ tval,
                               const int* __restrict__ rowlen_c, const int* __restrict__ dpos, int* __restrict__ col_c,
-                              T* __restrict__ val_c, int* __restrict__ diag_c)
+                              T* __restrict__ val_c, int* __restrict__ diag_c, int* status)
 {
     const int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (s >= nslices) return;
@@ -689,6 +635,7 @@ __global__ void k_gal_scatter(int nc, int nslices, const int* __restrict__ sp_c,
     if (row) {
         const int d = dpos[I];
         diag_c[I] = d >= 0 ? b + d * 32 + lane : -1;
+        if (d < 0) atomicOr(status, ST_BAD_INDEX);
     }
 }
 
@@ -699,6 +646,49 @@ __global__ void k_slice_width(int n, int nslices, const int* __restrict__ rowlen
     int w = 0;
     for (int r = s * 32; r < min(n, s * 32 + 32); ++r) w = max(w, rowlen[r]);
     width[s] = w * 32;
+}
+
+// Slice pointers of a coarse matrix of up to SELL_PTR_SLICES slices in one block: the widths (a warp reads
+// a slice's row lengths), their exclusive sum, the total behind it.
+constexpr int SELL_PTR_SLICES = 4096;
+__global__ void __launch_bounds__(1024) k_sell_ptr(int n, int nslices, const int* __restrict__ rowlen,
+                                                   int* __restrict__ sp)
+{
+    __shared__ int width[SELL_PTR_SLICES];
+    __shared__ int wsum[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int s = w; s < nslices; s += 32) {
+        int m = s * 32 + lane < n ? rowlen[s * 32 + lane] : 0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (lane == 0) width[s] = 32 * m;
+    }
+    __syncthreads();
+    constexpr int PER = SELL_PTR_SLICES / 1024;
+    int v[PER], sum = 0;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int s = PER * threadIdx.x + k;
+        v[k] = s < nslices ? width[s] : 0;
+        sum += v[k];
+    }
+    int inc = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+    }
+    if (lane == 31) wsum[w] = inc;
+    __syncthreads();
+    int run = inc - sum;
+    for (int k = 0; k < w; ++k) run += wsum[k];
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int s = PER * threadIdx.x + k;
+        if (s < nslices) sp[s] = run;
+        run += v[k];
+    }
+    if (threadIdx.x == 1023) sp[nslices] = run;
 }
 
 template <class T>
@@ -1330,41 +1320,85 @@ __global__ void k_dense_cholesky_inverse(int n, double* __restrict__ D, double* 
     }
 }
 
-// Inverse of the dense SPD matrix D (n <= DENSE_SMEM_N) by Gauss-Jordan elimination in shared
-// memory, one block of 32 x 32 threads (thread (tx, ty) owns the entries (ty + 32 a, tx + 32 b)):
-// for SPD matrices the pivots are the diagonal (no pivoting, as LDL^T).  Per pivot k, first every
-// entry outside row and column k is updated from the old row and column, then row and column k are
-// scaled: two barriers per pivot.  Non-positive or non-finite pivots set ST_NONFINITE.
-constexpr int DENSE_SMEM_N = 160;   // 200 KB of doubles
-__global__ void __launch_bounds__(1024) k_dense_gauss_jordan(int n, const double* __restrict__ D,
-                                                             double* __restrict__ Dinv, int* status)
+// Inverse of the coarsest matrix (SPD, n <= DENSE_CLUSTER_N) by Gauss-Jordan elimination (no pivoting, as
+// LDL^T) in the shared memory of one cluster: each block owns a contiguous part of the rows, a warp a row
+// at a time.  The owner of pivot row k scales it by the inverted pivot and stores it in every block (two
+// buffers); then a_ij -= a_ik r_j for all rows, with r_k the inverted pivot and a_ik taken as 0, and one
+// cluster barrier.  The next pivot row is updated first, so its division and scaling overlap the others'
+// updates.  FP64-issue bound (two operations a clock and SM): eight SMs, one FMA per entry and pivot, one
+// division per pivot instead of one per warp and pivot; 108 rows take 219 us, one block with a division in
+// every thread took 718 us.  Non-positive or non-finite pivots set ST_NONFINITE.
+// 1 / x by two Newton steps from the hardware's estimate (within an ulp or two; x normal)
+__device__ __forceinline__ double reciprocal(double x)
 {
-    extern __shared__ double A[];
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int q = threadIdx.x; q < n * n; q += blockDim.x) A[q] = D[q];
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    r = fma(r, fma(-x, r, 1.0), r);
+    return fma(r, fma(-x, r, 1.0), r);
+}
+
+constexpr int DENSE_CLUSTER_N = 160;
+constexpr int DENSE_CTAS = 8;
+template <class T>
+__global__ void __launch_bounds__(512, 1) k_dense_inverse(int n, const int* __restrict__ sp,
+                                                          const int* __restrict__ col,
+                                                          const int* __restrict__ rowlen, const T* __restrict__ M,
+                                                          double* __restrict__ Dinv, int* status)
+{
+    extern __shared__ double dsm[];
+    const int rank = int(cluster_rank()), tid = threadIdx.x, w = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
+    const int per = (n + DENSE_CTAS - 1) / DENSE_CTAS, r0 = min(n, rank * per), own = min(n, r0 + per) - r0;
+    double* R = dsm;               // [2][n]: scaled pivot rows
+    double* A = dsm + 2 * n;       // [own][n]
+    for (int q = tid; q < own * n; q += blockDim.x) A[q] = 0.0;
     __syncthreads();
-    for (int k = 0; k < n; ++k) {
-        const double akk = A[k * n + k];
+    if (tid < own)
+        for (int t = 0; t < rowlen[r0 + tid]; ++t) {
+            const int k = slot_of(sp, r0 + tid, t);
+            A[tid * n + col[k]] += double(M[k]);
+        }
+    __syncthreads();
+    // row k of this block, scaled, into buffer k & 1 of every block (its warp only)
+    auto publish = [&](int k) {
+        const double* a = A + (k - r0) * n;
+        const double akk = a[k];
         if (!(akk > 0.0) || !isfinite(akk)) {
-            if (threadIdx.x == 0) atomicOr(status, ST_NONFINITE);
-            return;   // uniform: every thread read the same pivot
+            if (lane == 0) atomicOr(status, ST_NONFINITE);
         }
-        const double piv = 1.0 / akk;
-        for (int i = ty; i < n; i += 32) {
-            if (i == k) continue;
-            const double aik = A[i * n + k] * piv;
-            for (int j = tx; j < n; j += 32)
-                if (j != k) A[i * n + j] -= aik * A[k * n + j];
+        const double piv = reciprocal(akk);
+        for (int j = lane; j < n; j += 32) {
+            const double v = j == k ? piv : a[j] * piv;
+            const unsigned at = smem_u32(R + (k & 1) * n + j);
+#pragma unroll
+            for (int c = 0; c < DENSE_CTAS; ++c) put(map_rank(at, unsigned(c)), v);
         }
-        __syncthreads();
-        if (ty == 0)
-            for (int j = tx; j < n; j += 32)
-                if (j != k) A[k * n + j] *= piv;
-        if (ty == 1)
-            for (int i = tx; i < n; i += 32) A[i * n + k] = (i == k) ? piv : -A[i * n + k] * piv;
-        __syncthreads();
+    };
+    cluster_sync();   // every block of the cluster runs
+    if (own > 0 && r0 == 0 && w == 0) publish(0);
+    cluster_sync();
+    for (int k = 0; k < n; ++k) {
+        const double* r = R + (k & 1) * n;
+        const int next = k + 1 - r0;   // local number of the next pivot row
+        auto update = [&](int i) {
+            double* a = A + i * n;
+            if (r0 + i == k) {
+                for (int j = lane; j < n; j += 32) a[j] = r[j];
+            } else {
+                const double f = a[k];
+                __syncwarp();
+                for (int j = lane; j < n; j += 32) a[j] = (j == k ? 0.0 : a[j]) - f * r[j];
+            }
+            __syncwarp();
+        };
+        if (k + 1 < n && next >= 0 && next < own && next % nw == w) {
+            update(next);
+            publish(k + 1);
+        }
+        for (int i = w; i < own; i += nw)
+            if (i != next || k + 1 >= n) update(i);
+        cluster_sync();
     }
-    for (int q = threadIdx.x; q < n * n; q += blockDim.x) Dinv[q] = A[q];
+    for (int q = tid; q < own * n; q += blockDim.x) Dinv[(size_t)r0 * n + q] = A[q];
 }
 
 template <class T>
@@ -1561,18 +1595,84 @@ void Amg<T>::members(cudaStream_t s, Aggregates& a)
     PORSOL_CUDA(cudaGetLastError());
 }
 
+// One pairing round: the aggregates of a level with their member lists.  Levels of up to AGG_ROWS rows run
+// as one cluster launch (aggregate.h), larger ones as a launch per sweep and step.  Both make the same
+// decisions and write the same arrays.
 template <class T>
 void Amg<T>::aggregate_round(cudaStream_t s, const SellPattern& P, const T* A, int n, bool neg_first,
                              Aggregates& out)
 {
-    int first = -1;
-    if (neg_first) {
-        pairwise(s, P, A, n, true, o_.strength, false, out);
-        first = out.nc;
+    out.offsets = false;
+    if (agg_small(n, P.nent)) {
+        aggregate_small(s, P, A, n, neg_first, out);
+        return;
     }
+    if (neg_first) pairwise(s, P, A, n, true, o_.strength, false, out);
     if (!neg_first || out.nc > 0.8 * n) pairwise(s, P, A, n, false, 0.0, true, out);
-    static const bool debug = std::getenv("PORSOL_DEBUG_AMG") != nullptr;
-    if (debug) std::fprintf(stderr, "[amg] round n=%d strong-negative pairs -> %d, final -> %d\n", n, first, out.nc);
+    members(s, out);
+}
+
+template <class T>
+void Amg<T>::aggregate_small(cudaStream_t s, const SellPattern& P, const T* A, int n, bool neg_first, Aggregates& out)
+{
+    s_rs_.alloc(n);
+    for (DBuf<int>* b : {&s_state_, &s_partner_, &s_join_, &s_best_, &s_cidx_, &s_cnt_}) b->alloc(size_t(n) + 1);
+    s_goff_.alloc(size_t(n) + 1);
+    s_woff_.alloc(n);
+    out.n = n;
+    out.agg.alloc(n);
+    out.ptr.alloc(size_t(n) + 1);
+    out.idx.alloc(n);
+    iscratch_.alloc(AGG_SCRATCH);
+    AggArgs<T> a{};
+    a.n = n;
+    a.sp = P.slice_ptr.p;
+    a.col = P.col.p;
+    a.rowlen = P.rowlen.p;
+    a.diag = P.diag.p;
+    a.A = A;
+    a.neg_first = neg_first ? 1 : 0;
+    a.theta = float(o_.strength);
+    a.rs = s_rs_.p;
+    a.state = s_state_.p;
+    a.partner = s_partner_.p;
+    a.join = s_join_.p;
+    a.best = s_best_.p;
+    a.cidx = s_cidx_.p;
+    a.cnt = s_cnt_.p;
+    a.agg = out.agg.p;
+    a.ptr = out.ptr.p;
+    a.idx = out.idx.p;
+    a.goff = s_goff_.p;
+    a.woff = s_woff_.p;
+    a.scratch = iscratch_.p;
+    agg_launch<T>(s, pick_lanes(n, P.nent), a);
+    int r[3];
+    PORSOL_CUDA(cudaMemcpyAsync(r, iscratch_.p, sizeof(r), cudaMemcpyDeviceToHost, s));
+    PORSOL_CUDA(cudaStreamSynchronize(s));
+    out.nc = r[0];
+    out.total = r[1];
+    out.bound = r[2];
+    out.offsets = true;   // s_goff_ and s_woff_ hold the candidate offsets of this round
+}
+
+// The aggregates of two rounds as one: `first` maps rows to those of the next round's aggregates, with
+// member lists.
+template <class T>
+void Amg<T>::compose(cudaStream_t s, Aggregates& first, const Aggregates& second)
+{
+    first.offsets = false;
+    first.nc = second.nc;
+    if (agg_small(first.n, 0)) {
+        s_cnt_.alloc(size_t(first.n) + 1);
+        first.ptr.alloc(size_t(first.n) + 1);
+        first.idx.alloc(first.n);
+        iscratch_.alloc(AGG_SCRATCH);
+        compose_launch(s, first.n, first.nc, first.agg.p, second.agg.p, s_cnt_.p, first.ptr.p, first.idx.p, iscratch_.p);
+        return;
+    }
+    PORSOL_LAUNCH(k_compose<<<div_up(first.n, TB), TB, 0, s>>>(first.n, first.agg.p, second.agg.p));
+    members(s, first);
 }
 
 template <class T>
@@ -1585,18 +1685,19 @@ void Amg<T>::galerkin(cudaStream_t s, const SellPattern& P, const T* A, const Ag
     Pc.rowlen.alloc(std::max(nc, 1));
     Pc.diag.alloc(std::max(nc, 1));
     Pc.slice_ptr.alloc(Pc.nslices + 1);
-    iscratch_.alloc(4);
-    PORSOL_CUDA(cudaMemsetAsync(iscratch_.p, 0, sizeof(int), s));
-    s_bnd_.alloc(std::max(nc, 1));
-    s_goff_.alloc(nc + 1);
-    PORSOL_LAUNCH(k_gal_rowbound<<<div_up(nc, TB), TB, 0, s>>>(nc, a.ptr.p, a.idx.p, P.rowlen.p, s_bnd_.p,
-                                                                iscratch_.p));
-    exclusive_scan(s, nc, s_bnd_.p, s_goff_.p, s_goff_.p + nc, scan_blocks_);
-    int hb[2] = {0, 0};
-    PORSOL_CUDA(cudaMemcpyAsync(&hb[0], iscratch_.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-    PORSOL_CUDA(cudaMemcpyAsync(&hb[1], s_goff_.p + nc, sizeof(int), cudaMemcpyDeviceToHost, s));
-    PORSOL_CUDA(cudaStreamSynchronize(s));
-    const int bound = hb[0], total = hb[1];
+    int bound = a.bound, total = a.total;
+    if (!a.offsets) {
+        iscratch_.alloc(4);
+        PORSOL_CUDA(cudaMemsetAsync(iscratch_.p, 0, sizeof(int), s));
+        s_bnd_.alloc(std::max(nc, 1));
+        s_goff_.alloc(nc + 1);
+        PORSOL_LAUNCH(k_gal_rowbound<<<div_up(nc, TB), TB, 0, s>>>(nc, a.ptr.p, a.idx.p, P.rowlen.p, s_bnd_.p,
+                                                                    iscratch_.p));
+        exclusive_scan(s, nc, s_bnd_.p, s_goff_.p, s_goff_.p + nc, scan_blocks_);
+        PORSOL_CUDA(cudaMemcpyAsync(&bound, iscratch_.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+        PORSOL_CUDA(cudaMemcpyAsync(&total, s_goff_.p + nc, sizeof(int), cudaMemcpyDeviceToHost, s));
+        PORSOL_CUDA(cudaStreamSynchronize(s));
+    }
     PORSOL_REQUIRE(bound <= 2048, PORSOL_ERR_BAD_ARG, "AMG: aggregate rows too long for the Galerkin merge");
     const bool warp = bound <= 1024;
     if (warp) {
@@ -1604,9 +1705,11 @@ void Amg<T>::galerkin(cudaStream_t s, const SellPattern& P, const T* A, const Ag
         s_tcol_.alloc(std::max(total, 1));
         s_tval_.alloc(std::max(total, 1));
         s_dpos_.alloc(std::max(nc, 1));
-        s_woff_.alloc(std::max(P.n, 1));
-        PORSOL_LAUNCH(k_gal_woff<<<div_up(nc, TB), TB, 0, s>>>(nc, a.ptr.p, a.idx.p, P.rowlen.p, s_goff_.p,
-                                                               s_woff_.p));
+        if (!a.offsets) {
+            s_woff_.alloc(std::max(P.n, 1));
+            PORSOL_LAUNCH(k_gal_woff<<<div_up(nc, TB), TB, 0, s>>>(nc, a.ptr.p, a.idx.p, P.rowlen.p, s_goff_.p,
+                                                                   s_woff_.p));
+        }
         const int cl = pick_lanes(P.n, P.nent);
         PORSOL_LANES(cl, PORSOL_LAUNCH((k_gal_cand<T, KL><<<div_up((long long)P.n * cl, TB), TB, 0, s>>>(
                              P.n, P.slice_ptr.p, P.col.p, P.rowlen.p, A, a.agg.p, s_woff_.p, s_tcol_.p, s_tval_.p))));
@@ -1630,25 +1733,29 @@ void Amg<T>::galerkin(cudaStream_t s, const SellPattern& P, const T* A, const Ag
         k_gal_count<T, 2048><<<nb, 64, 0, s>>>(nc, P.slice_ptr.p, P.col.p, P.rowlen.p, A, a.agg.p, a.ptr.p, a.idx.p,
                                                Pc.rowlen.p);
     }
-    DBuf<int>& width = s_width_;
-    width.alloc(Pc.nslices);
-    PORSOL_LAUNCH(k_slice_width<<<div_up(Pc.nslices, TB), TB, 0, s>>>(nc, Pc.nslices, Pc.rowlen.p, width.p));
-    exclusive_scan(s, Pc.nslices, width.p, Pc.slice_ptr.p, Pc.slice_ptr.p + Pc.nslices, scan_blocks_);
+    if (Pc.nslices <= SELL_PTR_SLICES) {
+        PORSOL_LAUNCH(k_sell_ptr<<<1, 1024, 0, s>>>(nc, Pc.nslices, Pc.rowlen.p, Pc.slice_ptr.p));
+    } else {
+        DBuf<int>& width = s_width_;
+        width.alloc(Pc.nslices);
+        PORSOL_LAUNCH(k_slice_width<<<div_up(Pc.nslices, TB), TB, 0, s>>>(nc, Pc.nslices, Pc.rowlen.p, width.p));
+        exclusive_scan(s, Pc.nslices, width.p, Pc.slice_ptr.p, Pc.slice_ptr.p + Pc.nslices, scan_blocks_);
+    }
     Pc.nent = read_int(s, Pc.slice_ptr.p + Pc.nslices);
     Pc.col.alloc(std::max<long long>(Pc.nent, 1));
     Ac.alloc(std::max<long long>(Pc.nent, 1));
     if (warp) {
         PORSOL_LAUNCH(k_gal_scatter<T><<<div_up(Pc.nslices, TB / 32), TB, 0, s>>>(
             nc, Pc.nslices, Pc.slice_ptr.p, s_goff_.p, s_tcol_.p, s_tval_.p, Pc.rowlen.p, s_dpos_.p, Pc.col.p, Ac.p,
-            Pc.diag.p));
+            Pc.diag.p, status_.p));
     } else {
         const int nb = div_up(nc, 64);
         PORSOL_COUNT_LAUNCH();
         k_gal_fill<T, 2048><<<nb, 64, 0, s>>>(nc, P.slice_ptr.p, P.col.p, P.rowlen.p, A, a.agg.p, a.ptr.p, a.idx.p,
                                               Pc.slice_ptr.p, Pc.col.p, Ac.p, Pc.diag.p);
         if (nc > 0) PORSOL_LAUNCH(k_pad_tail<T><<<1, 32, 0, s>>>(nc, Pc.nslices, Pc.slice_ptr.p, Pc.col.p, Ac.p));
+        PORSOL_LAUNCH(k_check_diag<<<div_up(nc, TB), TB, 0, s>>>(nc, Pc.diag.p, status_.p));
     }
-    PORSOL_LAUNCH(k_check_diag<<<div_up(nc, TB), TB, 0, s>>>(nc, Pc.diag.p, status_.p));
     PORSOL_CUDA(cudaGetLastError());
 }
 
@@ -1792,17 +1899,16 @@ void Amg<T>::build_coarse_solver(cudaStream_t s, const SellPattern& P, const T* 
 {
     nc_ = n;
     DBuf<double>&D = s_D_, &Linv = s_Linv_;
-    D.alloc(std::max<size_t>((size_t)n * n, 1));
-    Linv.alloc(std::max<size_t>((size_t)n * n, 1));
     cinv_.alloc(std::max<size_t>((size_t)n * n, 1));
     if (n > 0) {
-        PORSOL_LAUNCH(k_dense_from_sell<T><<<div_up(n, 128), 128, 0, s>>>(n, P.slice_ptr.p, P.col.p, P.rowlen.p, A, D.p));
-        if (n <= DENSE_SMEM_N) {
-            const int shm = n * n * int(sizeof(double));
-            PORSOL_CUDA(cudaFuncSetAttribute(k_dense_gauss_jordan, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             DENSE_SMEM_N * DENSE_SMEM_N * int(sizeof(double))));
-            PORSOL_LAUNCH(k_dense_gauss_jordan<<<1, 1024, shm, s>>>(n, D.p, cinv_.p, status_.p));
+        if (n <= DENSE_CLUSTER_N) {
+            const size_t shm = size_t(2 + div_up(n, DENSE_CTAS)) * n * sizeof(double);
+            launch_cluster(k_dense_inverse<T>, DENSE_CTAS, 512, shm, s, false, n, (const int*)P.slice_ptr.p,
+                           (const int*)P.col.p, (const int*)P.rowlen.p, A, cinv_.p, status_.p);
         } else {
+            Linv.alloc((size_t)n * n);
+            D.alloc((size_t)n * n);
+            PORSOL_LAUNCH(k_dense_from_sell<T><<<div_up(n, 128), 128, 0, s>>>(n, P.slice_ptr.p, P.col.p, P.rowlen.p, A, D.p));
             PORSOL_LAUNCH(k_dense_cholesky_inverse<<<1, 1024, 0, s>>>(n, D.p, Linv.p, cinv_.p, status_.p));
         }
     }
@@ -1857,26 +1963,20 @@ void Amg<T>::setup(cudaStream_t s, const SellPattern& P0, const T* A0, const Amg
         Level& next = *lv_[nlev_];
         // first pairing round on this level's matrix; L.agg maps rows to the intermediate level
         aggregate_round(s, P, L.A, n, o_.round1_negative, L.agg);
-        members(s, L.agg);
         galerkin(s, P, L.A, L.agg, tmp_pat_, tmp_val_);
         const int nc1 = L.agg.nc;
         if (nc1 > o.coarse_target) {
             // round 2 on the intermediate matrix: aggregates of about four rows
             aggregate_round(s, tmp_pat_, tmp_val_.p, nc1, o_.round2_negative, agg2_);
-            members(s, agg2_);
             galerkin(s, tmp_pat_, tmp_val_.p, agg2_, next.own, next.own_val);
-            PORSOL_LAUNCH(k_compose<<<div_up(n, TB), TB, 0, s>>>(n, L.agg.agg.p, agg2_.agg.p));
-            L.agg.nc = agg2_.nc;
+            compose(s, L.agg, agg2_);
             if (nlev_ > 1 && n < o.round3_below && agg2_.nc > o.coarse_target) {
                 // round 3 on the level just formed (coarse levels only)
                 aggregate_round(s, next.own, next.own_val.p, agg2_.nc, o_.round2_negative, agg2_);
-                members(s, agg2_);
                 galerkin(s, next.own, next.own_val.p, agg2_, tmp_pat_, tmp_val_);
                 adopt_tmp(next);
-                PORSOL_LAUNCH(k_compose<<<div_up(n, TB), TB, 0, s>>>(n, L.agg.agg.p, agg2_.agg.p));
-                L.agg.nc = agg2_.nc;
+                compose(s, L.agg, agg2_);
             }
-            members(s, L.agg);
         } else {
             adopt_tmp(next);
         }

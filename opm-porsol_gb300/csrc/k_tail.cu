@@ -5,34 +5,12 @@
 #include <mutex>
 
 #include "bulk.cuh"
+#include "cluster.cuh"
 #include "tail.h"
 
 namespace porsol {
 
 namespace {
-
-__device__ __forceinline__ unsigned cluster_rank()
-{
-    unsigned r;
-    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
-__device__ __forceinline__ void cluster_sync()
-{
-    cluster_arrive();
-    cluster_wait();
-}
-// address of this block's shared location `a` in the block of rank r
-__device__ __forceinline__ unsigned map_rank(unsigned a, unsigned r)
-{
-    unsigned d;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(r));
-    return d;
-}
-__device__ __forceinline__ void put(unsigned a, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
-__device__ __forceinline__ void put(unsigned a, double v) { asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory"); }
 
 __device__ __forceinline__ void copy16(unsigned dst, const void* src)
 {
@@ -428,21 +406,7 @@ void tail_launch(cudaStream_t s, bool half, const TailArgs<T>& a, int shm)
 {
     auto* f = half ? k_tail<T, true> : k_tail<T, false>;
     PORSOL_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, TAIL_SMEM));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = TAIL_CTAS;
-    cfg.blockDim = TAIL_THREADS;
-    cfg.dynamicSmemBytes = size_t(shm);
-    cfg.stream = s;
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = TAIL_CTAS;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = chain_enabled(TAIL_CTAS) ? 2 : 1;
-    PORSOL_CUDA(cudaLaunchKernelEx(&cfg, f, a));
-    PORSOL_COUNT_LAUNCH();
+    launch_cluster(f, TAIL_CTAS, TAIL_THREADS, size_t(shm), s, chain_enabled(TAIL_CTAS), a);
 }
 
 #define PORSOL_TAIL(T)                                                                                              \
