@@ -22,6 +22,7 @@
 #include "aggregate.h"
 #include "krylov.h"
 #include "tail.h"
+#include "vec3.cuh"
 
 namespace porsol {
 
@@ -43,6 +44,7 @@ struct AmgOpts {
     bool autotune = false;         // time the lane schedules of each new level shape once (the
                                    // choice then depends on timing: off where runs must be
                                    // bitwise reproducible)
+    bool three_vectors = false;    // work vectors of three right-hand sides (apply3; one with apply)
     int kcycle_levels = 0;         // K-cycle: the coarse corrections of levels 1 .. kcycle_levels are
                                    // two flexible-CG steps preconditioned by the cycle of that level
                                    // (0: plain V-cycle)
@@ -67,6 +69,8 @@ class Amg : public Precond<T> {
 public:
     void setup(cudaStream_t s, const SellPattern& P0, const T* A0, const AmgOpts& o);
     void apply(cudaStream_t s, const T* r, T* z, const int* stop) override;
+    // the same cycle for three right-hand sides at once (hierarchies set up with three_vectors)
+    void apply3(cudaStream_t s, const V3<T>* r, V3<T>* z, const int* stop);
     int levels() const { return nlev_; }
     void set_profiler(Profiler* p) { prof_ = p; }
     const std::vector<int>& level_sizes() const { return sizes_; }
@@ -141,9 +145,18 @@ private:
     void build_coarse_solver(cudaStream_t s, const SellPattern& P, const T* A, int n);
     // started: the first Chebyshev start from zero (r = D^-1 b, d = r / theta) was already done by
     // the restriction that produced b (k_restrict_start0)
-    void chebyshev(cudaStream_t s, Level& L, const T* b, T* x, bool from_zero, const T* xc, const int* agg,
+    template <class VT>
+    void chebyshev(cudaStream_t s, Level& L, const VT* b, VT* x, bool from_zero, const VT* xc, const int* agg,
                    const int* stop, bool started = false);
-    void vcycle(cudaStream_t s, int l, const T* b, T* x, const int* stop, bool started = false);
+    template <class VT>
+    void vcycle(cudaStream_t s, int l, const VT* b, VT* x, const int* stop, bool started = false);
+    // a work vector as elements VT (T, or V3<T> of a hierarchy set up with three_vectors)
+    template <class VT>
+    static VT* work(DBuf<T>& v)
+    {
+        return reinterpret_cast<VT*>(v.p);
+    }
+    size_t vec_width() const { return o_.three_vectors ? sizeof(V3<T>) / sizeof(T) : 1; }
     // coarse correction of level l - 1 solved on level l by two flexible-CG steps (K-cycle)
     void kcycle(cudaStream_t s, int l, const T* b, T* x, const int* stop, bool started = false);
     bool k_level(int l) const { return l >= 1 && l <= o_.kcycle_levels && l < nlev_ - 1; }

@@ -9,7 +9,9 @@
 // block diagonal too (an AMG hierarchy of the union is: aggregates never cross sub-grids).
 #pragma once
 
+#include "amg.h"
 #include "krylov.h"
+#include "vec3.cuh"
 
 namespace porsol {
 
@@ -19,6 +21,12 @@ struct BatchRanges {
     int nblk = 0, n = 0;
     std::vector<int> h;
     DBuf<int> ranges, blk;
+    // the unknowns in chunks of at most CHUNK of one block, block by block: (first unknown, unknowns,
+    // block, -), and each block's range of chunks
+    static constexpr int CHUNK = 2048;
+    int nchunks = 0;
+    DBuf<int4> chunks;
+    DBuf<int> cptr;
     void build(const std::vector<int>& four_per_block, int n_unknowns, cudaStream_t s);
 };
 
@@ -61,26 +69,53 @@ private:
                    const double* tol);
 };
 
-// FP64 Krylov with an FP32 block-diagonal preconditioner: z = isc_g * double(M32(float(sc_g r)))
-// per block g.  The preconditioner is linear and block diagonal, so the per-block scaling
-// (sc = 1 / ||r0_g||, isc = ||r0_g||) only keeps the FP32 vectors in range; the CG recurrences,
-// the solution and the stopping test stay FP64, so no restart is ever needed.
-class BatchCastPrecond : public Precond<double> {
-public:
-    void bind(Precond<float>* inner, const BatchRanges* B, const double* sc, const double* isc);
-    void apply(cudaStream_t s, const double* r, double* z, const int* stop) override;
-    void set_block_state(const int* conv) override;   // passed to the inner preconditioner
-
-private:
-    Precond<float>* m_ = nullptr;
-    const BatchRanges* B_ = nullptr;
-    const double *sc_ = nullptr, *isc_ = nullptr;
-    long long inner_gen_ = -1;
-    DBuf<float> r32_, z32_;
+// State of BatchedCg3 (device), mirrored for the host in mapped memory: blocks left and iterations run
+// per direction.
+struct Batch3Dev {
+    int iter, maxit, stop, left[3], iters[3], pad;
+};
+struct Batch3HostView {
+    volatile int stop, active, breakdown, iters[3];
 };
 
-// Per-block helper of the batched solve.
-// out[g] = ||a_g||_2 (deterministic order)
-template <class T>
-void batch_norms(cudaStream_t s, const BatchRanges& B, const T* a, double* out);
+// The three right-hand sides of an upscaling batch, one CG recurrence per block and direction (the
+// recurrences and tests of BatchedPcg), run together: the matrix and the AMG hierarchy are read once per
+// iteration for three products and three cycles.  The CG is FP64; with an FP32 hierarchy the residual of
+// each block and direction enters scaled by 1 / ||r0|| and the correction is scaled back (the hierarchy is
+// linear and block diagonal, so the scaling only keeps the FP32 vectors in range).
+class BatchedCg3 {
+public:
+    // b3, x3 (initial guess and result): three values per unknown, side by side.  Every block and
+    // direction stops when ||r|| < tol ||r0|| or ||r|| < 1e-30.  iterations of the result: the sum over the
+    // directions of the iterations until their last block stopped.
+    template <class T>
+    CgResult solve(cudaStream_t s, const SellPattern& P, const double* val, Amg<T>& M, const BatchRanges& B,
+                   const double* b3, double* x3, double tol, int maxit);
+    ~BatchedCg3();
+
+private:
+    void setup(const BatchRanges& B, bool fp32, cudaStream_t s);
+    template <class T>
+    void precondition(cudaStream_t s, Amg<T>& M);
+    template <class T>
+    void direction(cudaStream_t s, const BatchRanges& B, int first);
+    template <class T>
+    void iteration(cudaStream_t s, const SellPattern& P, const double* val, Amg<T>& M, const BatchRanges& B,
+                   V3<double>* x, double tol);
+    DBuf<V3<double>> r_, p_, q_, z64_, part_, part2_, scale_, iscale_;
+    DBuf<V3<float>> r32_, z32_;
+    DBuf<double> rho_, def0_, def_;
+    DBuf<int> done_, broken_, conv_;   // per block and direction: 0 active, 1 converged, 2 breakdown; per block
+    DBuf<Batch3Dev> st_;
+    DBuf<unsigned int> counter_;
+    Batch3HostView* hview_ = nullptr;
+    Batch3HostView* dview_ = nullptr;
+    std::vector<cudaEvent_t> ev_;
+    cudaGraphExec_t exec_ = nullptr;
+    const void* key_[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    long long key_gen_ = -1, nodes_ = 0;
+    int key_n_[2] = {0, 0};
+    double key_tol_ = 0.0;
+};
+
 }  // namespace porsol

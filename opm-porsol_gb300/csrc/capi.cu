@@ -283,6 +283,14 @@ void porsol_solver::ensure_recipe(const int* bct_host, const int* bct_dev)
 }
 
 namespace {
+[[noreturn]] void not_converged(int iterations, double reduction)
+{
+    std::ostringstream os;
+    os << "Linear solver failed to converge in " << iterations << " iterations.\n"
+       << "Residual reduction achieved is " << reduction << '\n';
+    throw Error(PORSOL_ERR_NOT_CONVERGED, os.str());
+}
+
 double now_ms()
 {
     return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now().time_since_epoch()).count();
@@ -330,12 +338,7 @@ void porsol_solver::linear_solve(const porsol_solve_opts& o, porsol_solve_stats&
     const SellPattern& P = S.pat;
     st.amg_levels = 0;
     st.outer_iterations = 1;
-    auto fail = [&](int iters, double red) {
-        std::ostringstream os;
-        os << "Linear solver failed to converge in " << iters << " iterations.\n"
-           << "Residual reduction achieved is " << red << '\n';
-        throw Error(PORSOL_ERR_NOT_CONVERGED, os.str());
-    };
+    auto fail = not_converged;
     if (batch.nblk > 0) {
         batched_solve(o, st, maxit);
         return;
@@ -373,7 +376,7 @@ void porsol_solver::linear_solve(const porsol_solve_opts& o, porsol_solve_stats&
     ao.kcycle_levels = o.linsolver_type == 2 ? 1 : 0;
     dirichlet_guess(stream, P, val.p, rhs.p, x.p);
     if (o.precision == PORSOL_FP64) {
-        if (!((o.same_matrix || reuse_amg) && amg_ready && amg_precision == PORSOL_FP64 &&
+        if (!(o.same_matrix && amg_ready && amg_precision == PORSOL_FP64 &&
               amg_kcycle == ao.kcycle_levels)) {
             amg64.set_row_blocks(nullptr);
             amg64.setup(stream, P, val.p, ao);
@@ -395,7 +398,7 @@ void porsol_solver::linear_solve(const porsol_solve_opts& o, porsol_solve_stats&
     // Mixed precision: FP32 matrix copy, FP32 AMG hierarchy and one FP32 CG recurrence with the
     // solution in FP64 and reliable updates (the iterated residual replaced by the FP64 residual
     // b - A x whenever it has dropped by inner_tolerance); see ReliableCg.
-    if (!((o.same_matrix || reuse_amg) && amg_ready && amg_precision == PORSOL_MIXED &&
+    if (!(o.same_matrix && amg_ready && amg_precision == PORSOL_MIXED &&
           amg_kcycle == ao.kcycle_levels)) {
         // the throughput path coarsens its small coarse levels by three pairing rounds instead of
         // two (on the 1M-cell system: 9 levels instead of 10, same CG iteration count, 2 % faster);
@@ -467,116 +470,68 @@ void porsol_solver::ilu_solve_reference_order(const porsol_solve_opts& o, porsol
     st.reduction = r.reduction;
     count_krylov_bytes(o, r.iterations, 0);
     if (r.breakdown) throw Error(PORSOL_ERR_NONFINITE, "CG breakdown (non-positive curvature)");
-    if (!r.converged) {
-        std::ostringstream os;
-        os << "Linear solver failed to converge in " << r.iterations << " iterations.\n"
-           << "Residual reduction achieved is " << r.reduction << '\n';
-        throw Error(PORSOL_ERR_NOT_CONVERGED, os.str());
-    }
+    if (!r.converged) not_converged(r.iterations, r.reduction);
 }
 
-// Block-diagonal systems (batched upscaling): one CG per block (BatchedPcg), each block with
-// the stopping test ||r_g|| < tol ||r_g^0|| that its own solve would use.  FP64: ILU0 or AMG
-// preconditioner; mixed: FP64 per-block residuals around FP32 batched CG + FP32 AMG.
+// Block-diagonal systems (batched upscaling), each block with the stopping test ||r_g|| < tol ||r_g^0|| that
+// its own solve would use.  ILU0 (type 0): one direction at a time.
 void porsol_solver::batched_solve(const porsol_solve_opts& o, porsol_solve_stats& st, int maxit)
 {
     const double t_begin = now_ms();
-    const int n = S.N, nb = batch.nblk;
     const SellPattern& P = S.pat;
     st.amg_levels = 0;
     st.outer_iterations = 1;
-    auto fail = [&](int iters, double red) {
-        std::ostringstream os;
-        os << "Linear solver failed to converge in " << iters << " iterations.\n"
-           << "Residual reduction achieved is " << red << '\n';
-        throw Error(PORSOL_ERR_NOT_CONVERGED, os.str());
-    };
-    std::vector<double> h(nb);
-    auto upload = [&](DBuf<double>& d, const std::vector<double>& v) { d.upload(v, stream); };
+    if (!ilu_levels) {
+        ilu.build_levels(P, stream);
+        ilu_levels = true;
+    }
+    ilu.factor(stream, P, val.p);
+    x.zero(stream);
+    PORSOL_CUDA(cudaStreamSynchronize(stream));
+    st.ms_precond_setup = now_ms() - t_begin;
+    btol.upload(std::vector<double>(size_t(batch.nblk), o.residual_tolerance), stream);
+    CgResult r = bcg64.solve(stream, P, val.p, ilu, batch, rhs.p, x.p, btol.p, maxit);
+    check_ilu_status();
+    st.iterations = r.iterations;
+    st.reduction = r.reduction;
+    if (r.breakdown) throw Error(PORSOL_ERR_NONFINITE, "CG breakdown (non-positive curvature)");
+    if (!r.converged) not_converged(r.iterations, r.reduction);
+}
+
+// AMG (types 1-3, the V-cycle): the three directions together (b3, x3: three values per unknown), FP64 CG
+// around an FP64 or (mixed) FP32 hierarchy.
+void porsol_solver::batched_solve3(const porsol_solve_opts& o, porsol_solve_stats& st, const double* b3, double* x3)
+{
+    const double t_begin = now_ms();
+    const SellPattern& P = S.pat;
+    const int maxit = o.linsolver_maxit > 0 ? o.linsolver_maxit : S.N;
+    const bool mixed = o.precision == PORSOL_MIXED;
+    st.outer_iterations = 3;
     AmgOpts ao;
     ao.smooth_steps = std::max(1, o.smooth_steps);
     ao.prolong = o.prolongate_factor;
     ao.autotune = true;   // the sub-grid union's level shapes are unlike a single grid's
+    ao.three_vectors = true;
     // FP32 smoother values: with the FP16 copy the full-tensor, rotated sub-grids needed 491 CG
     // iterations for 512 sub-grids x 3 solves against 282 (and 239 in FP64)
     ao.half_smoother = false;
-    const bool mixed = o.precision == PORSOL_MIXED && o.linsolver_type != 0;
-    if (!mixed) {
-        Precond<double>* M = nullptr;
-        if (o.linsolver_type == 0) {
-            if (!ilu_levels) {
-                ilu.build_levels(P, stream);
-                ilu_levels = true;
-            }
-            ilu.factor(stream, P, val.p);
-            x.zero(stream);
-            M = &ilu;
-        } else {
-            dirichlet_guess(stream, P, val.p, rhs.p, x.p);
-            if (!((o.same_matrix || reuse_amg) && amg_ready && amg_precision == PORSOL_FP64)) {
-                amg64.set_row_blocks(batch.blk.p);
-                amg64.setup(stream, P, val.p, ao);
-                amg_ready = true;
-                amg_precision = PORSOL_FP64;
-                amg_kcycle = 0;
-            }
-            st.amg_levels = amg64.levels();
-            M = &amg64;
-        }
+    auto run = [&](auto& amg, const auto* a) {
+        amg.set_row_blocks(batch.blk.p);
+        amg.setup(stream, P, a, ao);
+        amg_ready = true;
+        amg_precision = o.precision;
+        amg_kcycle = 0;
         PORSOL_CUDA(cudaStreamSynchronize(stream));
         st.ms_precond_setup = now_ms() - t_begin;
-        std::fill(h.begin(), h.end(), o.residual_tolerance);
-        upload(btol, h);
-        CgResult r = bcg64.solve(stream, P, val.p, *M, batch, rhs.p, x.p, btol.p, maxit);
-        if (o.linsolver_type == 0) check_ilu_status();
-        st.iterations = r.iterations;
-        st.reduction = r.reduction;
-        if (r.breakdown) throw Error(PORSOL_ERR_NONFINITE, "CG breakdown (non-positive curvature)");
-        if (!r.converged) fail(r.iterations, r.reduction);
-        return;
-    }
-    dirichlet_guess(stream, P, val.p, rhs.p, x.p);
-    if (!((o.same_matrix || reuse_amg) && amg_ready && amg_precision == PORSOL_MIXED)) {
-        amg32.set_row_blocks(batch.blk.p);
-        amg32.setup(stream, P, val32.p, ao);
-        amg_ready = true;
-        amg_precision = PORSOL_MIXED;
-        amg_kcycle = 0;
-    }
-    PORSOL_CUDA(cudaStreamSynchronize(stream));
-    st.ms_precond_setup = now_ms() - t_begin;
-    st.amg_levels = amg32.levels();
-    // FP64 batched CG around the FP32 AMG hierarchy, per-block scaled into FP32 range
-    ir_r.alloc(n);
-    bnorm.alloc(nb);
-    residual<double, double>(stream, P, val.p, x.p, rhs.p, ir_r.p);
-    batch_norms<double>(stream, batch, ir_r.p, bnorm.p);
-    std::vector<double> r0(nb), sc(nb);
-    bnorm.download(r0.data(), nb, stream);
-    PORSOL_CUDA(cudaStreamSynchronize(stream));
-    for (int g = 0; g < nb; ++g) {
-        const bool ok = r0[g] > 1e-300 && std::isfinite(r0[g]);
-        sc[g] = ok ? 1.0 / r0[g] : 0.0;
-        r0[g] = ok ? r0[g] : 0.0;
-    }
-    upload(bscale, sc);
-    upload(bnorm, r0);
-    cast_pre.bind(&amg32, &batch, bscale.p, bnorm.p);
-    std::fill(h.begin(), h.end(), o.residual_tolerance);
-    upload(btol, h);
-    CgResult r = bcg64.solve(stream, P, val.p, cast_pre, batch, rhs.p, x.p, btol.p, maxit);
-    // the FP32 hierarchy's finest level may run the bulk-staged smoother step: its status bits say
-    // whether every staged copy arrived (as after the single-system mixed solve)
-    if (const int ast = amg32.solve_status(stream)) {
-        amg_ready = false;   // the next solve sets the hierarchy (and its status) up again
-        throw Error((ast & ST_TIMEOUT) ? PORSOL_ERR_TIMEOUT : PORSOL_ERR_BAD_ARG,
-                    "AMG smoother: bulk copy of the matrix slices failed (wait gave up or staging area too small)");
-    }
+        st.amg_levels = amg.levels();
+        return bcg3.solve(stream, P, val.p, amg, batch, b3, x3, o.residual_tolerance, maxit);
+    };
+    const CgResult r = mixed ? run(amg32, val32.p) : run(amg64, val.p);
     st.iterations = r.iterations;
-    st.outer_iterations = 1;
     st.reduction = r.reduction;
+    st.ms_krylov = now_ms() - t_begin - st.ms_precond_setup;
     if (r.breakdown) throw Error(PORSOL_ERR_NONFINITE, "CG breakdown (non-positive curvature)");
-    if (!r.converged) fail(r.iterations, r.reduction);
+    if (!r.converged) not_converged(r.iterations, r.reduction);
 }
 
 void porsol_solver::solve(const porsol_fluid* fluid, const double* sat, const double* mobd, const int* bct,
@@ -903,20 +858,46 @@ void porsol_solver::upscale(const porsol_grid* grid, int ngrids, const int* cell
     up_last = UpscaleSchedule{};
     auto finish = [&] {
         assemble_only = false;
-        reuse_amg = false;
         reg_rows.clear();
         batch.nblk = 0;
     };
-    if (upscale_schedule == PORSOL_UPSCALE_PERSISTENT) {
-        // the three systems differ only in their right-hand sides: assemble each (matrix and
-        // pinned rows), keep its right-hand side, solve all sub-grids and directions in one
-        // launch, then recover each direction's fluxes
-        try {
+    auto tensors = [&](int d) {   // column d of the effective tensors from the recovered fluxes
+        launch_side_fluxes(stream, ngrids, cellpos_d.p, facepos.p, side_d.p, outflux.p, q_d.p);
+        q_d.download(q.data(), q.size(), stream);
+        PORSOL_CUDA(cudaStreamSynchronize(stream));
+        for (int g = 0; g < ngrids; ++g)
+            for (int i = 0; i < 3; ++i)
+                keff[9 * size_t(g) + 3 * i + d] = L[3 * size_t(g) + d] * q[3 * size_t(g) + i] / A[3 * size_t(g) + i];
+    };
+    const bool persistent = upscale_schedule == PORSOL_UPSCALE_PERSISTENT;
+    try {
+        if (!persistent && o.linsolver_type == 0) {
+            for (int d = 0; d < 3; ++d) {
+                jumps(d);
+                porsol_solve_stats st{};
+                solve(&fl, up_ones.p, up_zeros.p, in_bctype.p, up_bcv.p, up_zeros.p, &o, &st, true);
+                tensors(d);
+                acc.iterations += st.iterations;
+                acc.outer_iterations += st.outer_iterations;
+                acc.reduction = std::max(acc.reduction, st.reduction);
+                acc.mass_balance = std::max(acc.mass_balance, st.mass_balance);
+                acc.ms_assemble += st.ms_assemble;
+                acc.ms_precond_setup += st.ms_precond_setup;
+                acc.ms_krylov += st.ms_krylov;
+                acc.ms_recover += st.ms_recover;
+            }
+        } else {
+            // the three systems differ only in their right-hand sides: assemble each (matrix and pinned
+            // rows), keep its right-hand side and starting vector, solve the three directions together
+            // (in one persistent launch, or batched CG around one AMG hierarchy), then recover each
+            // direction's fluxes
             const int N = S.N;
             up_b3.alloc(3 * size_t(N));
             up_x3.alloc(3 * size_t(N));
-            o.precision = PORSOL_MIXED;   // the assembly also writes the FP32 copy of the matrix
-            o.linsolver_type = 1;
+            if (persistent) {
+                o.precision = PORSOL_MIXED;   // the assembly also writes the FP32 copy of the matrix
+                o.linsolver_type = 1;
+            }
             for (int d = 0; d < 3; ++d) {
                 jumps(d);
                 porsol_solve_stats st{};
@@ -924,86 +905,55 @@ void porsol_solver::upscale(const porsol_grid* grid, int ngrids, const int* cell
                 solve(&fl, up_ones.p, up_zeros.p, in_bctype.p, up_bcv.p, up_zeros.p, &o, &st, true);
                 assemble_only = false;
                 launch_put3(stream, N, rhs.p, up_b3.p, d);
+                if (!persistent) {
+                    dirichlet_guess(stream, S.pat, val.p, rhs.p, x.p);
+                    launch_put3(stream, N, x.p, up_x3.p, d);
+                }
                 acc.ms_assemble += st.ms_assemble;
             }
-            const double t0 = now_ms();
-            // 0: the unknowns of the largest sub-grid (each sub-grid is its own system)
-            int largest = 1;
-            for (size_t g = 0; g + 3 < batch.h.size(); g += 4)
-                largest = std::max(largest, (batch.h[g + 1] - batch.h[g]) + (batch.h[g + 3] - batch.h[g + 2]));
-            const int maxit = o.linsolver_maxit > 0 ? o.linsolver_maxit : largest;
-            const UpscaleResult r = pup.solve(stream, S.pat, val.p, val32.p, batch.h, batch.ranges.p, up_b3.p,
-                                              up_x3.p, o.residual_tolerance,
-                                              o.inner_tolerance > 0 ? o.inner_tolerance : 3e-3, maxit, upscale_fixed);
-            up_last = pup.last_schedule();
-            acc.ms_krylov = now_ms() - t0;
-            bytes_krylov = pup.bytes();
-            vcycle_level_bytes.clear();
-            if (r.breakdown) throw Error(PORSOL_ERR_NONFINITE, "CG breakdown (non-positive curvature)");
-            if (!r.converged) {
-                std::ostringstream os;
-                os << "Linear solver failed to converge in " << maxit << " iterations.\n"
-                   << "Residual reduction achieved is " << r.reduction << '\n';
-                throw Error(PORSOL_ERR_NOT_CONVERGED, os.str());
+            int layout = 0;
+            if (persistent) {
+                const double t0 = now_ms();
+                // 0: the unknowns of the largest sub-grid (each sub-grid is its own system)
+                int largest = 1;
+                for (size_t g = 0; g + 3 < batch.h.size(); g += 4)
+                    largest = std::max(largest, (batch.h[g + 1] - batch.h[g]) + (batch.h[g + 3] - batch.h[g + 2]));
+                const int maxit = o.linsolver_maxit > 0 ? o.linsolver_maxit : largest;
+                const UpscaleResult r = pup.solve(stream, S.pat, val.p, val32.p, batch.h, batch.ranges.p, up_b3.p,
+                                                  up_x3.p, o.residual_tolerance,
+                                                  o.inner_tolerance > 0 ? o.inner_tolerance : 3e-3, maxit, upscale_fixed);
+                up_last = pup.last_schedule();
+                layout = up_last.layout;
+                acc.ms_krylov = now_ms() - t0;
+                bytes_krylov = pup.bytes();
+                vcycle_level_bytes.clear();
+                if (r.breakdown) throw Error(PORSOL_ERR_NONFINITE, "CG breakdown (non-positive curvature)");
+                if (!r.converged) not_converged(maxit, r.reduction);
+                acc.iterations = 3 * r.iterations;
+                acc.outer_iterations = 1;
+                acc.reduction = r.reduction;
+                acc.amg_levels = 0;
+            } else {
+                porsol_solve_stats st{};
+                batched_solve3(o, st, up_b3.p, up_x3.p);
+                st.ms_assemble = acc.ms_assemble;
+                acc = st;
             }
-            acc.iterations = 3 * r.iterations;
-            acc.outer_iterations = 1;
-            acc.reduction = r.reduction;
-            acc.amg_levels = 0;
             for (int d = 0; d < 3; ++d) {
-                launch_get3(stream, N, up_x3.p, x.p, d, up_last.layout);
+                launch_get3(stream, N, up_x3.p, x.p, d, layout);
                 porsol_solve_stats st{};
                 recover_solution(st);
                 acc.mass_balance = std::max(acc.mass_balance, st.mass_balance);
                 acc.ms_recover += st.ms_recover;
-                launch_side_fluxes(stream, ngrids, cellpos_d.p, facepos.p, side_d.p, outflux.p, q_d.p);
-                q_d.download(q.data(), q.size(), stream);
-                PORSOL_CUDA(cudaStreamSynchronize(stream));
-                for (int g = 0; g < ngrids; ++g)
-                    for (int i = 0; i < 3; ++i)
-                        keff[9 * size_t(g) + 3 * i + d] =
-                            L[3 * size_t(g) + d] * q[3 * size_t(g) + i] / A[3 * size_t(g) + i];
+                tensors(d);
             }
             solved = true;
-        } catch (...) {
-            finish();
-            throw;
-        }
-        finish();
-        if (stats) *stats = acc;
-        return;
-    }
-    try {
-        for (int d = 0; d < 3; ++d) {
-            jumps(d);
-            reuse_amg = d > 0;
-            porsol_solve_stats st{};
-            solve(&fl, up_ones.p, up_zeros.p, in_bctype.p, up_bcv.p, up_zeros.p, &o, &st, true);
-            launch_side_fluxes(stream, ngrids, cellpos_d.p, facepos.p, side_d.p, outflux.p, q_d.p);
-            q_d.download(q.data(), q.size(), stream);
-            PORSOL_CUDA(cudaStreamSynchronize(stream));
-            for (int g = 0; g < ngrids; ++g)
-                for (int i = 0; i < 3; ++i)
-                    keff[9 * size_t(g) + 3 * i + d] = L[3 * size_t(g) + d] * q[3 * size_t(g) + i] / A[3 * size_t(g) + i];
-            acc.iterations += st.iterations;
-            acc.outer_iterations += st.outer_iterations;
-            acc.reduction = std::max(acc.reduction, st.reduction);
-            acc.amg_levels = st.amg_levels;
-            acc.mass_balance = std::max(acc.mass_balance, st.mass_balance);
-            acc.ms_assemble += st.ms_assemble;
-            acc.ms_precond_setup += st.ms_precond_setup;
-            acc.ms_krylov += st.ms_krylov;
-            acc.ms_recover += st.ms_recover;
         }
     } catch (...) {
-        reuse_amg = false;
-        reg_rows.clear();
-        batch.nblk = 0;
+        finish();
         throw;
     }
-    reuse_amg = false;
-    reg_rows.clear();
-    batch.nblk = 0;
+    finish();
     if (stats) *stats = acc;
 }
 

@@ -748,16 +748,18 @@ __global__ void __launch_bounds__(256) k_cheb_setup(int n, const int* __restrict
     }
 }
 
+// The kernels of the cycle work on vector elements VT: T itself, or V3<T> for the three right-hand sides of a
+// batched upscaling solve at once.
 // start from x = 0: r = D^-1 b, d = r / theta
-template <class T>
-__global__ void k_cheb_start0(int n, const T* __restrict__ dinv, const T* __restrict__ b, T* __restrict__ r,
-                              T* __restrict__ d, T inv_theta, const int* stop, const unsigned char* __restrict__ act)
+template <class VT, class T = scalar_t<VT>>
+__global__ void k_cheb_start0(int n, const T* __restrict__ dinv, const VT* __restrict__ b, VT* __restrict__ r,
+                              VT* __restrict__ d, T inv_theta, const int* stop, const unsigned char* __restrict__ act)
 {
     chain_wait();
     if (*stop) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n || slice_idle(act, i, n)) return;
-    const T ri = dinv[i] * b[i];
+    const VT ri = dinv[i] * b[i];
     r[i] = ri;
     d[i] = ri * inv_theta;
 }
@@ -766,18 +768,18 @@ __global__ void k_cheb_start0(int n, const T* __restrict__ dinv, const T* __rest
 // sum_j a_rj x(j) for row r: the coalesced one-thread-per-row form for K = 1, the SELL-32x4 copy
 // (sp, col, A its slice offsets, columns and FP16 values) for K = 0, the SELL-32x4 copy with 16-bit
 // column offsets (col: CI = short) for K = -1, K lanes otherwise
-template <int K, class T, class V, class XF, class CI>
-__device__ __forceinline__ T row_dot(const int* __restrict__ sp, const CI* __restrict__ col, const V* __restrict__ A,
+template <int K, class VT, class V, class XF, class CI>
+__device__ __forceinline__ VT row_dot(const int* __restrict__ sp, const CI* __restrict__ col, const V* __restrict__ A,
                                      const int* __restrict__ rowlen, int r, int q, bool valid, XF xf)
 {
     if constexpr (K == -1) {
-        return valid ? sell4_dot16<T>(sp, col, A, r, xf) : T(0);
+        return valid ? sell4_dot16<VT>(sp, col, A, r, xf) : VT{};
     } else if constexpr (K == 0) {
-        return valid ? sell4_dot<T>(sp, col, A, r, xf) : T(0);
+        return valid ? sell4_dot<VT>(sp, col, A, r, xf) : VT{};
     } else if constexpr (K == 1) {
-        return valid ? sell_dot<T>(sp, col, A, r, xf) : T(0);
+        return valid ? sell_dot<VT>(sp, col, A, r, xf) : VT{};
     } else {
-        return sell_dot_lanes<K, T>(sp, col, A, rowlen, r, q, valid, xf);
+        return sell_dot_lanes<K, VT>(sp, col, A, rowlen, r, q, valid, xf);
     }
 }
 
@@ -785,12 +787,12 @@ __device__ __forceinline__ T row_dot(const int* __restrict__ sp, const CI* __res
 // row dot already carries the 1/a_ii factor; the unscaled residual multiplies it back by a_ii.
 
 // start from y = t + w P xc (xc may be null: y = t): x = y, r = D^-1 (b - A y), d = r / theta
-template <class T, int K, class V, bool SCALED, class CI = int>
+template <class VT, int K, class V, bool SCALED, class CI = int, class T = scalar_t<VT>>
 __global__ void k_cheb_start(int n, const int* __restrict__ sp, const CI* __restrict__ col,
                              const int* __restrict__ rowlen, const V* __restrict__ A, const T* __restrict__ dinv,
-                             const T* __restrict__ b, const T* __restrict__ t, const T* __restrict__ xc,
-                             const int* __restrict__ agg, T wp, T* __restrict__ x, T* __restrict__ r,
-                             T* __restrict__ d, T inv_theta, const int* stop, const unsigned char* __restrict__ act)
+                             const VT* __restrict__ b, const VT* __restrict__ t, const VT* __restrict__ xc,
+                             const int* __restrict__ agg, T wp, VT* __restrict__ x, VT* __restrict__ r,
+                             VT* __restrict__ d, T inv_theta, const int* stop, const unsigned char* __restrict__ act)
 {
     chain_wait();
     if (*stop) return;
@@ -799,44 +801,44 @@ __global__ void k_cheb_start(int n, const int* __restrict__ sp, const CI* __rest
     if (slice_idle(act, i, n)) return;
     const bool valid = i < n;
     if (K <= 1 && !valid) return;
-    T acc;
+    VT acc;
     if (xc) {
-        acc = row_dot<K, T>(sp, col, A, rowlen, i, q, valid, [t, xc, agg, wp](int j) {
+        acc = row_dot<K, VT>(sp, col, A, rowlen, i, q, valid, [t, xc, agg, wp](int j) {
             const int aj = agg[j];
-            return t[j] + (aj >= 0 ? wp * xc[aj] : T(0));
+            return aj >= 0 ? VT(t[j] + wp * xc[aj]) : t[j];
         });
     } else {
-        acc = row_dot<K, T>(sp, col, A, rowlen, i, q, valid, [t](int j) { return t[j]; });
+        acc = row_dot<K, VT>(sp, col, A, rowlen, i, q, valid, [t](int j) { return t[j]; });
     }
     if (!valid || q != 0) return;
     if (xc) {
         const int ai = agg[i];
-        x[i] = t[i] + (ai >= 0 ? wp * xc[ai] : T(0));
+        x[i] = ai >= 0 ? VT(t[i] + wp * xc[ai]) : t[i];
     }
-    const T ri = SCALED ? dinv[i] * b[i] - acc : dinv[i] * (b[i] - acc);
+    const VT ri = SCALED ? VT(dinv[i] * b[i] - acc) : VT(dinv[i] * (b[i] - acc));
     r[i] = ri;
     d[i] = ri * inv_theta;
 }
 
 // y = t + w P xc (the coarse correction), for the levels whose smoother then gathers one vector
-template <class T>
-__global__ void k_prolong_add(int n, const T* __restrict__ t, const T* __restrict__ xc, const int* __restrict__ agg,
-                              T wp, T* __restrict__ y, const int* stop, const unsigned char* __restrict__ act)
+template <class VT, class T = scalar_t<VT>>
+__global__ void k_prolong_add(int n, const VT* __restrict__ t, const VT* __restrict__ xc, const int* __restrict__ agg,
+                              T wp, VT* __restrict__ y, const int* stop, const unsigned char* __restrict__ act)
 {
     chain_wait();
     if (*stop) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n || slice_idle(act, i, n)) return;
     const int ai = agg[i];
-    y[i] = t[i] + (ai >= 0 ? wp * xc[ai] : T(0));
+    y[i] = ai >= 0 ? VT(t[i] + wp * xc[ai]) : t[i];
 }
 
 // x_out = x_in + d_in; r -= D^-1 A d_in; d_out = c1 d_in + c2 r; final: x_out += d_out
-template <class T, int K, class V, bool SCALED, class CI = int>
+template <class VT, int K, class V, bool SCALED, class CI = int, class T = scalar_t<VT>>
 __global__ void k_cheb_step(int n, const int* __restrict__ sp, const CI* __restrict__ col,
                             const int* __restrict__ rowlen, const V* __restrict__ A, const T* __restrict__ dinv,
-                            const T* x_in, const T* __restrict__ d_in, T* __restrict__ r, T* __restrict__ d_out,
-                            T* x_out, T c1, T c2, int final_step, const int* stop,
+                            const VT* x_in, const VT* __restrict__ d_in, VT* __restrict__ r, VT* __restrict__ d_out,
+                            VT* x_out, T c1, T c2, int final_step, const int* stop,
                             const unsigned char* __restrict__ act)
 {
     chain_wait();
@@ -848,26 +850,27 @@ __global__ void k_cheb_step(int n, const int* __restrict__ sp, const CI* __restr
     if (K <= 1 && !valid) return;
     // FP32: the row's own values are loaded before the row dot, so their loads overlap its gathers
     // (in FP64 the early values would take the kernel past 32 registers)
-    constexpr bool early = sizeof(T) == 4;
+    constexpr bool early = sizeof(VT) == 4;
     const bool own = valid && q == 0;
-    T di = T(0), xo = T(0), r0 = T(0), dv = T(0);
+    VT di{}, xo{}, r0{};
+    T dv = T(0);
     if (early && own) {
         di = d_in[i];
-        xo = x_in ? x_in[i] : T(0);
+        if (x_in) xo = x_in[i];
         r0 = r[i];
         if (!SCALED) dv = dinv[i];
     }
-    const T acc = row_dot<K, T>(sp, col, A, rowlen, i, q, valid, [d_in](int j) { return d_in[j]; });
+    const VT acc = row_dot<K, VT>(sp, col, A, rowlen, i, q, valid, [d_in](int j) { return d_in[j]; });
     if (!own) return;
     if (!early) {
         di = d_in[i];
-        xo = x_in ? x_in[i] : T(0);
+        if (x_in) xo = x_in[i];
         r0 = r[i];
         if (!SCALED) dv = dinv[i];
     }
-    T xi = xo + di;
-    const T ri = SCALED ? r0 - acc : r0 - dv * acc;
-    const T dn = c1 * di + c2 * ri;
+    VT xi = xo + di;
+    const VT ri = SCALED ? VT(r0 - acc) : VT(r0 - dv * acc);
+    const VT dn = c1 * di + c2 * ri;
     if (final_step) xi += dn;
     r[i] = ri;
     d_out[i] = dn;
@@ -976,10 +979,10 @@ __global__ void __launch_bounds__(BULK_SLICES * 32)
     x_out[i] = xi;
 }
 
-template <class T, int K, class V, bool SCALED, class CI = int>
+template <class VT, int K, class V, bool SCALED, class CI = int, class T = scalar_t<VT>>
 __global__ void k_resid(int n, const int* __restrict__ sp, const CI* __restrict__ col, const int* __restrict__ rowlen,
-                        const V* __restrict__ A, const T* __restrict__ diagv, const T* __restrict__ b,
-                        const T* __restrict__ x, T* __restrict__ r, const int* stop,
+                        const V* __restrict__ A, const T* __restrict__ diagv, const VT* __restrict__ b,
+                        const VT* __restrict__ x, VT* __restrict__ r, const int* stop,
                         const unsigned char* __restrict__ act)
 {
     chain_wait();
@@ -989,9 +992,9 @@ __global__ void k_resid(int n, const int* __restrict__ sp, const CI* __restrict_
     if (slice_idle(act, i, n)) return;
     const bool valid = i < n;
     if (K <= 1 && !valid) return;
-    const T acc = row_dot<K, T>(sp, col, A, rowlen, i, q, valid, [x](int j) { return x[j]; });
+    const VT acc = row_dot<K, VT>(sp, col, A, rowlen, i, q, valid, [x](int j) { return x[j]; });
     if (!valid || q != 0) return;
-    r[i] = SCALED ? b[i] - diagv[i] * acc : b[i] - acc;
+    r[i] = SCALED ? VT(b[i] - diagv[i] * acc) : VT(b[i] - acc);
 }
 
 // D^-1 A in FP16 (padding slots stay 0) and the diagonal, for the scaled smoother
@@ -1092,35 +1095,35 @@ __global__ void k_scale_half4(int n, int nslices, const int* __restrict__ sp, co
     }
 }
 
-template <class T>
-__global__ void k_restrict(int nc, const int* __restrict__ ptr, const int* __restrict__ idx, const T* __restrict__ r,
-                           T* __restrict__ bc, const int* stop, const unsigned char* __restrict__ act)
+template <class VT>
+__global__ void k_restrict(int nc, const int* __restrict__ ptr, const int* __restrict__ idx, const VT* __restrict__ r,
+                           VT* __restrict__ bc, const int* stop, const unsigned char* __restrict__ act)
 {
     chain_wait();
     if (*stop) return;
     const int I = blockIdx.x * blockDim.x + threadIdx.x;
     if (I >= nc || slice_idle(act, I, nc)) return;
-    T s = 0;
+    VT s{};
     for (int q = ptr[I]; q < ptr[I + 1]; ++q) s += r[idx[q]];
     bc[I] = s;
 }
 
 // k_restrict fused with the coarse level's first Chebyshev start from zero (k_cheb_start0 on bc):
 // the same sums, the same rc and dc
-template <class T>
+template <class VT, class T = scalar_t<VT>>
 __global__ void k_restrict_start0(int nc, const int* __restrict__ ptr, const int* __restrict__ idx,
-                                  const T* __restrict__ r, T* __restrict__ bc, const T* __restrict__ dinv_c,
-                                  T* __restrict__ rc, T* __restrict__ dc, T inv_theta, const int* stop,
+                                  const VT* __restrict__ r, VT* __restrict__ bc, const T* __restrict__ dinv_c,
+                                  VT* __restrict__ rc, VT* __restrict__ dc, T inv_theta, const int* stop,
                                   const unsigned char* __restrict__ act)
 {
     chain_wait();
     if (*stop) return;
     const int I = blockIdx.x * blockDim.x + threadIdx.x;
     if (I >= nc || slice_idle(act, I, nc)) return;
-    T s = 0;
+    VT s{};
     for (int q = ptr[I]; q < ptr[I + 1]; ++q) s += r[idx[q]];
     bc[I] = s;
-    const T ri = dinv_c[I] * s;
+    const VT ri = dinv_c[I] * s;
     rc[I] = ri;
     dc[I] = ri * inv_theta;
 }
@@ -1134,18 +1137,28 @@ __global__ void k_level_blocks(int nc, const int* __restrict__ ptr, const int* _
     if (I < nc) blk_c[I] = blk_f[idx[ptr[I]]];
 }
 
-// act[s] = 1 when a row of slice s belongs to a block still iterating (conv == 0); one warp per slice
-__global__ void k_slice_active(int n, int nslices, const int* __restrict__ blk, const int* __restrict__ conv,
-                               unsigned char* __restrict__ act, const int* stop)
+// act[s] = 1 when a row of slice s belongs to a block still iterating (conv == 0); one warp per slice, all
+// levels in one launch (a launch per level cost 4 us each, 5 % of an iteration on 48 sub-grids)
+struct SliceLevels {
+    static constexpr int MAX = 24;
+    int levels;
+    int first[MAX + 1];   // slices before each level
+    int n[MAX];
+    const int* blk[MAX];
+    unsigned char* act[MAX];
+};
+__global__ void k_slice_active(const __grid_constant__ SliceLevels S, const int* __restrict__ conv, const int* stop)
 {
     chain_wait();
     if (*stop) return;
-    const int sl = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (sl >= nslices) return;   // whole warps
-    const int r = sl * 32 + (threadIdx.x & 31);
-    const bool live = r < n && conv[blk[r]] == 0;
+    const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (w >= S.first[S.levels]) return;   // whole warps
+    int l = 0;
+    while (w >= S.first[l + 1]) ++l;
+    const int sl = w - S.first[l], r = sl * 32 + (threadIdx.x & 31);
+    const bool live = r < S.n[l] && conv[S.blk[l][r]] == 0;
     const unsigned any = __ballot_sync(0xffffffffu, live);
-    if ((threadIdx.x & 31) == 0) act[sl] = any ? 1 : 0;
+    if ((threadIdx.x & 31) == 0) S.act[l][sl] = any ? 1 : 0;
 }
 
 // ---------------- K-cycle (Krylov-accelerated coarse correction) ----------------
@@ -1401,30 +1414,32 @@ __global__ void __launch_bounds__(512, 1) k_dense_inverse(int n, const int* __re
     for (int q = tid; q < own * n; q += blockDim.x) Dinv[(size_t)r0 * n + q] = A[q];
 }
 
-template <class T>
-__global__ void k_dense_apply(int n, const double* __restrict__ Dinv, const T* __restrict__ b, T* __restrict__ x,
+template <class VT>
+__global__ void k_dense_apply(int n, const double* __restrict__ Dinv, const VT* __restrict__ b, VT* __restrict__ x,
                               const int* stop, const unsigned char* __restrict__ act, const int* __restrict__ blk,
                               const int* __restrict__ conv)
 {
     chain_wait();
     if (*stop) return;
-    extern __shared__ double sb[];
+    extern __shared__ __align__(16) unsigned char dense_smem[];
+    using W = wide_t<VT>;
+    W* sb = reinterpret_cast<W*>(dense_smem);
     // batched solves (blk, conv not null): the block-diagonal inverse couples nothing across blocks,
     // but its zeros would still carry a converged block's values (0 * Inf is NaN), so those enter as
     // 0: a converged block's rows are only partly recomputed, from partly stale inputs, and in FP32
     // that mix can overflow
-    for (int j = threadIdx.x; j < n; j += blockDim.x) sb[j] = (conv && conv[blk[j]] != 0) ? 0.0 : double(b[j]);
+    for (int j = threadIdx.x; j < n; j += blockDim.x) sb[j] = (conv && conv[blk[j]] != 0) ? W{} : to_wide(b[j]);
     __syncthreads();
     // one warp per row, blockDim/32 rows per block: a large coarsest level (up to 2048 rows
     // when coarsening stalls) spreads over many SMs instead of one
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int i = blockIdx.x * nw + warp;
     if (i >= n || slice_idle(act, i, n)) return;   // one row per warp
-    double s = 0.0;
-    for (int j = lane; j < n; j += 32) s += Dinv[(size_t)i * n + j] * sb[j];
+    W s{};
+    for (int j = lane; j < n; j += 32) s = multiply_add(s, Dinv[(size_t)i * n + j], sb[j]);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) x[i] = T(s);
+    for (int o = 16; o > 0; o >>= 1) s += shfl_xor(s, o);
+    if (lane == 0) x[i] = from_wide<VT>(s);
 }
 
 int read_int(cudaStream_t s, const int* d)
@@ -1800,10 +1815,11 @@ void Amg<T>::smoother_setup(cudaStream_t s, Level& L, int level)
             n, L.P->slice_ptr.p, L.P->rowlen.p, L.P->diag.p, L.A, L.dinv.p, L.ah.p, L.diagv.p));
         PORSOL_CUDA(cudaGetLastError());
     }
-    L.t.alloc(n);
-    L.r.alloc(n);
-    L.d0.alloc(n);
-    L.d1.alloc(n);
+    const size_t nv = size_t(n) * vec_width();
+    L.t.alloc(nv);
+    L.r.alloc(nv);
+    L.d0.alloc(nv);
+    L.d1.alloc(nv);
     L.lanes = L.v4 ? 1 : tune_lanes(s, L);
     // coarse levels smoothed one thread per row on the plain layout (FP64 hierarchies): 16-bit column
     // offsets as the system matrix has them, when the level's couplings allow (checked in setup())
@@ -1984,8 +2000,8 @@ void Amg<T>::setup(cudaStream_t s, const SellPattern& P0, const T* A0, const Amg
         next.n = L.agg.nc;
         next.P = &next.own;
         next.A = next.own_val.p;
-        next.b.alloc(std::max(next.n, 1));
-        next.x.alloc(std::max(next.n, 1));
+        next.b.alloc(size_t(std::max(next.n, 1)) * vec_width());
+        next.x.alloc(size_t(std::max(next.n, 1)) * vec_width());
         sizes_.push_back(next.n);
         nnzs_.push_back(next.own.nent);
         ++nlev_;
@@ -2053,6 +2069,7 @@ void Amg<T>::setup(cudaStream_t s, const SellPattern& P0, const T* A0, const Amg
             for (DBuf<T>* v : {&K.kc1, &K.kc2, &K.kv1, &K.kv2, &K.kr2}) v->alloc(std::max(K.n, 1));
         }
     Level& C = *lv_[nlev_ - 1];
+    PORSOL_REQUIRE(nlev_ <= SliceLevels::MAX, PORSOL_ERR_BAD_ARG, "AMG: too many levels");
     PORSOL_REQUIRE(C.n <= 2048, PORSOL_ERR_BAD_ARG, "AMG: coarsening stalled above the dense-solve limit");
     build_coarse_solver(s, *C.P, C.A, C.n);
     targs_.cinv = cinv_.p;
@@ -2151,9 +2168,13 @@ int Amg<T>::solve_status(cudaStream_t s) const
 // One Chebyshev application (degree o_.cheb_degree) on [lmax/30, lmax]:
 //   from_zero: x = p(D^-1 A) D^-1 b;  otherwise from y = x0 (+ w P xc when xc is given).
 template <class T>
-void Amg<T>::chebyshev(cudaStream_t s, Level& L, const T* b, T* x, bool from_zero, const T* xc, const int* agg,
+template <class VT>
+void Amg<T>::chebyshev(cudaStream_t s, Level& L, const VT* b, VT* x, bool from_zero, const VT* xc, const int* agg,
                        const int* stop, bool started)
 {
+    constexpr bool one = !is_v3<VT>;   // the FP16 and staged forms exist for one right-hand side
+    VT* const Lr = work<VT>(L.r);
+    VT* const Lt = work<VT>(L.t);
     const int n = L.n;
     const int nb = div_up(n, TB);
     const SellPattern& P = *L.P;
@@ -2161,44 +2182,49 @@ void Amg<T>::chebyshev(cudaStream_t s, Level& L, const T* b, T* x, bool from_zer
     const double theta = 0.5 * (bmax + amin), delta = 0.5 * (bmax - amin);
     const double sigma = theta / delta;
     double rho = 1.0 / sigma;
-    T* d = L.d0.p;
-    T* dn = L.d1.p;
+    VT* d = work<VT>(L.d0);
+    VT* dn = work<VT>(L.d1);
     const unsigned char* act = level_act(L);
     if (from_zero) {
-        if (!started) chain(k_cheb_start0<T>, nb, TB, 0, s, n, L.dinv.p, b, L.r.p, d, T(1.0 / theta), stop, act);
+        if (!started) chain(k_cheb_start0<VT>, nb, TB, 0, s, n, L.dinv.p, b, Lr, d, T(1.0 / theta), stop, act);
     } else {
         // x holds the start vector (or the pre-smoothed t when xc is given; then x gets y)
-        const T* t = xc ? L.t.p : x;
+        const VT* t = xc ? Lt : x;
         const int nbk = div_up(n * L.lanes, TB);
         // levels smoothed one thread per row (the large ones): form y = t + w P xc first, so the
         // start's row dot gathers one vector instead of t, agg and xc (the same y, the same sums)
         if (xc && L.lanes == 1) {
-            chain(k_prolong_add<T>, nb, TB, 0, s, n, t, xc, agg, T(o_.prolong), x, stop, act);
+            chain(k_prolong_add<VT>, nb, TB, 0, s, n, t, xc, agg, T(o_.prolong), x, stop, act);
             t = x;
             xc = nullptr;
         }
-        if (L.v4 && L.c16) {
-            chain(k_cheb_start<T, -1, __half, true, short>, nb, TB, 0, s, n, L.sp4.p, L.off4.p, nullptr, L.ah4.p,
-                L.dinv.p, b, x, nullptr, nullptr, T(o_.prolong), x, L.r.p, d, T(1.0 / theta), stop, act);
-        } else if (L.v4) {
-            chain(k_cheb_start<T, 0, __half, true>, nb, TB, 0, s, n, L.sp4.p, L.col4.p, nullptr, L.ah4.p, L.dinv.p, b,
-                x, nullptr, nullptr, T(o_.prolong), x, L.r.p, d, T(1.0 / theta), stop, act);
-        } else if (L.half) {
-            PORSOL_LANES(L.lanes, chain(k_cheb_start<T, KL, __half, true>, nbk, TB, 0, s, n, P.slice_ptr.p, P.col.p,
-                P.rowlen.p, L.ah.p, L.dinv.p, b, t, xc, agg, T(o_.prolong), x, L.r.p, d, T(1.0 / theta), stop, act));
+        if (one && L.half) {
+            if constexpr (one) {
+                if (L.v4 && L.c16) {
+                    chain(k_cheb_start<T, -1, __half, true, short>, nb, TB, 0, s, n, L.sp4.p, L.off4.p, nullptr, L.ah4.p,
+                        L.dinv.p, b, x, nullptr, nullptr, T(o_.prolong), x, Lr, d, T(1.0 / theta), stop, act);
+                } else if (L.v4) {
+                    chain(k_cheb_start<T, 0, __half, true>, nb, TB, 0, s, n, L.sp4.p, L.col4.p, nullptr, L.ah4.p,
+                        L.dinv.p, b, x, nullptr, nullptr, T(o_.prolong), x, Lr, d, T(1.0 / theta), stop, act);
+                } else {
+                    PORSOL_LANES(L.lanes, chain(k_cheb_start<T, KL, __half, true>, nbk, TB, 0, s, n, P.slice_ptr.p,
+                        P.col.p, P.rowlen.p, L.ah.p, L.dinv.p, b, t, xc, agg, T(o_.prolong), x, Lr, d, T(1.0 / theta),
+                        stop, act));
+                }
+            }
         } else if (plain16(L)) {
-            chain(k_cheb_start<T, 1, T, false, short>, nb, TB, 0, s, n, P.slice_ptr.p, P.off16.p, P.rowlen.p, L.A,
-                L.dinv.p, b, t, xc, agg, T(o_.prolong), x, L.r.p, d, T(1.0 / theta), stop, act);
+            chain(k_cheb_start<VT, 1, T, false, short>, nb, TB, 0, s, n, P.slice_ptr.p, P.off16.p, P.rowlen.p, L.A,
+                L.dinv.p, b, t, xc, agg, T(o_.prolong), x, Lr, d, T(1.0 / theta), stop, act);
         } else {
-            PORSOL_LANES(L.lanes, chain(k_cheb_start<T, KL, T, false>, nbk, TB, 0, s, n, P.slice_ptr.p, P.col.p,
-                P.rowlen.p, L.A, L.dinv.p, b, t, xc, agg, T(o_.prolong), x, L.r.p, d, T(1.0 / theta), stop, act));
+            PORSOL_LANES(L.lanes, chain(k_cheb_start<VT, KL, T, false>, nbk, TB, 0, s, n, P.slice_ptr.p, P.col.p,
+                P.rowlen.p, L.A, L.dinv.p, b, t, xc, agg, T(o_.prolong), x, Lr, d, T(1.0 / theta), stop, act));
         }
     }
     const int deg = std::max(1, o_.cheb_degree);
     for (int k = 1; k <= deg; ++k) {
         const double rho1 = 1.0 / (2.0 * sigma - rho);
         const double c1 = rho1 * rho, c2 = 2.0 * rho1 / delta;
-        const T* xin = (from_zero && k == 1) ? nullptr : x;
+        const VT* xin = (from_zero && k == 1) ? nullptr : x;
         // algorithmic bytes: matrix values + columns (16-bit offsets on c16 levels), d gathered
         // once, dinv (unscaled form only), r and x in, r/d/x out
         const double bytes = double(P.nent) * ((L.half ? 2 : sizeof(T)) +
@@ -2208,33 +2234,37 @@ void Amg<T>::chebyshev(cudaStream_t s, Level& L, const T* b, T* x, bool from_zer
         cudaEvent_t ev = nullptr;
         if (prof_here) prof_->begin(s, PK_CHEB, bytes, &ev);
         const int nbk = div_up(n * L.lanes, TB);
-        if (L.bulk_groups > 0 && L.c16) {
-            const int cap = 128 * L.bulk_groups;   // entries per slice
-            const size_t shm = 128 + size_t(BULK_SLICES) * cap * 4;
-            chain(k_cheb_step_bulk<T, short>, div_up(P.nslices, BULK_SLICES), BULK_SLICES * 32, shm, s, n, P.nslices,
-                L.sp4.p, L.off4.p, L.ah4.p, xin, d, L.r.p, dn, x, T(c1), T(c2), k == deg ? 1 : 0, stop, cap,
-                status_.p, 0u);
-        } else if (L.bulk_groups > 0) {
-            const int cap = 128 * L.bulk_groups;   // entries per slice
-            const size_t shm = 128 + size_t(BULK_SLICES) * cap * 6;
-            chain(k_cheb_step_bulk<T, int>, div_up(P.nslices, BULK_SLICES), BULK_SLICES * 32, shm, s, n, P.nslices,
-                L.sp4.p, L.col4.p, L.ah4.p, xin, d, L.r.p, dn, x, T(c1), T(c2), k == deg ? 1 : 0, stop, cap,
-                status_.p, 0u);
-        } else if (L.v4 && L.c16) {
-            chain(k_cheb_step<T, -1, __half, true, short>, nb, TB, 0, s, n, L.sp4.p, L.off4.p, nullptr, L.ah4.p,
-                L.dinv.p, xin, d, L.r.p, dn, x, T(c1), T(c2), k == deg ? 1 : 0, stop, act);
-        } else if (L.v4) {
-            chain(k_cheb_step<T, 0, __half, true>, nb, TB, 0, s, n, L.sp4.p, L.col4.p, nullptr, L.ah4.p, L.dinv.p,
-                xin, d, L.r.p, dn, x, T(c1), T(c2), k == deg ? 1 : 0, stop, act);
-        } else if (L.half) {
-            PORSOL_LANES(L.lanes, chain(k_cheb_step<T, KL, __half, true>, nbk, TB, 0, s, n, P.slice_ptr.p, P.col.p,
-                P.rowlen.p, L.ah.p, L.dinv.p, xin, d, L.r.p, dn, x, T(c1), T(c2), k == deg ? 1 : 0, stop, act));
+        if (one && L.half) {
+            if constexpr (one) {
+                if (L.bulk_groups > 0 && L.c16) {
+                    const int cap = 128 * L.bulk_groups;   // entries per slice
+                    const size_t shm = 128 + size_t(BULK_SLICES) * cap * 4;
+                    chain(k_cheb_step_bulk<T, short>, div_up(P.nslices, BULK_SLICES), BULK_SLICES * 32, shm, s, n, P.nslices,
+                        L.sp4.p, L.off4.p, L.ah4.p, xin, d, Lr, dn, x, T(c1), T(c2), k == deg ? 1 : 0, stop, cap,
+                        status_.p, 0u);
+                } else if (L.bulk_groups > 0) {
+                    const int cap = 128 * L.bulk_groups;   // entries per slice
+                    const size_t shm = 128 + size_t(BULK_SLICES) * cap * 6;
+                    chain(k_cheb_step_bulk<T, int>, div_up(P.nslices, BULK_SLICES), BULK_SLICES * 32, shm, s, n, P.nslices,
+                        L.sp4.p, L.col4.p, L.ah4.p, xin, d, Lr, dn, x, T(c1), T(c2), k == deg ? 1 : 0, stop, cap,
+                        status_.p, 0u);
+                } else if (L.v4 && L.c16) {
+                    chain(k_cheb_step<T, -1, __half, true, short>, nb, TB, 0, s, n, L.sp4.p, L.off4.p, nullptr, L.ah4.p,
+                        L.dinv.p, xin, d, Lr, dn, x, T(c1), T(c2), k == deg ? 1 : 0, stop, act);
+                } else if (L.v4) {
+                    chain(k_cheb_step<T, 0, __half, true>, nb, TB, 0, s, n, L.sp4.p, L.col4.p, nullptr, L.ah4.p, L.dinv.p,
+                        xin, d, Lr, dn, x, T(c1), T(c2), k == deg ? 1 : 0, stop, act);
+                } else if (L.half) {
+                    PORSOL_LANES(L.lanes, chain(k_cheb_step<T, KL, __half, true>, nbk, TB, 0, s, n, P.slice_ptr.p, P.col.p,
+                        P.rowlen.p, L.ah.p, L.dinv.p, xin, d, Lr, dn, x, T(c1), T(c2), k == deg ? 1 : 0, stop, act));
+                }
+            }
         } else if (plain16(L)) {
-            chain(k_cheb_step<T, 1, T, false, short>, nb, TB, 0, s, n, P.slice_ptr.p, P.off16.p, P.rowlen.p, L.A,
-                L.dinv.p, xin, d, L.r.p, dn, x, T(c1), T(c2), k == deg ? 1 : 0, stop, act);
+            chain(k_cheb_step<VT, 1, T, false, short>, nb, TB, 0, s, n, P.slice_ptr.p, P.off16.p, P.rowlen.p, L.A,
+                L.dinv.p, xin, d, Lr, dn, x, T(c1), T(c2), k == deg ? 1 : 0, stop, act);
         } else {
-            PORSOL_LANES(L.lanes, chain(k_cheb_step<T, KL, T, false>, nbk, TB, 0, s, n, P.slice_ptr.p, P.col.p,
-                P.rowlen.p, L.A, L.dinv.p, xin, d, L.r.p, dn, x, T(c1), T(c2), k == deg ? 1 : 0, stop, act));
+            PORSOL_LANES(L.lanes, chain(k_cheb_step<VT, KL, T, false>, nbk, TB, 0, s, n, P.slice_ptr.p, P.col.p,
+                P.rowlen.p, L.A, L.dinv.p, xin, d, Lr, dn, x, T(c1), T(c2), k == deg ? 1 : 0, stop, act));
         }
         if (prof_here) prof_->end(s, PK_CHEB, bytes, ev);
         rho = rho1;
@@ -2244,11 +2274,13 @@ void Amg<T>::chebyshev(cudaStream_t s, Level& L, const T* b, T* x, bool from_zer
 }
 
 template <class T>
-void Amg<T>::vcycle(cudaStream_t s, int l, const T* b, T* x, const int* stop, bool started)
+template <class VT>
+void Amg<T>::vcycle(cudaStream_t s, int l, const VT* b, VT* x, const int* stop, bool started)
 {
+    constexpr bool one = !is_v3<VT>;
     if (l == nlev_ - 1) {
         if (nc_ > 0)
-            chain(k_dense_apply<T>, div_up(nc_, 8), 256, nc_ * sizeof(double), s, nc_, cinv_.p, b, x, stop,
+            chain(k_dense_apply<VT>, div_up(nc_, 8), 256, nc_ * sizeof(wide_t<VT>), s, nc_, cinv_.p, b, x, stop,
                 level_act(*lv_[size_t(l)]), lv_[size_t(l)]->blkp, level_act(*lv_[size_t(l)]) ? conv_ : nullptr);
         return;
     }
@@ -2258,24 +2290,30 @@ void Amg<T>::vcycle(cudaStream_t s, int l, const T* b, T* x, const int* stop, bo
     const int nb = div_up(n, TB);
     const SellPattern& P = *L.P;
     // pre-smoothing into t
-    chebyshev(s, L, b, L.t.p, true, nullptr, nullptr, stop, started);
-    for (int k = 1; k < o_.smooth_steps; ++k) chebyshev(s, L, b, L.t.p, false, nullptr, nullptr, stop);
+    const VT* none = nullptr;
+    VT *const Lt = work<VT>(L.t), *const Lr = work<VT>(L.r), *const Nb = work<VT>(Nx.b), *const Nxx = work<VT>(Nx.x);
+    chebyshev(s, L, b, Lt, true, none, nullptr, stop, started);
+    for (int k = 1; k < o_.smooth_steps; ++k) chebyshev(s, L, b, Lt, false, none, nullptr, stop);
     // restrict the residual
-    if (L.v4 && L.c16) {
-        chain(k_resid<T, -1, __half, true, short>, nb, TB, 0, s, n, L.sp4.p, L.off4.p, nullptr, L.ah4.p, L.diagv.p, b,
-            L.t.p, L.r.p, stop, level_act(L));
-    } else if (L.v4) {
-        chain(k_resid<T, 0, __half, true>, nb, TB, 0, s, n, L.sp4.p, L.col4.p, nullptr, L.ah4.p, L.diagv.p, b, L.t.p,
-            L.r.p, stop, level_act(L));
-    } else if (L.half) {
-        PORSOL_LANES(L.lanes, chain(k_resid<T, KL, __half, true>, div_up(n * L.lanes, TB), TB, 0, s, n, P.slice_ptr.p,
-            P.col.p, P.rowlen.p, L.ah.p, L.diagv.p, b, L.t.p, L.r.p, stop, level_act(L)));
+    if (one && L.half) {
+        if constexpr (one) {
+            if (L.v4 && L.c16) {
+                chain(k_resid<T, -1, __half, true, short>, nb, TB, 0, s, n, L.sp4.p, L.off4.p, nullptr, L.ah4.p, L.diagv.p, b,
+                    Lt, Lr, stop, level_act(L));
+            } else if (L.v4) {
+                chain(k_resid<T, 0, __half, true>, nb, TB, 0, s, n, L.sp4.p, L.col4.p, nullptr, L.ah4.p, L.diagv.p, b, Lt,
+                    Lr, stop, level_act(L));
+            } else if (L.half) {
+                PORSOL_LANES(L.lanes, chain(k_resid<T, KL, __half, true>, div_up(n * L.lanes, TB), TB, 0, s, n, P.slice_ptr.p,
+                    P.col.p, P.rowlen.p, L.ah.p, L.diagv.p, b, Lt, Lr, stop, level_act(L)));
+            }
+        }
     } else if (plain16(L)) {
-        chain(k_resid<T, 1, T, false, short>, nb, TB, 0, s, n, P.slice_ptr.p, P.off16.p, P.rowlen.p, L.A, L.diagv.p,
-            b, L.t.p, L.r.p, stop, level_act(L));
+        chain(k_resid<VT, 1, T, false, short>, nb, TB, 0, s, n, P.slice_ptr.p, P.off16.p, P.rowlen.p, L.A, L.diagv.p,
+            b, Lt, Lr, stop, level_act(L));
     } else {
-        PORSOL_LANES(L.lanes, chain(k_resid<T, KL, T, false>, div_up(n * L.lanes, TB), TB, 0, s, n, P.slice_ptr.p,
-            P.col.p, P.rowlen.p, L.A, L.diagv.p, b, L.t.p, L.r.p, stop, level_act(L)));
+        PORSOL_LANES(L.lanes, chain(k_resid<VT, KL, T, false>, div_up(n * L.lanes, TB), TB, 0, s, n, P.slice_ptr.p,
+            P.col.p, P.rowlen.p, L.A, L.diagv.p, b, Lt, Lr, stop, level_act(L)));
     }
     // the coarse level's cycle starts with a Chebyshev start from zero on Nx.b (its first cycle
     // under a K-cycle): done here, in the restriction; the coarsest level solves directly
@@ -2284,17 +2322,18 @@ void Amg<T>::vcycle(cudaStream_t s, int l, const T* b, T* x, const int* stop, bo
         targs_.stop = stop;
         tail_launch<T>(s, lv_[size_t(tail_)]->half, targs_, tail_shm_);
     } else if (fuse)
-        chain(k_restrict_start0<T>, div_up(Nx.n, TB), TB, 0, s, Nx.n, L.agg.ptr.p, L.agg.idx.p, L.r.p, Nx.b.p,
-            Nx.dinv.p, Nx.r.p, Nx.d0.p, T(cheb_inv_theta(Nx)), stop, level_act(Nx));
+        chain(k_restrict_start0<VT>, div_up(Nx.n, TB), TB, 0, s, Nx.n, L.agg.ptr.p, L.agg.idx.p, Lr, Nb,
+            Nx.dinv.p, work<VT>(Nx.r), work<VT>(Nx.d0), T(cheb_inv_theta(Nx)), stop, level_act(Nx));
     else
-        chain(k_restrict<T>, div_up(Nx.n, TB), TB, 0, s, Nx.n, L.agg.ptr.p, L.agg.idx.p, L.r.p, Nx.b.p, stop,
+        chain(k_restrict<VT>, div_up(Nx.n, TB), TB, 0, s, Nx.n, L.agg.ptr.p, L.agg.idx.p, Lr, Nb, stop,
             level_act(Nx));
-    if (l + 1 == tail_) {
-    } else if (k_level(l + 1)) kcycle(s, l + 1, Nx.b.p, Nx.x.p, stop, fuse);
-    else vcycle(s, l + 1, Nx.b.p, Nx.x.p, stop, fuse);
+    if (l + 1 != tail_) {
+        if (!k_level(l + 1)) vcycle(s, l + 1, (const VT*)Nb, Nxx, stop, fuse);
+        else if constexpr (one) kcycle(s, l + 1, Nb, Nxx, stop, fuse);   // batched solves run the V-cycle
+    }
     // post-smoothing from t + w P xc
-    chebyshev(s, L, b, x, false, Nx.x.p, L.agg.agg.p, stop);
-    for (int k = 1; k < o_.smooth_steps; ++k) chebyshev(s, L, b, x, false, nullptr, nullptr, stop);
+    chebyshev(s, L, b, x, false, (const VT*)Nxx, L.agg.agg.p, stop);
+    for (int k = 1; k < o_.smooth_steps; ++k) chebyshev(s, L, b, x, false, none, nullptr, stop);
     PORSOL_CUDA(cudaGetLastError());
 }
 
@@ -2407,14 +2446,27 @@ void Amg<T>::apply(cudaStream_t s, const T* r, T* z, const int* stop)
     ChainPause plain(prof_here);   // events between the kernels time each one
     cudaEvent_t ev = nullptr;
     if (prof_here) prof_->begin(s, PK_VCYCLE, 0.0, &ev);
-    if (conv_ && nlev_ > 0 && lv_[0]->blkp)
-        for (int l = 0; l < nlev_; ++l) {
-            const Level& L = *lv_[size_t(l)];
-            const int ns = L.P->nslices;
-            chain(k_slice_active, div_up(ns, TB / 32), TB, 0, s, L.n, ns, L.blkp, conv_, L.act.p, stop);
-        }
     vcycle(s, 0, r, z, stop);
     if (prof_here) prof_->end(s, PK_VCYCLE, 0.0, ev);
+}
+
+// the three right-hand sides of a batched solve
+template <class T>
+void Amg<T>::apply3(cudaStream_t s, const V3<T>* r, V3<T>* z, const int* stop)
+{
+    if (conv_ && nlev_ > 0 && lv_[0]->blkp) {
+        SliceLevels S{};
+        S.levels = nlev_;
+        for (int l = 0; l < nlev_; ++l) {
+            const Level& L = *lv_[size_t(l)];
+            S.first[l + 1] = S.first[l] + L.P->nslices;
+            S.n[l] = L.n;
+            S.blk[l] = L.blkp;
+            S.act[l] = L.act.p;
+        }
+        chain(k_slice_active, div_up(S.first[nlev_], TB / 32), TB, 0, s, S, conv_, stop);
+    }
+    vcycle(s, 0, r, z, stop);
 }
 
 template class Amg<double>;

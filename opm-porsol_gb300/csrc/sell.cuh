@@ -8,6 +8,8 @@
 
 #include <cuda_fp16.h>
 
+#include "vec3.cuh"
+
 namespace porsol {
 
 // Column of stored entry k of row r: the column itself (int), or its 16-bit offset from the row
@@ -15,27 +17,29 @@ namespace porsol {
 __device__ __forceinline__ int sell_col(const int* __restrict__ col, int k, int) { return col[k]; }
 __device__ __forceinline__ int sell_col(const short* __restrict__ off, int k, int r) { return r + off[k]; }
 
-// sum_t val[k_t] * xf(col[k_t]) accumulated in Acc; xf maps a column index to the vector value.
+// sum_t val[k_t] * xf(col[k_t]) accumulated in Acc (a scalar or three values, vec3.cuh); xf maps a column
+// index to the vector value.
 template <class Acc, class TV, class XF, class CI = int>
 __device__ __forceinline__ Acc sell_dot(const int* __restrict__ sp, const CI* __restrict__ col,
                                         const TV* __restrict__ val, int r, XF xf)
 {
     const int s = r >> 5, lane = r & 31;
     const int b = sp[s], w = (sp[s + 1] - b) >> 5;
-    Acc acc = Acc(0);
+    using S = scalar_t<Acc>;
+    Acc acc{};
     int k = b + lane;
     int t = 0;
     for (; t + 4 <= w; t += 4, k += 128) {
         const int c0 = sell_col(col, k, r), c1 = sell_col(col, k + 32, r), c2 = sell_col(col, k + 64, r),
                   c3 = sell_col(col, k + 96, r);
-        const Acc v0 = Acc(val[k]), v1 = Acc(val[k + 32]), v2 = Acc(val[k + 64]), v3 = Acc(val[k + 96]);
+        const S v0 = S(val[k]), v1 = S(val[k + 32]), v2 = S(val[k + 64]), v3 = S(val[k + 96]);
         const Acc x0 = Acc(xf(c0)), x1 = Acc(xf(c1)), x2 = Acc(xf(c2)), x3 = Acc(xf(c3));
-        acc += v0 * x0;
-        acc += v1 * x1;
-        acc += v2 * x2;
-        acc += v3 * x3;
+        acc = multiply_add(acc, v0, x0);
+        acc = multiply_add(acc, v1, x1);
+        acc = multiply_add(acc, v2, x2);
+        acc = multiply_add(acc, v3, x3);
     }
-    for (; t < w; ++t, k += 32) acc += Acc(val[k]) * Acc(xf(sell_col(col, k, r)));
+    for (; t < w; ++t, k += 32) acc = multiply_add(acc, S(val[k]), Acc(xf(sell_col(col, k, r))));
     return acc;
 }
 
@@ -50,7 +54,8 @@ __device__ __forceinline__ Acc sell_dot_lanes(const int* __restrict__ sp, const 
                                               const TV* __restrict__ val, const int* __restrict__ rowlen, int r,
                                               int q, bool valid, XF xf)
 {
-    Acc acc = Acc(0);
+    using S = scalar_t<Acc>;
+    Acc acc{};
     if (valid) {
         const int b = sp[r >> 5] + (r & 31);
         const int len = rowlen[r];
@@ -58,18 +63,18 @@ __device__ __forceinline__ Acc sell_dot_lanes(const int* __restrict__ sp, const 
         for (; t + K < len; t += 2 * K) {
             const int k0 = b + 32 * t, k1 = b + 32 * (t + K);
             const int c0 = col[k0], c1 = col[k1];
-            const Acc v0 = Acc(val[k0]), v1 = Acc(val[k1]);
+            const S v0 = S(val[k0]), v1 = S(val[k1]);
             const Acc x0 = Acc(xf(c0)), x1 = Acc(xf(c1));
-            acc += v0 * x0;
-            acc += v1 * x1;
+            acc = multiply_add(acc, v0, x0);
+            acc = multiply_add(acc, v1, x1);
         }
         if (t < len) {
             const int k0 = b + 32 * t;
-            acc += Acc(val[k0]) * Acc(xf(col[k0]));
+            acc = multiply_add(acc, S(val[k0]), Acc(xf(col[k0])));
         }
     }
 #pragma unroll
-    for (int o = K / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    for (int o = K / 2; o > 0; o >>= 1) acc += shfl_xor(acc, o);
     return acc;
 }
 

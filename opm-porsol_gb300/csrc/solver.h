@@ -62,7 +62,6 @@ struct porsol_solver {
     bool amg_ready = false;
     int amg_precision = -1;
     int amg_kcycle = -1;   // the K-cycle levels the hierarchy was set up with
-    porsol::DBuf<double> ir_r;   // batched residual
     // the reference numbering's system for the ILU0 path of a renumbered structure:
     // dof permutation, slot sources, values, right-hand side and solution
     porsol::DBuf<int> dof_perm_d, ref_slot_src_d;
@@ -74,17 +73,17 @@ struct porsol_solver {
     porsol::Profiler prof;
 
     // batched periodic upscaling: the pinned row of each sub-grid (its first DOF, the row the
-    // single-grid regularisation acts on), and whether the AMG hierarchy of the previous solve
-    // is reused
+    // single-grid regularisation acts on)
     std::vector<int> reg_rows;
     porsol::DBuf<int> reg_rows_d;
-    bool reuse_amg = false;
-    // ... and solved with one CG per sub-grid (empty: one CG over the whole system)
+    // ... and solved with one CG per sub-grid (empty: one CG over the whole system), the three directions
+    // together (AMG) or one after the other (ILU0)
     porsol::BatchRanges batch;
+    porsol::BatchedCg3 bcg3;
     porsol::BatchedPcg<double, double> bcg64;
-    porsol::BatchCastPrecond cast_pre;   // mixed: FP32 AMG inside the FP64 batched CG
-    porsol::DBuf<double> btol, bscale, bnorm;
+    porsol::DBuf<double> btol;
     void batched_solve(const porsol_solve_opts& o, porsol_solve_stats& st, int maxit);
+    void batched_solve3(const porsol_solve_opts& o, porsol_solve_stats& st, const double* b3, double* x3);
     // ... or all three directions of every sub-grid in one persistent launch
     int upscale_schedule = PORSOL_UPSCALE_AMG;
     porsol::UpscaleSchedule upscale_fixed;   // cta_threads 0: the autotuner's choice
