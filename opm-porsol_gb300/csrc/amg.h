@@ -69,6 +69,8 @@ class Amg : public Precond<T> {
 public:
     void setup(cudaStream_t s, const SellPattern& P0, const T* A0, const AmgOpts& o);
     void apply(cudaStream_t s, const T* r, T* z, const int* stop) override;
+    typename Precond<T>::Start start() override;
+    void apply_started(cudaStream_t s, const T* r, T* z, const int* stop) override;
     // the same cycle for three right-hand sides at once (hierarchies set up with three_vectors)
     void apply3(cudaStream_t s, const V3<T>* r, V3<T>* z, const int* stop);
     int levels() const { return nlev_; }
@@ -162,6 +164,7 @@ private:
     bool k_level(int l) const { return l >= 1 && l <= o_.kcycle_levels && l < nlev_ - 1; }
     double cycle_bytes(int l, std::vector<double>* per_level, bool started = false) const;
     // 1 / theta of the level's Chebyshev interval [lmax / 30, lmax]
+    void cycle(cudaStream_t s, const T* r, T* z, const int* stop, bool started);
     static double cheb_inv_theta(const Level& L) { return 1.0 / (0.5 * (L.lmax + L.lmax / 30.0)); }
     // The smallest levels as one cluster launch (tail.h): levels tail_ .. nlev_ - 1, -1: none.
     void choose_tail(cudaStream_t s);

@@ -805,7 +805,7 @@ __global__ void k_cheb_start(int n, const int* __restrict__ sp, const CI* __rest
     if (xc) {
         acc = row_dot<K, VT>(sp, col, A, rowlen, i, q, valid, [t, xc, agg, wp](int j) {
             const int aj = agg[j];
-            return aj >= 0 ? VT(t[j] + wp * xc[aj]) : t[j];
+            return VT(t[j] + (aj >= 0 ? VT(wp * xc[aj]) : VT{}));
         });
     } else {
         acc = row_dot<K, VT>(sp, col, A, rowlen, i, q, valid, [t](int j) { return t[j]; });
@@ -813,7 +813,7 @@ __global__ void k_cheb_start(int n, const int* __restrict__ sp, const CI* __rest
     if (!valid || q != 0) return;
     if (xc) {
         const int ai = agg[i];
-        x[i] = ai >= 0 ? VT(t[i] + wp * xc[ai]) : t[i];
+        x[i] = t[i] + (ai >= 0 ? VT(wp * xc[ai]) : VT{});
     }
     const VT ri = SCALED ? VT(dinv[i] * b[i] - acc) : VT(dinv[i] * (b[i] - acc));
     r[i] = ri;
@@ -830,7 +830,7 @@ __global__ void k_prolong_add(int n, const VT* __restrict__ t, const VT* __restr
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n || slice_idle(act, i, n)) return;
     const int ai = agg[i];
-    y[i] = ai >= 0 ? VT(t[i] + wp * xc[ai]) : t[i];
+    y[i] = t[i] + (ai >= 0 ? VT(wp * xc[ai]) : VT{});
 }
 
 // x_out = x_in + d_in; r -= D^-1 A d_in; d_out = c1 d_in + c2 r; final: x_out += d_out
@@ -2088,7 +2088,7 @@ void Amg<T>::choose_tail(cudaStream_t s)
 {
     tail_ = tail_first_ = -1;
     const int last = nlev_ - 2;
-    if (blk0_ || o_.smooth_steps != 1 || o_.cheb_degree != 2 || last < 1 || lv_[nlev_ - 1]->n > TAIL_DENSE ||
+    if (blk0_ || lv_[0]->n > TAIL_SYSTEM || o_.smooth_steps != 1 || o_.cheb_degree != 2 || last < 1 || lv_[nlev_ - 1]->n > TAIL_DENSE ||
         lv_[nlev_ - 1]->n < 1 || !tail_fits<T>(lv_[last]->half, TAIL_SMEM))
         return;
     const long long most = sizeof(T) == 8 ? TAIL_ENTRIES_FP64 : TAIL_ENTRIES_FP16;
@@ -2442,11 +2442,38 @@ void Amg<T>::set_block_state(const int* conv)
 template <class T>
 void Amg<T>::apply(cudaStream_t s, const T* r, T* z, const int* stop)
 {
+    cycle(s, r, z, stop, false);
+}
+
+// the first Chebyshev start on the finest level (none when that is the dense one)
+template <class T>
+typename Precond<T>::Start Amg<T>::start()
+{
+    typename Precond<T>::Start st;
+    if (nlev_ > 1) {
+        Level& L = *lv_[0];
+        st.dinv = L.dinv.p;
+        st.r0 = L.r.p;
+        st.d = L.d0.p;
+        st.inv_theta = T(cheb_inv_theta(L));
+    }
+    return st;
+}
+
+template <class T>
+void Amg<T>::apply_started(cudaStream_t s, const T* r, T* z, const int* stop)
+{
+    cycle(s, r, z, stop, true);
+}
+
+template <class T>
+void Amg<T>::cycle(cudaStream_t s, const T* r, T* z, const int* stop, bool started)
+{
     const bool prof_here = prof_ && prof_->on;
     ChainPause plain(prof_here);   // events between the kernels time each one
     cudaEvent_t ev = nullptr;
     if (prof_here) prof_->begin(s, PK_VCYCLE, 0.0, &ev);
-    vcycle(s, 0, r, z, stop);
+    vcycle(s, 0, r, z, stop, started);
     if (prof_here) prof_->end(s, PK_VCYCLE, 0.0, ev);
 }
 

@@ -1,9 +1,12 @@
 // k_krylov.cu -- SELL-32 SpMV, fused CG updates with deterministic last-block
 // reductions, and level-scheduled ILU(0).
 //
-// Reductions: every block writes one FP64 partial sum; the last block to arrive (arrival
-// counter + threadfence) adds the partials in block order and updates the CG scalars in
-// device memory.  The summation order is fixed, so results are run-to-run reproducible.
+// Reductions: every 256 threads write one FP64 partial sum.  Where the next kernel needs the total, each of
+// its blocks adds the partials (sum_parts); where the preconditioner must know whether to run (the residual
+// norms), the last block to arrive (arrival counter + threadfence) adds them and updates the scalars.
+// The order is fixed and the same either way, so results are run-to-run reproducible.  At 255k unknowns the
+// sums of p.q and z.r with their fences and arrivals took 9.2 and 7.0 us, now 5.9 and 3.3, and the kernels that
+// add the partials 1 to 4 us more than before; a CG iteration 143 us, now 139, in FP64 on 38k unknowns 138, now 128.
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -17,22 +20,28 @@ namespace porsol {
 
 namespace {
 
-constexpr int RB = 256;  // threads per block of the vector kernels
+constexpr int RB = 256;           // threads per block of the plain vector kernels
+constexpr int RED_THREADS = 1024;   // of the reducing kernels at most
 
-// Blocks of the reduction kernels: at most 8 per SM, grid-stride beyond.  The last-block
-// reduction costs one fence + atomic per block, so a grid of one thread per row (12k blocks at
-// 3 M rows) spends more time arriving than summing.  The cap depends only on the device, so
-// the summation order stays fixed.
-int red_blocks(int n)
+// Launch shape of the reducing kernels: at most two blocks per SM (the partials the next kernel adds), of 256
+// threads while those cover n (every SM works on small systems), of up to 1024 beyond, then grid-stride.
+// The shape depends only on n and the device, so the summation order stays fixed.
+struct RedShape {
+    int blocks, threads;
+    int partials() const { return blocks * (threads / RB); }
+};
+RedShape red_shape(int n)
 {
     static int cap = 0;
     if (cap == 0) {
         int dev = 0, sms = 0;
         PORSOL_CUDA(cudaGetDevice(&dev));
         PORSOL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        cap = std::max(1, 8 * sms);
+        cap = std::max(1, 2 * sms);
     }
-    return std::max(1, std::min(div_up(std::max(n, 1), RB), cap));
+    int t = 256;
+    while (t < RED_THREADS && div_up(std::max(n, 1), t) > cap) t *= 2;
+    return {std::min(div_up(std::max(n, 1), t), cap), t};
 }
 
 template <class V>
@@ -43,44 +52,64 @@ __device__ __forceinline__ V warp_sum(V v)
     return v;
 }
 
-// Block reduce + last-block finalisation.  Returns true in thread 0 of the last block,
-// with *total holding the full sum.  The per-thread value type V is the vector type: FP32
-// vectors are summed in FP32 within a warp (32 terms) and in FP64 from there on, so the
-// FP64 unit (a small fraction of GB300's FP32 rate) only sees one value per warp.
-template <class V>
-__device__ bool block_reduce_last(V v0, double* partial, unsigned int* counter, double* total)
+// One partial sum per 256 threads (RB), written to part.  The per-thread value type V is the vector type: FP32
+// vectors are summed in FP32 within a warp (32 terms) and in FP64 from there on, so the FP64 unit (a small
+// fraction of GB300's FP32 rate) only sees one value per warp.
+template <int K = 0, class V>
+__device__ __forceinline__ void block_partials(V v0, double* __restrict__ part)
 {
-    __shared__ double ws[RB / 32];
-    __shared__ bool amlast;
+    __shared__ double ws[RED_THREADS / 32];
     const double v = double(warp_sum<V>(v0));
     if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
     __syncthreads();
     if (threadIdx.x < 32) {
         double t = threadIdx.x < (blockDim.x >> 5) ? ws[threadIdx.x] : 0.0;
-        t = warp_sum<double>(t);
-        if (threadIdx.x == 0) {
-            partial[blockIdx.x] = t;
-            __threadfence();
-            const unsigned int prev = atomicAdd(counter, 1u);
-            amlast = (prev == gridDim.x - 1);
-        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (threadIdx.x < (blockDim.x >> 5) && threadIdx.x % 8 == 0)
+            part[blockIdx.x * (blockDim.x / RB) + threadIdx.x / 8] = t;
+    }
+}
+
+// Total of the preceding kernel's partials (same launch shape), in thread 0: the partials over RB threads, a
+// tree per warp, the warps in order.  Thread 0 goes on to form the scalars the block needs from it and hands
+// them over in shared memory: a warp's FP64 instruction holds the FP64 pipe of the SM for 16 cycles, so a
+// quotient in each of 64 warps would cost more than the whole vector operation (9 us against 4 at 255k unknowns).
+template <int K = 0>   // a kernel's sums: K of each its own (their shared memory then needs no barrier between)
+__device__ __forceinline__ double sum_parts(const volatile double* part)
+{
+    __shared__ double ws[RB / 32];
+    if (threadIdx.x < RB) {
+        const int n = int(gridDim.x * (blockDim.x / RB));
+        double s = 0.0;
+        for (int b = threadIdx.x; b < n; b += RB) s += part[b];
+        s = warp_sum<double>(s);
+        if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
+    }
+    __syncthreads();
+    double t = 0.0;
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int w = 0; w < RB / 32; ++w) t += ws[w];
+    return t;
+}
+
+// Partials, and their total in the last block to arrive.  Returns true in thread 0 of that block.
+template <class V>
+__device__ bool block_reduce_last(V v0, double* partial, unsigned int* counter, double* total)
+{
+    __shared__ bool amlast;
+    block_partials(v0, partial);
+    if (threadIdx.x < 32) {
+        __threadfence();
+        __syncwarp();
+        if (threadIdx.x == 0) amlast = atomicAdd(counter, 1u) == gridDim.x - 1;
     }
     __syncthreads();
     if (!amlast) return false;
-    // last block: sum partials in block order
     __threadfence();
-    double s = 0.0;
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) s += ((volatile double*)partial)[b];
-    // fixed-order tree over threads
-    s = warp_sum<double>(s);
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += ws[w];
-        *total = t;
-        *counter = 0u;
-    }
+    *total = sum_parts(partial);
+    if (threadIdx.x == 0) *counter = 0u;
     return threadIdx.x == 0;
 }
 
@@ -114,14 +143,14 @@ __global__ void k_residual(int n, const int* __restrict__ sp, const int* __restr
 
 // r = b - A x; def0 = ||r||
 template <class TV, class T, class CI>
-__global__ void __launch_bounds__(RB) k_cg_init(int n, const int* __restrict__ sp, const CI* __restrict__ col,
+__global__ void __launch_bounds__(RED_THREADS, 2) k_cg_init(int n, const int* __restrict__ sp, const CI* __restrict__ col,
                                                 const TV* __restrict__ val, const T* __restrict__ x,
                                                 const T* __restrict__ b, T* __restrict__ r, CgDev* st,
                                                 double* partial, unsigned int* counter, CgHostView* hv)
 {
     chain_wait();
     T v = 0;
-    for (int i = blockIdx.x * RB + threadIdx.x; i < n; i += gridDim.x * RB) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const T ri = b[i] - sell_row(sp, col, val, x, i);
         r[i] = ri;
         v += ri * ri;
@@ -141,73 +170,64 @@ __global__ void __launch_bounds__(RB) k_cg_init(int n, const int* __restrict__ s
         hv->converged = st->converged;
         hv->stop = st->stop;
         hv->breakdown = 0;
-        __threadfence_system();
     }
 }
 
-// rho = z . r ; which = 0: first direction p = z, rholast = rho; which = 1: rho for beta
+// partial sums of z . r
 template <class T>
-__global__ void __launch_bounds__(RB) k_dot_zr(int n, const T* __restrict__ z, const T* __restrict__ r, CgDev* st,
-                                               double* partial, unsigned int* counter)
+__global__ void __launch_bounds__(RED_THREADS, 2) k_dot_zr(int n, const T* __restrict__ z, const T* __restrict__ r,
+                                                           const CgDev* st, double* __restrict__ part)
 {
     chain_wait();
     if (st->stop) return;
     T v = 0;
-    for (int i = blockIdx.x * RB + threadIdx.x; i < n; i += gridDim.x * RB) v += z[i] * r[i];
-    double tot;
-    if (block_reduce_last<T>(v, partial, counter, &tot)) {
-        st->rho = tot;
-        st->beta = tot / st->rholast;
-    }
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) v += z[i] * r[i];
+    block_partials(v, part);
 }
 
-template <class T>
-__global__ void k_first_direction(int n, const T* __restrict__ z, T* __restrict__ p, CgDev* st)
-{
-    chain_wait();
-    if (st->stop) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = z[i];
-    if (i == 0) st->rholast = st->rho;   // other threads do not read rholast here
-}
-
-// q = A p ; alpha = p . q
+// q = A p; partial sums of p . q
 template <class TV, class T, class CI>
-__global__ void __launch_bounds__(RB) k_spmv_pq(int n, const int* __restrict__ sp, const CI* __restrict__ col,
+__global__ void __launch_bounds__(RED_THREADS, 2) k_spmv_pq(int n, const int* __restrict__ sp, const CI* __restrict__ col,
                                                 const TV* __restrict__ val, const T* __restrict__ p,
-                                                T* __restrict__ q, CgDev* st, double* partial,
-                                                unsigned int* counter)
+                                                T* __restrict__ q, const CgDev* st, double* __restrict__ part)
 {
     chain_wait();
     if (st->stop) return;
     T v = 0;
-    for (int i = blockIdx.x * RB + threadIdx.x; i < n; i += gridDim.x * RB) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const T qi = sell_row(sp, col, val, p, i);
         q[i] = qi;
         v += p[i] * qi;
     }
-    double tot;
-    if (block_reduce_last<T>(v, partial, counter, &tot)) {
-        st->alpha = tot;
-        st->lambda = st->rholast / tot;
-    }
+    block_partials(v, part);
 }
 
-// lambda = rholast/alpha; x += lambda p; r -= lambda q; def = ||r||; convergence test
+// lambda = rho / (p . q); x += lambda p; r -= lambda q; the preconditioner's start from r; def = ||r|| and the
+// convergence test
 template <class T>
-__global__ void __launch_bounds__(RB) k_cg_update(int n, T* __restrict__ x, T* __restrict__ r,
+__global__ void __launch_bounds__(RED_THREADS, 2) k_cg_update(int n, T* __restrict__ x, T* __restrict__ r,
                                                   const T* __restrict__ p, const T* __restrict__ q, CgDev* st,
-                                                  double* partial, unsigned int* counter, CgHostView* hv)
+                                                  const double* __restrict__ pq,
+                                                  typename Precond<T>::Start start, double* partial,
+                                                  unsigned int* counter, CgHostView* hv)
 {
     chain_wait();
     if (st->stop) return;
-    const double alpha = st->alpha;
-    const T lambda = T(st->lambda);
+    __shared__ T s_lambda;
+    const double alpha = sum_parts(pq);
+    if (threadIdx.x == 0) s_lambda = T(st->rho[st->iter & 1] / alpha);
+    __syncthreads();
+    const T lambda = s_lambda;
     T v = 0;
-    for (int i = blockIdx.x * RB + threadIdx.x; i < n; i += gridDim.x * RB) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         x[i] = x[i] + lambda * p[i];
         const T ri = r[i] - lambda * q[i];
         r[i] = ri;
+        if (start.dinv) {
+            const T s = start.dinv[i] * ri;
+            start.r0[i] = s;
+            start.d[i] = s * start.inv_theta;
+        }
         v += ri * ri;
     }
     double tot;
@@ -223,21 +243,26 @@ __global__ void __launch_bounds__(RB) k_cg_update(int n, T* __restrict__ x, T* _
         hv->converged = st->converged;
         hv->breakdown = st->breakdown;
         hv->stop = st->stop;
-        __threadfence_system();
     }
 }
 
-// beta = rho/rholast; p = z + beta p; rholast = rho for the next iteration (no thread of
-// this kernel reads rholast)
+// rho = z . r; beta = rho / last rho; p = z + beta p (first: p = z)
 template <class T>
-__global__ void k_cg_direction(int n, const T* __restrict__ z, T* __restrict__ p, CgDev* st)
+__global__ void __launch_bounds__(RED_THREADS, 2) k_cg_direction(int n, const T* __restrict__ z, T* __restrict__ p,
+                                                                 CgDev* st, const double* __restrict__ zr,
+                                                                 int first)
 {
     chain_wait();
     if (st->stop) return;
-    const T beta = T(st->beta);
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = z[i] + beta * p[i];
-    if (i == 0) st->rholast = st->rho;
+    __shared__ T s_beta;
+    const double rho = sum_parts(zr);
+    const int it = st->iter;
+    if (threadIdx.x == 0) s_beta = first ? T(0) : T(rho / st->rho[(it + 1) & 1]);
+    __syncthreads();
+    const T beta = s_beta;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        p[i] = first ? z[i] : z[i] + beta * p[i];
+    if (blockIdx.x == 0 && threadIdx.x == 0) st->rho[it & 1] = rho;
 }
 
 template <class TA, class TB>
@@ -272,16 +297,18 @@ __global__ void k_dirichlet_guess(int n, const int* __restrict__ sp, const int* 
 }
 
 template <class T>
-__global__ void __launch_bounds__(RB) k_norm2(int n, const T* __restrict__ x, double* partial, unsigned int* counter,
-                                              double* out)
+__global__ void __launch_bounds__(RED_THREADS, 2) k_norm2(int n, const T* __restrict__ x, double* partial,
+                                                          unsigned int* counter, double* out)
 {
     T v = 0;
-    for (int i = blockIdx.x * RB + threadIdx.x; i < n; i += gridDim.x * RB) v += x[i] * x[i];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) v += x[i] * x[i];
     double tot;
     if (block_reduce_last<T>(v, partial, counter, &tot)) *out = tot;
 }
 
 // ---------------- mixed-precision CG with reliable updates ----------------
+constexpr int RC_STAGE = 128;   // iterations without a replacement after which the recurrence is guarded
+
 __device__ __forceinline__ void rc_publish(const RcDev* st, CgHostView* hv)
 {
     hv->def0 = st->def0;
@@ -290,19 +317,18 @@ __device__ __forceinline__ void rc_publish(const RcDev* st, CgHostView* hv)
     hv->converged = st->converged;
     hv->breakdown = st->breakdown;
     hv->stop = st->stop;
-    __threadfence_system();
 }
 
 // r64 = b - A x (FP64); def0 = sigma = ||r64||
 template <class CI>
-__global__ void __launch_bounds__(RB) k_rc_init(int n, const int* __restrict__ sp, const CI* __restrict__ col,
+__global__ void __launch_bounds__(RED_THREADS, 2) k_rc_init(int n, const int* __restrict__ sp, const CI* __restrict__ col,
                                                 const double* __restrict__ val, const double* __restrict__ x,
                                                 const double* __restrict__ b, double* __restrict__ r64, RcDev* st,
                                                 double* partial, unsigned int* counter, CgHostView* hv)
 {
     chain_wait();
     double v = 0.0;
-    for (int i = blockIdx.x * RB + threadIdx.x; i < n; i += gridDim.x * RB) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const double ri = b[i] - sell_row(sp, col, val, x, i);
         r64[i] = ri;
         v += ri * ri;
@@ -312,8 +338,8 @@ __global__ void __launch_bounds__(RB) k_rc_init(int n, const int* __restrict__ s
         const double d = sqrt(tot);
         st->def0 = st->true_def = st->sigma = d;
         st->isig = d > 0.0 ? 1.0 / d : 0.0;
-        st->factor = 1.0;
-        st->iter = st->nrep = st->replace = st->breakdown = 0;
+        st->factor = 1.0f;
+        st->iter = st->last = st->nrep = st->replaced = st->breakdown = st->guard = st->restart = 0;
         st->converged = (d < 1e-30) ? 1 : 0;
         st->stop = st->converged || !isfinite(d);
         st->breakdown = !isfinite(d);
@@ -321,91 +347,124 @@ __global__ void __launch_bounds__(RB) k_rc_init(int n, const int* __restrict__ s
     }
 }
 
-// r32 = r64 / sigma; p *= factor (after a replacement, or at the start when p is unused)
+// at the start and after a replacement: r = r64 / sigma in FP32, p in the new units, the preconditioner's
+// start from r
 __global__ void k_rc_rescale(int n, const double* __restrict__ r64, float* __restrict__ r, float* __restrict__ p,
-                             const RcDev* st, int init)
+                             const RcDev* st, Precond<float>::Start start, int init)
 {
     chain_wait();
-    if (st->stop || !(init || st->replace)) return;
+    if (st->stop || !(init || st->replaced)) return;
     const double is = st->isig;
-    const float f = float(st->factor);
-    for (int i = blockIdx.x * RB + threadIdx.x; i < n; i += gridDim.x * RB) {
-        r[i] = float(r64[i] * is);
+    const float f = st->factor;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const float ri = float(r64[i] * is);
+        r[i] = ri;
+        if (start.dinv) {
+            const float s = start.dinv[i] * ri;
+            start.r0[i] = s;
+            start.d[i] = s * start.inv_theta;
+        }
         if (!init) p[i] *= f;
     }
 }
 
-// q = A32 p; alpha = rho / (p . q)
+// q = A32 p; partial sums of p . q, guarded (RcDev) of p . r too
 template <class CI>
-__global__ void __launch_bounds__(RB) k_rc_pq(int n, const int* __restrict__ sp, const CI* __restrict__ col,
+__global__ void __launch_bounds__(RED_THREADS, 2) k_rc_pq(int n, const int* __restrict__ sp, const CI* __restrict__ col,
                                               const float* __restrict__ val, const float* __restrict__ p,
-                                              float* __restrict__ q, RcDev* st, double* partial,
-                                              unsigned int* counter, CgHostView* hv)
+                                              const float* __restrict__ r, float* __restrict__ q, const RcDev* st,
+                                              double* __restrict__ pq, double* __restrict__ pr)
 {
     chain_wait();
     if (st->stop) return;
-    float v = 0.0f;
-    for (int i = blockIdx.x * RB + threadIdx.x; i < n; i += gridDim.x * RB) {
+    const int guard = st->guard;
+    float v = 0.0f, w = 0.0f;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float qi = sell_row(sp, col, val, p, i);
         q[i] = qi;
         v += p[i] * qi;
+        if (guard) w += p[i] * r[i];
     }
-    double tot;
-    if (block_reduce_last<float>(v, partial, counter, &tot)) {
-        if (!(tot > 0.0) || !isfinite(tot)) {
-            st->alpha = 0.0;
-            st->breakdown = 1;
-            st->stop = 1;
-            rc_publish(st, hv);
-        } else {
-            st->alpha = st->rho / tot;
-        }
-    }
+    block_partials<0>(v, pq);
+    if (guard) block_partials<1>(w, pr);
 }
 
-// x += sigma alpha p (FP64); r -= alpha q; decide on a replacement
-__global__ void __launch_bounds__(RB) k_rc_update(int n, double* __restrict__ x, float* __restrict__ r,
+// alpha = rho / (p . q) (guarded: (p . r) / (p . q)); x += sigma alpha p (FP64); r -= alpha q; the
+// preconditioner's start from r; partial sums of r . r.  Where the curvature is not positive nothing changes
+// (alpha = 0): the direction starts anew from z, guarded; the solve stops if it had just done so.
+__global__ void __launch_bounds__(RED_THREADS, 2) k_rc_update(int n, double* __restrict__ x, float* __restrict__ r,
                                                   const float* __restrict__ p, const float* __restrict__ q,
-                                                  RcDev* st, double* partial, unsigned int* counter,
-                                                  CgHostView* hv)
+                                                  RcDev* st, const double* __restrict__ pq,
+                                                  const double* __restrict__ pr, Precond<float>::Start start,
+                                                  double* __restrict__ part, CgHostView* hv)
 {
     chain_wait();
     if (st->stop) return;
-    const double sa = st->sigma * st->alpha;
-    const float a = float(st->alpha);
+    __shared__ double s_sa;
+    __shared__ float s_a;
+    const int guard = st->guard;
+    const double curv = sum_parts<0>(pq);
+    const double pr_sum = guard ? sum_parts<1>(pr) : 0.0;
+    if (threadIdx.x == 0) {
+        const bool ok = curv > 0.0 && isfinite(curv);
+        const double alpha = ok ? (guard ? pr_sum : st->rho[st->iter & 1]) / curv : 0.0;
+        s_sa = st->sigma * alpha;
+        s_a = float(alpha);
+        if (blockIdx.x == 0) {
+            st->pq = curv;
+            st->restart = !ok;
+            if (!ok && (st->fresh || !isfinite(curv))) {
+                st->breakdown = 1;
+                st->stop = 1;
+                rc_publish(st, hv);
+            }
+        }
+    }
+    __syncthreads();
+    const double sa = s_sa;
+    const float a = s_a;
     float v = 0.0f;
-    for (int i = blockIdx.x * RB + threadIdx.x; i < n; i += gridDim.x * RB) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         x[i] += sa * double(p[i]);
         const float ri = r[i] - a * q[i];
         r[i] = ri;
+        if (start.dinv) {
+            const float s = start.dinv[i] * ri;
+            start.r0[i] = s;
+            start.d[i] = s * start.inv_theta;
+        }
         v += ri * ri;
     }
-    double tot;
-    if (block_reduce_last<float>(v, partial, counter, &tot)) {
-        const double defs = sqrt(tot);
-        st->defs = defs;
-        st->iter += 1;
-        const double est = defs * st->sigma;
-        st->replace = (defs < st->delta || est < st->tol * st->def0 || est < 1e-30 || !isfinite(defs) ||
-                       st->iter >= st->maxit)
-                          ? 1
-                          : 0;
-        hv->iter = st->iter;
-        __threadfence_system();
-    }
+    block_partials(v, part);
 }
 
-// Replacement: r64 = b - A x in FP64; convergence is decided on this true residual only
+// Replacement, when the iterated residual has dropped by delta since the last one or its estimate reaches
+// the tolerance: r64 = b - A x in FP64, convergence decided on this true residual only; otherwise the kernel
+// ends at once.
 template <class CI>
-__global__ void __launch_bounds__(RB) k_rc_true(int n, const int* __restrict__ sp, const CI* __restrict__ col,
+__global__ void __launch_bounds__(RED_THREADS) k_rc_true(int n, const int* __restrict__ sp, const CI* __restrict__ col,
                                                 const double* __restrict__ val, const double* __restrict__ x,
                                                 const double* __restrict__ b, double* __restrict__ r64, RcDev* st,
-                                                double* partial, unsigned int* counter, CgHostView* hv)
+                                                const double* __restrict__ rr, double* partial,
+                                                unsigned int* counter, CgHostView* hv)
 {
     chain_wait();
-    if (st->stop || !st->replace) return;
+    if (st->stop) return;
+    __shared__ int s_replace;
+    const double ss = sum_parts(rr);
+    if (threadIdx.x == 0) {
+        const double defs = sqrt(ss), est = defs * st->sigma;
+        s_replace = defs < st->delta || est < st->tol * st->def0 || est < 1e-30 || !isfinite(defs) ||
+                    st->iter + 1 >= st->maxit;
+        if (!s_replace && blockIdx.x == 0) {
+            st->replaced = 0;   // k_rc_zr counts the iteration
+            if (st->restart || st->iter + 1 - st->last >= RC_STAGE) st->guard = 1;
+        }
+    }
+    __syncthreads();
+    if (!s_replace) return;
     double v = 0.0;
-    for (int i = blockIdx.x * RB + threadIdx.x; i < n; i += gridDim.x * RB) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const double ri = b[i] - sell_row(sp, col, val, x, i);
         r64[i] = ri;
         v += ri * ri;
@@ -413,20 +472,24 @@ __global__ void __launch_bounds__(RB) k_rc_true(int n, const int* __restrict__ s
     double tot;
     if (block_reduce_last<double>(v, partial, counter, &tot)) {
         const double d = sqrt(tot);
+        const int it = st->iter + 1;
         st->true_def = d;
         st->nrep += 1;
+        st->iter = st->last = it;
+        st->replaced = 1;
         if (!isfinite(d)) {
             st->breakdown = 1;
             st->stop = 1;
         } else if (d < st->tol * st->def0 || d < 1e-30) {
             st->converged = 1;
             st->stop = 1;
-        } else if (st->iter >= st->maxit) {
+        } else if (it >= st->maxit) {
             st->stop = 1;
         } else {
             // continue on the rescaled system: r and p in units of the new sigma
-            st->factor = st->sigma / d;
-            st->rho *= st->factor * st->factor;
+            const double f = st->sigma / d;
+            st->factor = float(f);
+            st->rho[(it + 1) & 1] *= f * f;
             st->sigma = d;
             st->isig = 1.0 / d;
         }
@@ -434,30 +497,45 @@ __global__ void __launch_bounds__(RB) k_rc_true(int n, const int* __restrict__ s
     }
 }
 
-// rho_new = z . r; beta = rho_new / rho
-__global__ void __launch_bounds__(RB) k_rc_zr(int n, const float* __restrict__ z, const float* __restrict__ r,
-                                              RcDev* st, double* partial, unsigned int* counter, int init)
+// partial sums of z . r (guarded: z . q); counts the iteration where no replacement did
+__global__ void __launch_bounds__(RED_THREADS, 2) k_rc_zr(int n, const float* __restrict__ z, const float* __restrict__ r,
+                                              const float* __restrict__ q, RcDev* st, double* __restrict__ part,
+                                              int init)
 {
     chain_wait();
     if (st->stop) return;
+    const float* __restrict__ w = st->guard ? q : r;
     float v = 0.0f;
-    for (int i = blockIdx.x * RB + threadIdx.x; i < n; i += gridDim.x * RB) v += z[i] * r[i];
-    double tot;
-    if (block_reduce_last<float>(v, partial, counter, &tot)) {
-        st->beta = init ? 0.0 : tot / st->rho;
-        st->rho = tot;
-        st->replace = 0;
-    }
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) v += z[i] * w[i];
+    block_partials(v, part);
+    if (blockIdx.x == 0 && threadIdx.x == 0 && !init && !st->replaced) st->iter += 1;
 }
 
-// p = z + beta p (beta = 0 at the start)
-__global__ void k_rc_direction(int n, const float* __restrict__ z, float* __restrict__ p, const RcDev* st, int init)
+// rho = z . r; beta = rho / last rho (guarded: -(z . q) / (p . q), q in the units before a replacement);
+// p = z + beta p (at the start and anew: p = z)
+__global__ void __launch_bounds__(RED_THREADS, 2) k_rc_direction(int n, const float* __restrict__ z, float* __restrict__ p,
+                                                                 RcDev* st, const double* __restrict__ zr, int init)
 {
     chain_wait();
     if (st->stop) return;
-    const float beta = float(st->beta);
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = init ? z[i] : z[i] + beta * p[i];
+    __shared__ float s_beta;
+    const bool fresh = init || st->restart;
+    const double sum = sum_parts(zr);
+    if (threadIdx.x == 0) {
+        const int it = st->iter;
+        const bool guard = !init && st->guard;
+        if (fresh) s_beta = 0.0f;
+        else if (guard) s_beta = float(-sum / (st->pq * double(st->replaced ? st->factor : 1.0f)));
+        else s_beta = float(sum / st->rho[(it + 1) & 1]);
+        if (blockIdx.x == 0) {
+            st->rho[it & 1] = sum;
+            st->fresh = fresh;
+        }
+    }
+    __syncthreads();
+    const float beta = s_beta;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        p[i] = fresh ? z[i] : z[i] + beta * p[i];
 }
 
 // ---------------- ILU(0) ----------------
@@ -762,7 +840,10 @@ void PcgSolver<TV, T>::setup(int n, cudaStream_t s)
     p_.alloc(n);
     q_.alloc(n);
     st_.alloc(1);
-    red_.ensure(div_up(std::max(n, 1), RB), s);
+    const int nr = red_shape(n).partials();
+    red_.ensure(nr, s);
+    pq_.alloc(nr);
+    zr_.alloc(nr);
     if (!hview_) {
         PORSOL_CUDA(cudaHostAlloc((void**)&hview_, sizeof(CgHostView), cudaHostAllocMapped));
         PORSOL_CUDA(cudaHostGetDevicePointer((void**)&dview_, hview_, 0));
@@ -786,7 +867,7 @@ void PcgSolver<TV, T>::iteration(cudaStream_t s, const SellPattern& P, const TV*
                                  Profiler* prof, int prof_kernel)
 {
     const int n = P.n;
-    const int nb = div_up(n, RB), nr = red_blocks(n);
+    const auto [nr, tb] = red_shape(n);
     const int* stop = &st_.p->stop;
     const double spmv_bytes = double(P.nent) * (sizeof(TV) + (P.has_off16() ? 2 : 4)) + 2.0 * n * sizeof(T);
     {
@@ -794,17 +875,18 @@ void PcgSolver<TV, T>::iteration(cudaStream_t s, const SellPattern& P, const TV*
         cudaEvent_t ev = nullptr;
         if (pf) prof->begin(s, prof_kernel, spmv_bytes, &ev);
         if (P.has_off16())
-            chain(k_spmv_pq<TV, T, short>, nr, RB, 0, s, n, P.slice_ptr.p, P.off16.p, val, p_.p, q_.p, st_.p,
-                red_.partial.p, red_.counter.p);
+            chain(k_spmv_pq<TV, T, short>, nr, tb, 0, s, n, P.slice_ptr.p, P.off16.p, val, p_.p, q_.p, st_.p, pq_.p);
         else
-            chain(k_spmv_pq<TV, T, int>, nr, RB, 0, s, n, P.slice_ptr.p, P.col.p, val, p_.p, q_.p, st_.p,
-                red_.partial.p, red_.counter.p);
+            chain(k_spmv_pq<TV, T, int>, nr, tb, 0, s, n, P.slice_ptr.p, P.col.p, val, p_.p, q_.p, st_.p, pq_.p);
         if (pf) prof->end(s, prof_kernel, spmv_bytes, ev);
     }
-    chain(k_cg_update<T>, nr, RB, 0, s, n, x, r_.p, p_.p, q_.p, st_.p, red_.partial.p, red_.counter.p, dview_);
-    M.apply(s, r_.p, z_.p, stop);
-    chain(k_dot_zr<T>, nr, RB, 0, s, n, z_.p, r_.p, st_.p, red_.partial.p, red_.counter.p);
-    chain(k_cg_direction<T>, nb, RB, 0, s, n, z_.p, p_.p, st_.p);
+    const typename Precond<T>::Start start = M.start();
+    chain(k_cg_update<T>, nr, tb, 0, s, n, x, r_.p, p_.p, q_.p, st_.p, pq_.p, start, red_.partial.p, red_.counter.p,
+          dview_);
+    if (start.dinv) M.apply_started(s, r_.p, z_.p, stop);
+    else M.apply(s, r_.p, z_.p, stop);
+    chain(k_dot_zr<T>, nr, tb, 0, s, n, z_.p, r_.p, st_.p, zr_.p);
+    chain(k_cg_direction<T>, nr, tb, 0, s, n, z_.p, p_.p, st_.p, zr_.p, 0);
 }
 
 template <class TV, class T>
@@ -820,22 +902,22 @@ CgResult PcgSolver<TV, T>::solve(cudaStream_t s, const SellPattern& P, const TV*
     }
     setup(n, s);
     M.set_block_state(nullptr);   // one system: every row works
-    const int nb = div_up(n, RB), nr = red_blocks(n);
+    const auto [nr, tb] = red_shape(n);
     CgDev init{};
     init.tol = tol;
     init.maxit = maxit;
     PORSOL_CUDA(cudaMemcpyAsync(st_.p, &init, sizeof(CgDev), cudaMemcpyHostToDevice, s));
     if (P.has_off16())
-        chain(k_cg_init<TV, T, short>, nr, RB, 0, s, n, P.slice_ptr.p, P.off16.p, val, x, b, r_.p, st_.p,
+        chain(k_cg_init<TV, T, short>, nr, tb, 0, s, n, P.slice_ptr.p, P.off16.p, val, x, b, r_.p, st_.p,
             red_.partial.p, red_.counter.p, dview_);
     else
-        chain(k_cg_init<TV, T, int>, nr, RB, 0, s, n, P.slice_ptr.p, P.col.p, val, x, b, r_.p, st_.p, red_.partial.p,
+        chain(k_cg_init<TV, T, int>, nr, tb, 0, s, n, P.slice_ptr.p, P.col.p, val, x, b, r_.p, st_.p, red_.partial.p,
             red_.counter.p, dview_);
     PORSOL_CUDA(cudaGetLastError());
     const int* stop = &st_.p->stop;
     M.apply(s, r_.p, z_.p, stop);
-    chain(k_dot_zr<T>, nr, RB, 0, s, n, z_.p, r_.p, st_.p, red_.partial.p, red_.counter.p);
-    chain(k_first_direction<T>, nb, RB, 0, s, n, z_.p, p_.p, st_.p);
+    chain(k_dot_zr<T>, nr, tb, 0, s, n, z_.p, r_.p, st_.p, zr_.p);
+    chain(k_cg_direction<T>, nr, tb, 0, s, n, z_.p, p_.p, st_.p, zr_.p, 1);
     PORSOL_CUDA(cudaGetLastError());
     // One iteration is captured into a CUDA graph (re-captured when the matrix, vectors or
     // preconditioner change) unless per-kernel profiling is on.
@@ -912,7 +994,9 @@ void ReliableCg::setup(int n, cudaStream_t s)
         n_ = n;
     }
     st_.alloc(1);
-    red_.ensure(div_up(std::max(n, 1), RB), s);
+    const int nr = red_shape(n).partials();
+    red_.ensure(nr, s);
+    for (DBuf<double>* v : {&pq_, &pr_, &rr_, &zr_}) v->alloc(nr);
     if (!hview_) {
         PORSOL_CUDA(cudaHostAlloc((void**)&hview_, sizeof(CgHostView), cudaHostAllocMapped));
         PORSOL_CUDA(cudaHostGetDevicePointer((void**)&dview_, hview_, 0));
@@ -933,7 +1017,8 @@ ReliableCg::~ReliableCg()
 void ReliableCg::iteration(cudaStream_t s, const SellPattern& P, const double* val64, const float* val32,
                            Precond<float>& M, const double* b, double* x, Profiler* prof)
 {
-    const int n = P.n, nb = div_up(n, RB), nr = red_blocks(n);
+    const int n = P.n;
+    const auto [nr, tb] = red_shape(n);
     const int* stop = &st_.p->stop;
     {
         const bool pf = prof && prof->on;
@@ -941,24 +1026,26 @@ void ReliableCg::iteration(cudaStream_t s, const SellPattern& P, const double* v
         cudaEvent_t ev = nullptr;
         if (pf) prof->begin(s, PK_SPMV32, bytes, &ev);
         if (P.has_off16())
-            chain(k_rc_pq<short>, nr, RB, 0, s, n, P.slice_ptr.p, P.off16.p, val32, p_.p, q_.p, st_.p, red_.partial.p,
-                red_.counter.p, dview_);
+            chain(k_rc_pq<short>, nr, tb, 0, s, n, P.slice_ptr.p, P.off16.p, val32, p_.p, r_.p, q_.p, st_.p, pq_.p,
+                pr_.p);
         else
-            chain(k_rc_pq<int>, nr, RB, 0, s, n, P.slice_ptr.p, P.col.p, val32, p_.p, q_.p, st_.p, red_.partial.p,
-                red_.counter.p, dview_);
+            chain(k_rc_pq<int>, nr, tb, 0, s, n, P.slice_ptr.p, P.col.p, val32, p_.p, r_.p, q_.p, st_.p, pq_.p,
+                pr_.p);
         if (pf) prof->end(s, PK_SPMV32, bytes, ev);
     }
-    chain(k_rc_update, nr, RB, 0, s, n, x, r_.p, p_.p, q_.p, st_.p, red_.partial.p, red_.counter.p, dview_);
+    const Precond<float>::Start start = M.start();
+    chain(k_rc_update, nr, tb, 0, s, n, x, r_.p, p_.p, q_.p, st_.p, pq_.p, pr_.p, start, rr_.p, dview_);
     if (P.has_off16())
-        chain(k_rc_true<short>, nr, RB, 0, s, n, P.slice_ptr.p, P.off16.p, val64, x, b, r64_.p, st_.p, red_.partial.p,
-            red_.counter.p, dview_);
+        chain(k_rc_true<short>, nr, tb, 0, s, n, P.slice_ptr.p, P.off16.p, val64, x, b, r64_.p, st_.p, rr_.p,
+              red_.partial.p, red_.counter.p, dview_);
     else
-        chain(k_rc_true<int>, nr, RB, 0, s, n, P.slice_ptr.p, P.col.p, val64, x, b, r64_.p, st_.p, red_.partial.p,
-            red_.counter.p, dview_);
-    chain(k_rc_rescale, nr, RB, 0, s, n, r64_.p, r_.p, p_.p, st_.p, 0);
-    M.apply(s, r_.p, z_.p, stop);
-    chain(k_rc_zr, nr, RB, 0, s, n, z_.p, r_.p, st_.p, red_.partial.p, red_.counter.p, 0);
-    chain(k_rc_direction, nb, RB, 0, s, n, z_.p, p_.p, st_.p, 0);
+        chain(k_rc_true<int>, nr, tb, 0, s, n, P.slice_ptr.p, P.col.p, val64, x, b, r64_.p, st_.p, rr_.p,
+              red_.partial.p, red_.counter.p, dview_);
+    chain(k_rc_rescale, nr, tb, 0, s, n, r64_.p, r_.p, p_.p, st_.p, start, 0);
+    if (start.dinv) M.apply_started(s, r_.p, z_.p, stop);
+    else M.apply(s, r_.p, z_.p, stop);
+    chain(k_rc_zr, nr, tb, 0, s, n, z_.p, r_.p, q_.p, st_.p, zr_.p, 0);
+    chain(k_rc_direction, nr, tb, 0, s, n, z_.p, p_.p, st_.p, zr_.p, 0);
 }
 
 CgResult ReliableCg::solve(cudaStream_t s, const SellPattern& P, const double* val64, const float* val32,
@@ -974,23 +1061,25 @@ CgResult ReliableCg::solve(cudaStream_t s, const SellPattern& P, const double* v
     }
     setup(n, s);
     M.set_block_state(nullptr);   // one system: every row works
-    const int nb = div_up(n, RB), nr = red_blocks(n);
+    const auto [nr, tb] = red_shape(n);
     RcDev init{};
     init.tol = tol;
     init.maxit = maxit;
     init.delta = delta;
     PORSOL_CUDA(cudaMemcpyAsync(st_.p, &init, sizeof(RcDev), cudaMemcpyHostToDevice, s));
     if (P.has_off16())
-        chain(k_rc_init<short>, nr, RB, 0, s, n, P.slice_ptr.p, P.off16.p, val64, x, b, r64_.p, st_.p, red_.partial.p,
+        chain(k_rc_init<short>, nr, tb, 0, s, n, P.slice_ptr.p, P.off16.p, val64, x, b, r64_.p, st_.p, red_.partial.p,
             red_.counter.p, dview_);
     else
-        chain(k_rc_init<int>, nr, RB, 0, s, n, P.slice_ptr.p, P.col.p, val64, x, b, r64_.p, st_.p, red_.partial.p,
+        chain(k_rc_init<int>, nr, tb, 0, s, n, P.slice_ptr.p, P.col.p, val64, x, b, r64_.p, st_.p, red_.partial.p,
             red_.counter.p, dview_);
-    chain(k_rc_rescale, nr, RB, 0, s, n, r64_.p, r_.p, p_.p, st_.p, 1);
+    const Precond<float>::Start start = M.start();
+    chain(k_rc_rescale, nr, tb, 0, s, n, r64_.p, r_.p, p_.p, st_.p, start, 1);
     const int* stop = &st_.p->stop;
-    M.apply(s, r_.p, z_.p, stop);
-    chain(k_rc_zr, nr, RB, 0, s, n, z_.p, r_.p, st_.p, red_.partial.p, red_.counter.p, 1);
-    chain(k_rc_direction, nb, RB, 0, s, n, z_.p, p_.p, st_.p, 1);
+    if (start.dinv) M.apply_started(s, r_.p, z_.p, stop);
+    else M.apply(s, r_.p, z_.p, stop);
+    chain(k_rc_zr, nr, tb, 0, s, n, z_.p, r_.p, q_.p, st_.p, zr_.p, 1);
+    chain(k_rc_direction, nr, tb, 0, s, n, z_.p, p_.p, st_.p, zr_.p, 1);
     PORSOL_CUDA(cudaGetLastError());
     // per-kernel event timing records events inside the V-cycle: no graph capture then
     const bool graphs = !(prof && prof->on);
@@ -1293,9 +1382,10 @@ template <class T>
 double norm2(cudaStream_t s, int n, const T* x, RedScratch& red)
 {
     if (n == 0) return 0.0;
-    const int nb = red_blocks(n);
+    const RedShape sh = red_shape(n);
+    const int nb = sh.partials();
     red.ensure(nb + 1, s);
-    PORSOL_LAUNCH(k_norm2<T><<<nb, RB, 0, s>>>(n, x, red.partial.p, red.counter.p, red.partial.p + nb));
+    PORSOL_LAUNCH(k_norm2<T><<<sh.blocks, sh.threads, 0, s>>>(n, x, red.partial.p, red.counter.p, red.partial.p + nb));
     PORSOL_CUDA(cudaGetLastError());
     double out = 0.0;
     PORSOL_CUDA(cudaMemcpyAsync(&out, red.partial.p + nb, sizeof(double), cudaMemcpyDeviceToHost, s));

@@ -5,14 +5,16 @@
 
 namespace porsol {
 
-// Device-resident CG scalars.  Written by the last block of each reduction kernel; read by
-// the next kernel in stream order, so no host round trip is needed per iteration.
+// Device-resident CG scalars, written by one thread of a kernel and read by the next ones in stream order,
+// so no host round trip is needed per iteration.  rho alternates between two slots (iter & 1): the blocks of
+// the kernel that writes the new one still read the last.
 struct CgDev {
-    double rho, rholast, alpha, def0, def, tol, lambda, beta;
+    double rho[2], def0, def, tol;
     int iter, maxit, converged, stop, breakdown, pad;
 };
 
-// Mirror of CgDev in mapped pinned host memory, written at the end of every iteration.
+// Mirror of the stopping state in mapped pinned host memory; the host reads it after an event behind the
+// kernel that wrote it.
 struct CgHostView {
     volatile double def0, def;
     volatile int iter, converged, stop, breakdown;
@@ -32,6 +34,15 @@ struct Precond {
     // z = M^{-1} r; kernels must do nothing when *stop != 0.  apply() must not synchronise
     // or allocate: it is captured into a CUDA graph.
     virtual void apply(cudaStream_t s, const T* r, T* z, const int* stop) = 0;
+    // A preconditioner whose first kernel only forms r0 = dinv r and d = inv_theta r0 names them here; the
+    // CG's last update of r then writes them and calls apply_started() (one launch and one pass less).
+    struct Start {
+        const T* dinv = nullptr;
+        T *r0 = nullptr, *d = nullptr;
+        T inv_theta = T(0);
+    };
+    virtual Start start() { return {}; }
+    virtual void apply_started(cudaStream_t s, const T* r, T* z, const int* stop) { apply(s, r, z, stop); }
     // Batched solves: the per-block convergence flags (device, 0: block still iterating), so a
     // block-diagonal preconditioner may skip the rows of converged blocks; null for one system.
     virtual void set_block_state(const int*) {}
@@ -73,7 +84,8 @@ private:
     int n_ = 0;
     DBuf<T> r_, z_, p_, q_;
     DBuf<CgDev> st_;
-    RedScratch red_;
+    RedScratch red_;       // residual norms
+    DBuf<double> pq_, zr_;   // partial sums of p.q and z.r
     CgHostView* hview_ = nullptr;
     CgHostView* dview_ = nullptr;
     std::vector<cudaEvent_t> ev_;
@@ -95,9 +107,19 @@ private:
 // direction is kept across replacements (rescaled), so no Krylov information and no extra
 // preconditioner application is lost.  Stops when the true residual satisfies
 // ||b - A x|| < tol ||b - A x0|| (or < 1e-30).
+//
+// The recurrence's alpha and beta hold while r stays orthogonal to the last direction and z to the last
+// residual.  Rounding and replacements take that away in some large, strongly heterogeneous systems: the
+// residual then hardly drops (1M cells with log-normal layers: 3 of 48 realisations took 150 iterations to
+// thousands or broke down, the others 40 to 80).  A stage between replacements that lasts RC_STAGE iterations
+// (10 to 15 are usual), or a curvature that is not positive, switches to the guarded form, alpha = p.r / p.q
+// and beta = -z.q / p.q, which minimise along the direction at hand whatever came before: a solve of 5874
+// iterations then takes 180.
 struct RcDev {
-    double rho, alpha, beta, sigma, isig, factor, def0, defs, tol, delta, true_def;
-    int iter, maxit, stop, converged, breakdown, replace, nrep, pad;
+    double rho[2], pq, sigma, isig, def0, tol, delta, true_def;
+    float factor;
+    int iter, last, maxit, stop, converged, breakdown, replaced, nrep;
+    int guard, restart, fresh;   // fresh: p = z; restart: make it so
 };
 
 class ReliableCg {
@@ -112,9 +134,10 @@ public:
 private:
     int n_ = 0, nrep_ = 0;
     DBuf<float> r_, z_, p_, q_;
-    DBuf<double> r64_;
+    DBuf<double> r64_;       // the true residual at a replacement
     DBuf<RcDev> st_;
-    RedScratch red_;
+    RedScratch red_;         // FP64 residual norms
+    DBuf<double> pq_, pr_, rr_, zr_;   // partial sums of p.q, p.r, r.r and z.r (guarded: z.q)
     CgHostView* hview_ = nullptr;
     CgHostView* dview_ = nullptr;
     std::vector<cudaEvent_t> ev_;
