@@ -40,9 +40,6 @@ namespace cg = cooperative_groups;
 
 // The group of threads that solves one sub-grid: a warp, a CTA, or a cluster of CTAs.
 constexpr int G_WARP = 0, G_CTA = 1, G_CLUSTER = 2;
-// One reduction buffer: the per-warp partials (up to 32 warps x 6 values), then the CTA's totals
-// (6 values, read by the other CTAs of a cluster).  Two buffers alternate.
-constexpr int SB_STRIDE = UP_MAX_WARPS * 6 + 6;
 
 struct UpArgs {
     int nitems, ncl, ntile, maxit, n;   // items [0, ncl): clusters; then ntile CTA items; then warp items
@@ -73,17 +70,31 @@ struct Rows {
     __device__ __forceinline__ int row(int k) const { return k < n1 ? r0 + k : r2 + (k - n1); }
 };
 
-// Sums over the group.  The warp butterfly leaves the bitwise-same total in every lane (each step
-// adds two equal pairs in swapped order); a CTA then adds the per-warp totals in warp order in FP64,
-// every thread reading them from shared memory; in a cluster every CTA forms its total that way, and
-// after the cluster barrier each thread adds the CTAs' totals in CTA order, reading them from the
-// other CTAs' shared memory (one remote load per CTA and value, not one per warp); so all threads
-// of the group hold the same sums.  Two buffers alternate from one reduction to the
-// next (rb): a thread that has left one reduction's barrier may write the next one while others
-// still read this one.  FP32 partials (the CG's dot products) are summed in FP32 within a warp and in
-// FP64 across warps.
+// Shared memory of a CTA: the per-warp partials of a reduction, the CTA's totals (read by the other CTAs of a
+// cluster; two sets alternate, since a CTA may form its next totals while another still reads these), the
+// values handed to all threads.
+struct UpShared {
+    double part[UP_MAX_WARPS * 6];
+    double total[2][6];
+    double dval[6];
+    float fval[6];
+    int mask[2];
+};
+
+template <int G>
+__device__ __forceinline__ bool leader()
+{
+    return G == G_WARP || threadIdx.x < 32;
+}
+
+// Sums over the group, in its leader warp(s) (the first warp of every CTA).  FP32 partials (the CG's dot
+// products) are summed in FP32 within a warp and in FP64 across warps (a butterfly: every lane gets the
+// total) and CTAs (in CTA order), so every leader of the group holds the same sums.  One warp adds them: a
+// warp's FP64 instruction holds the SM's FP64 pipe for 16 cycles, and each of 32 warps adding all partials
+// and forming all scalars of the CG cost an iteration 10 to 20 us.  The batch of 192 sub-grids of 5 to 17 cells
+// a side went from 86 to 58.5 ms (10 us per iteration on 600 unknowns, 66 on 15,606 by two CTAs).
 template <int G, int NV, class T>
-__device__ __forceinline__ void group_sum(const T (&v)[NV], double (&out)[NV], double* sb, int& rb)
+__device__ __forceinline__ void group_sum(const T (&v)[NV], double (&out)[NV], UpShared* sh, int& rb)
 {
     T w[NV];
 #pragma unroll
@@ -92,50 +103,81 @@ __device__ __forceinline__ void group_sum(const T (&v)[NV], double (&out)[NV], d
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) w[i] += __shfl_xor_sync(FULL, w[i], o);
     }
-    if constexpr (G == G_CTA) {
-        double* buf = sb + rb * SB_STRIDE;
-        rb ^= 1;
-        const int wi = threadIdx.x >> 5, nw = blockDim.x >> 5;
-        if ((threadIdx.x & 31) == 0)
-#pragma unroll
-            for (int i = 0; i < NV; ++i) buf[wi * NV + i] = double(w[i]);
-        __syncthreads();
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            double s = 0.0;
-            for (int j = 0; j < nw; ++j) s += buf[j * NV + i];
-            out[i] = s;
-        }
-    } else if constexpr (G == G_CLUSTER) {
-        cg::cluster_group cl = cg::this_cluster();
-        double* buf = sb + rb * SB_STRIDE;
-        double* ctot = buf + UP_MAX_WARPS * 6;
-        rb ^= 1;
-        const int wi = threadIdx.x >> 5, nw = blockDim.x >> 5;
-        if ((threadIdx.x & 31) == 0)
-#pragma unroll
-            for (int i = 0; i < NV; ++i) buf[wi * NV + i] = double(w[i]);
-        __syncthreads();
-        if (threadIdx.x == 0)
-#pragma unroll
-            for (int i = 0; i < NV; ++i) {
-                double s = 0.0;
-                for (int j = 0; j < nw; ++j) s += buf[j * NV + i];
-                ctot[i] = s;
-            }
-        cl.sync();
-        const int nc = int(cl.num_blocks());
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            double s = 0.0;
-            for (int c = 0; c < nc; ++c) s += cl.map_shared_rank(ctot, c)[i];
-            out[i] = s;
-        }
-    } else {
+    if constexpr (G == G_WARP) {
 #pragma unroll
         for (int i = 0; i < NV; ++i) out[i] = double(w[i]);
         __syncwarp();
+    } else {
+        T* buf = reinterpret_cast<T*>(sh->part);
+        const int wi = threadIdx.x >> 5, nw = blockDim.x >> 5, lane = threadIdx.x & 31;
+        if (lane == 0)
+#pragma unroll
+            for (int i = 0; i < NV; ++i) buf[i * UP_MAX_WARPS + wi] = w[i];
+        __syncthreads();
+        if (wi == 0) {
+#pragma unroll
+            for (int i = 0; i < NV; ++i) {
+                out[i] = lane < nw ? double(buf[i * UP_MAX_WARPS + lane]) : 0.0;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) out[i] += __shfl_xor_sync(FULL, out[i], o);
+            }
+        }
+        if constexpr (G == G_CLUSTER) {
+            cg::cluster_group cl = cg::this_cluster();
+            double* tot = sh->total[rb];
+            rb ^= 1;
+            if (threadIdx.x == 0)
+#pragma unroll
+                for (int i = 0; i < NV; ++i) tot[i] = out[i];
+            cl.sync();
+            if (wi == 0) {
+                const int nc = int(cl.num_blocks());
+#pragma unroll
+                for (int i = 0; i < NV; ++i) {
+                    double t = 0.0;
+                    for (int c = 0; c < nc; ++c) t += cl.map_shared_rank(tot, c)[i];
+                    out[i] = t;
+                }
+            }
+        }
     }
+}
+
+// What the leader's lanes 0 .. 2 hold for the three directions, to all threads of the group: put() by the
+// leader, then publish() by all, then get().
+template <int G, class T>
+__device__ __forceinline__ void get3(T v, const T* slot, T (&out)[3])
+{
+#pragma unroll
+    for (int d = 0; d < 3; ++d) out[d] = G == G_WARP ? __shfl_sync(FULL, v, d) : slot[d];
+}
+template <int G, class T>
+__device__ __forceinline__ void put3(T v, T* slot)
+{
+    if (G != G_WARP && threadIdx.x < 3) slot[threadIdx.x] = v;
+}
+template <int G>
+__device__ __forceinline__ void publish()
+{
+    if (G != G_WARP) __syncthreads();
+}
+// a bit per direction
+template <int G>
+__device__ __forceinline__ void put_mask(bool b, int& mine, int* slot)
+{
+    mine = int(__ballot_sync(FULL, b) & 7u);
+    if (G != G_WARP && threadIdx.x == 0) *slot = mine;
+}
+__device__ __forceinline__ void bits(int m, bool (&b)[3])
+{
+#pragma unroll
+    for (int d = 0; d < 3; ++d) b[d] = (m >> d) & 1;
+}
+// the value of direction d = lane (lanes above: direction 2), values v[first + d]
+template <int FIRST, int NV>
+__device__ __forceinline__ double lane_pick(const double (&v)[NV], int d)
+{
+    return d == 0 ? v[FIRST] : d == 1 ? v[FIRST + 1] : v[FIRST + 2];
 }
 
 template <int G>
@@ -231,12 +273,16 @@ __device__ __forceinline__ void row_apply3(const int* __restrict__ sp, const int
 // Each pass loads all of a row's values before it stores any, and frozen directions keep their
 // values.  Thread 0 keeps the per-direction iteration count and reduction in global memory.
 template <int G, int L>
-__device__ void solve_one(const UpArgs& a, int g, int tid, int nthr, double* sb)
+__device__ void solve_one(const UpArgs& a, int g, int tid, int nthr, UpShared* sh)
 {
     constexpr bool all[3] = {true, true, true};
     const int* rg = a.ranges + 4 * g;
     const Rows R{rg[0], rg[1] - rg[0], rg[2], (rg[1] - rg[0]) + (rg[3] - rg[2])};
     const int n = a.n;
+    const int dir = min(int(threadIdx.x & 31), 2);   // the direction whose scalars this lane of the leader keeps
+    double* const dv0 = G == G_WARP ? nullptr : sh->dval;
+    float *const fv0 = G == G_WARP ? nullptr : sh->fval, *const fv1 = G == G_WARP ? nullptr : sh->fval + 3;
+    int* const mk = G == G_WARP ? nullptr : sh->mask;
     int rb = 0;
     bool bad = false;
     double v[3] = {0.0, 0.0, 0.0}, sum[3];
@@ -253,22 +299,30 @@ __device__ void solve_one(const UpArgs& a, int g, int tid, int nthr, double* sb)
         for (int d = 0; d < 3; ++d) v[d] += b[d] * b[d];
     }
     if (bad) atomicOr(a.status, ST_NONFINITE);
-    group_sum<G, 3>(v, sum, sb, rb);
-    double sig[3], def0[3], rho[3];
-    bool act[3];
-    bool brk = false;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        def0[d] = sig[d] = sqrt(sum[d]);
-        const bool fin = isfinite(def0[d]);
-        brk |= !fin;
-        act[d] = fin && !(def0[d] < 1e-30);
-        if (tid == 0) {
-            a.iters[3 * g + d] = fin ? (act[d] ? -1 : 0) : -1;
-            a.red[3 * g + d] = act[d] ? 1.0 : 0.0;
+    group_sum<G, 3>(v, sum, sh, rb);
+    // the leader's: sigma, ||b||, r.D^-1 r of direction dir
+    double sigma = 0.0, def0 = 0.0, rho = 0.0;
+    bool on = false, brk = false;
+    int m = 0;   // directions still iterating
+    if (leader<G>()) {
+        def0 = sigma = sqrt(lane_pick<0>(sum, dir));
+        const bool fin = isfinite(def0);
+        brk = !fin;
+        on = fin && !(def0 < 1e-30);
+        if (tid < 3) {
+            a.iters[3 * g + tid] = fin ? (on ? -1 : 0) : -1;
+            a.red[3 * g + tid] = on ? 1.0 : 0.0;
         }
+        put3<G>(sigma, dv0);
+        put_mask<G>(on, m, mk);
     }
+    publish<G>();
     {
+        double sig[3];
+        get3<G>(sigma, dv0, sig);
+        if (G != G_WARP) m = mk[0];
+        bool act[3];
+        bits(m, act);
         float u[3] = {0.f, 0.f, 0.f};
         for (int k = tid; k < R.n; k += nthr) {
             const int r = R.row(k);
@@ -285,10 +339,12 @@ __device__ void solve_one(const UpArgs& a, int g, int tid, int nthr, double* sb)
             st3<L>(a.r32, r, n, all, rr);
             st3<L>(a.p32, r, n, all, pp);
         }
-        group_sum<G, 3>(u, rho, sb, rb);
+        group_sum<G, 3>(u, sum, sh, rb);
+        if (leader<G>()) rho = lane_pick<0>(sum, dir);
+        publish<G>();   // the leader has read the partials
     }
     int it = 0;
-    while ((act[0] || act[1] || act[2]) && it < a.maxit) {
+    while (m && it < a.maxit) {
         ++it;
         // pass A: q = A32 p, p.q
         {
@@ -302,20 +358,34 @@ __device__ void solve_one(const UpArgs& a, int g, int tid, int nthr, double* sb)
 #pragma unroll
                 for (int d = 0; d < 3; ++d) w[d] += p[d] * q[d];
             }
-            group_sum<G, 3>(w, sum, sb, rb);
+            group_sum<G, 3>(w, sum, sh, rb);
         }
-        double al[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            if (act[d] && !(sum[d] > 0.0 && isfinite(sum[d]))) {   // non-positive curvature: stop
-                act[d] = false;
+        double alpha = 0.0;
+        if (leader<G>()) {
+            const double c = lane_pick<0>(sum, dir);
+            if (on && !(c > 0.0 && isfinite(c))) {   // non-positive curvature: stop
+                on = false;
                 brk = true;
             }
-            al[d] = act[d] ? rho[d] / sum[d] : 0.0;
+            alpha = on ? rho / c : 0.0;
+            put3<G>(sigma * alpha, dv0);
+            put3<G>(float(alpha), fv0);
+            put_mask<G>(on, m, mk);
         }
+        publish<G>();
         // pass B: x += sigma alpha p, r -= alpha q; r.D^-1 r, r.r
-        double u[3], rr2[3];
+        double u = 0.0;       // r.D^-1 r (leader)
+        bool again = false;   // this direction replaces its residual (leader)
+        int mrep = 0;
+        float beta = 0.f;
         {
+            double sa[3];
+            float al[3];
+            get3<G>(sigma * alpha, dv0, sa);
+            get3<G>(float(alpha), fv0, al);
+            if (G != G_WARP) m = mk[0];
+            bool act[3];
+            bits(m, act);
             float part[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             for (int k = tid; k < R.n; k += nthr) {
                 const int r = R.row(k);
@@ -329,8 +399,8 @@ __device__ void solve_one(const UpArgs& a, int g, int tid, int nthr, double* sb)
 #pragma unroll
                 for (int d = 0; d < 3; ++d)
                     if (act[d]) {
-                        const float rn = rr[d] - float(al[d]) * q[d];
-                        x[d] += (sig[d] * al[d]) * double(p[d]);
+                        const float rn = rr[d] - al[d] * q[d];
+                        x[d] += sa[d] * double(p[d]);
                         rr[d] = rn;
                         part[d] += rn * (dv * rn);
                         part[3 + d] += rn * rn;
@@ -339,24 +409,32 @@ __device__ void solve_one(const UpArgs& a, int g, int tid, int nthr, double* sb)
                 st3<L>(a.r32, r, n, act, rr);
             }
             double tot[6];
-            group_sum<G, 6>(part, tot, sb, rb);
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                u[d] = tot[d];
-                rr2[d] = tot[3 + d];
+            group_sum<G, 6>(part, tot, sh, rb);
+            if (leader<G>()) {
+                // reliable update: which directions replace their residual
+                u = lane_pick<0>(tot, dir);
+                const double ratio = u / rho;
+                const double defs = sqrt(lane_pick<3>(tot, dir)), est = defs * sigma;
+                again = on && (defs < a.delta || est < a.tol * def0 || est < 1e-30 || !isfinite(defs) || it >= a.maxit);
+                put_mask<G>(again, mrep, mk + 1);
+                if (mrep == 0) {
+                    if (on && !isfinite(u)) {
+                        on = false;
+                        brk = true;
+                    }
+                    beta = on ? float(ratio) : 0.f;
+                    rho = u;
+                    put3<G>(beta, fv0);
+                    put_mask<G>(on, m, mk);
+                }
             }
         }
-        // reliable update: which directions replace their residual
-        bool rep[3], any = false;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const double defs = sqrt(rr2[d]), est = defs * sig[d];
-            rep[d] = act[d] && (defs < a.delta || est < a.tol * def0[d] || est < 1e-30 || !isfinite(defs) ||
-                                it >= a.maxit);
-            any |= rep[d];
-        }
-        if (any) {
+        publish<G>();
+        if (G != G_WARP) mrep = mk[1];
+        if (mrep) {
             // pass R: the true residual b - A x (FP64) of the replacing directions
+            bool rep[3];
+            bits(mrep, rep);
             double t2[3] = {0.0, 0.0, 0.0};
             for (int k = tid; k < R.n; k += nthr) {
                 const int r = R.row(k);
@@ -372,34 +450,44 @@ __device__ void solve_one(const UpArgs& a, int g, int tid, int nthr, double* sb)
                     }
                 st3<L>(a.r64, r, n, rep, t);
             }
-            group_sum<G, 3>(t2, sum, sb, rb);
-            bool resc[3], anyr = false;
-            double fac[3];
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                resc[d] = false;
-                fac[d] = 1.0;
-                if (!rep[d]) continue;
-                const double dd = sqrt(sum[d]);
-                if (tid == 0) a.red[3 * g + d] = dd / def0[d];
-                if (!isfinite(dd)) {
-                    act[d] = false;
-                    brk = true;
-                } else if (dd < a.tol * def0[d] || dd < 1e-30) {
-                    act[d] = false;
-                    if (tid == 0) a.iters[3 * g + d] = it;
-                } else if (it >= a.maxit) {
-                    act[d] = false;
-                } else {
-                    fac[d] = sig[d] / dd;
-                    rho[d] *= fac[d] * fac[d];
-                    sig[d] = dd;
-                    resc[d] = true;
-                    anyr = true;
+            group_sum<G, 3>(t2, sum, sh, rb);
+            float fac = 1.f;
+            bool scaled = false;
+            int mres = 0;
+            if (leader<G>()) {
+                const double dd = sqrt(lane_pick<0>(sum, dir));
+                if (again) {
+                    if (tid < 3) a.red[3 * g + tid] = dd / def0;
+                    if (!isfinite(dd)) {
+                        on = false;
+                        brk = true;
+                    } else if (dd < a.tol * def0 || dd < 1e-30) {
+                        on = false;
+                        if (tid < 3) a.iters[3 * g + tid] = it;
+                    } else if (it >= a.maxit) {
+                        on = false;
+                    } else {
+                        const double f = sigma / dd;
+                        fac = float(f);
+                        rho *= f * f;
+                        sigma = dd;
+                        scaled = true;
+                    }
                 }
+                put3<G>(sigma, dv0);
+                put3<G>(fac, fv1);
+                put_mask<G>(scaled, mres, mk + 1);
             }
-            if (anyr) {
+            publish<G>();
+            double sig[3];
+            float fc[3];
+            get3<G>(sigma, dv0, sig);
+            get3<G>(fac, fv1, fc);
+            if (G != G_WARP) mres = mk[1];
+            if (mres) {
                 // pass S: r = r_true / sigma, p in units of the new sigma; r.D^-1 r of the new r
+                bool resc[3];
+                bits(mres, resc);
                 float uu[3] = {0.f, 0.f, 0.f};
                 for (int k = tid; k < R.n; k += nthr) {
                     const int r = R.row(k);
@@ -413,34 +501,34 @@ __device__ void solve_one(const UpArgs& a, int g, int tid, int nthr, double* sb)
                     for (int d = 0; d < 3; ++d)
                         if (resc[d]) {
                             rr[d] = float(t[d] / sig[d]);
-                            p[d] *= float(fac[d]);
+                            p[d] *= fc[d];
                             uu[d] += rr[d] * (dv * rr[d]);
                         }
                     st3<L>(a.r32, r, n, resc, rr);
                     st3<L>(a.p32, r, n, resc, p);
                 }
-                double un[3];
-                group_sum<G, 3>(uu, un, sb, rb);
-#pragma unroll
-                for (int d = 0; d < 3; ++d)
-                    if (resc[d]) u[d] = un[d];
+                group_sum<G, 3>(uu, sum, sh, rb);
+                if (leader<G>() && scaled) u = lane_pick<0>(sum, dir);
             }
-        }
-        double be[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            be[d] = 0.0;
-            if (!act[d]) continue;
-            if (!isfinite(u[d])) {
-                act[d] = false;
-                brk = true;
-                continue;
+            if (leader<G>()) {
+                if (on && !isfinite(u)) {
+                    on = false;
+                    brk = true;
+                }
+                beta = on ? float(u / rho) : 0.f;
+                rho = u;
+                put3<G>(beta, fv0);
+                put_mask<G>(on, m, mk);
             }
-            be[d] = u[d] / rho[d];
-            rho[d] = u[d];
+            publish<G>();
         }
-        if (!(act[0] || act[1] || act[2])) break;
+        if (G != G_WARP) m = mk[0];
+        if (!m) break;
         // pass C: p = D^-1 r + beta p
+        float be[3];
+        get3<G>(beta, fv0, be);
+        bool act[3];
+        bits(m, act);
         for (int k = tid; k < R.n; k += nthr) {
             const int r = R.row(k);
             const float dv = a.dinv[r];
@@ -449,12 +537,12 @@ __device__ void solve_one(const UpArgs& a, int g, int tid, int nthr, double* sb)
             ld3<L>(a.r32, r, n, act, rr);
 #pragma unroll
             for (int d = 0; d < 3; ++d)
-                if (act[d]) p[d] = dv * rr[d] + float(be[d]) * p[d];
+                if (act[d]) p[d] = dv * rr[d] + be[d] * p[d];
             st3<L>(a.p32, r, n, act, p);
         }
         group_sync<G>();
     }
-    if (tid == 0 && brk) atomicOr(a.status, ST_BREAKDOWN);
+    if (brk && tid < 3) atomicOr(a.status, ST_BREAKDOWN);
 }
 
 // The persistent kernel: cluster items while any is left (rank 0 of the cluster takes the next
@@ -467,7 +555,7 @@ __device__ void solve_one(const UpArgs& a, int g, int tid, int nthr, double* sb)
 template <int L, bool CLUSTER>
 __global__ void __launch_bounds__(UP_MAX_THREADS, 1) k_upscale_persistent(const UpArgs a)
 {
-    __shared__ double sb[2 * SB_STRIDE];
+    __shared__ UpShared sh;
     __shared__ int s_item;
     if constexpr (CLUSTER) {
         cg::cluster_group cl = cg::this_cluster();
@@ -479,7 +567,7 @@ __global__ void __launch_bounds__(UP_MAX_THREADS, 1) k_upscale_persistent(const 
             cl.sync();   // every CTA has read rank 0's s_item before it is written again
             if (item >= a.ncl) break;
             solve_one<G_CLUSTER, L>(a, a.order[item], crank * int(blockDim.x) + int(threadIdx.x),
-                                    csize * int(blockDim.x), sb);
+                                    csize * int(blockDim.x), &sh);
         }
     }
     for (;;) {
@@ -488,7 +576,7 @@ __global__ void __launch_bounds__(UP_MAX_THREADS, 1) k_upscale_persistent(const 
         const int item = s_item;
         __syncthreads();   // every thread has read s_item before thread 0 writes it again
         if (item >= a.ntile) break;
-        solve_one<G_CTA, L>(a, a.order[a.ncl + item], threadIdx.x, blockDim.x, sb);
+        solve_one<G_CTA, L>(a, a.order[a.ncl + item], threadIdx.x, blockDim.x, &sh);
     }
     const int lane = threadIdx.x & 31;
     const int first = a.ncl + a.ntile, nwarp = a.nitems - first;
