@@ -189,6 +189,7 @@ void porsol_solver::init_structure(const porsol_grid* grid, const int* flow_type
     amg_ready = false;
     ilu_levels = false;
     S = Structure();
+    ++topology_builds;
     S.build(grid, flow_type, partner_bid);
     PORSOL_REQUIRE(S.max_ncf <= 12, PORSOL_ERR_BAD_ARG, "cells with more than 12 faces are not supported");
     maxnf = S.max_ncf <= 6 ? 6 : 12;
@@ -755,6 +756,46 @@ double porsol_solver::post_process()
     return d;
 }
 
+// Unknowns of each sub-grid: its internal faces and its boundary faces are each numbered contiguously (faces
+// are numbered in cell order, internal before boundary); its first unknown.  A program upscales realisations
+// of one batch again and again, so the ranges stay while the topology and the sub-grids' cells do.
+void porsol_solver::upscale_ranges(int ngrids, const int* cellpos)
+{
+    const HostGrid& hg = S.g;
+    const bool same = up_topology == topology_builds && up_cellpos.size() == size_t(ngrids) + 1 &&
+                      std::equal(up_cellpos.begin(), up_cellpos.end(), cellpos);
+    if (!same) {
+        up_topology = -1;
+        up_dof0.resize(size_t(ngrids));
+        std::vector<int> rg(4 * size_t(ngrids));
+        for (int g = 0; g < ngrids; ++g) {
+            int lo[2] = {S.N, S.N}, hi[2] = {-1, -1};
+            long long cnt[2] = {0, 0};
+            for (int hf = hg.facepos[cellpos[g]]; hf < hg.facepos[cellpos[g + 1]]; ++hf) {
+                const int b = hg.boundary(hf) ? 1 : 0;
+                lo[b] = std::min(lo[b], S.cf[hf]);
+                hi[b] = std::max(hi[b], S.cf[hf]);
+                cnt[b] += b ? 2 : 1;   // internal faces are seen from both cells
+            }
+            up_dof0[size_t(g)] = std::min(lo[0], lo[1]);
+            for (int b = 0; b < 2; ++b) {
+                if (hi[b] < 0) lo[b] = hi[b] = 0;
+                else
+                    PORSOL_REQUIRE(cnt[b] == 2LL * (hi[b] - lo[b] + 1), PORSOL_ERR_BAD_ARG,
+                                   "upscale: face unknowns of a sub-grid are not contiguous");
+                rg[4 * size_t(g) + 2 * b] = lo[b];
+                rg[4 * size_t(g) + 2 * b + 1] = hi[b] < 0 ? 0 : hi[b] + 1;
+            }
+        }
+        batch.build(rg, S.N, stream);
+        up_cellpos.assign(cellpos, cellpos + ngrids + 1);
+        up_topology = topology_builds;
+    }
+    batch.nblk = ngrids;
+    reg_rows = up_dof0;
+    reg_rows_d.upload(reg_rows, stream);
+}
+
 // Batched periodic upscaling: one block-diagonal system over the disjoint union of the
 // sub-grids, solved for the three unit pressure drops with one AMG hierarchy.
 void porsol_solver::upscale(const porsol_grid* grid, int ngrids, const int* cellpos, const int* partner,
@@ -781,65 +822,30 @@ void porsol_solver::upscale(const porsol_grid* grid, int ngrids, const int* cell
     PORSOL_REQUIRE(!S.renumbered(), PORSOL_ERR_STATE, "upscale: unexpected internal face numbering");
     const double zero3[3] = {0.0, 0.0, 0.0};
     compute_inner_products(perm_h, zero3);
-    // per sub-grid: side areas A_i (high sides), extents L_d, first DOF
+    // per sub-grid: side areas A_i (high sides), extents L_d, from its boundary half-faces
     std::vector<double> A(3 * size_t(ngrids), 0.0), L(3 * size_t(ngrids), 0.0);
-    std::vector<int> dof0(ngrids);
     const HostGrid& hg = S.g;   // topology; the geometry is read from the caller's grid
-    for (int g = 0; g < ngrids; ++g) {
+    for (size_t k = 0, g = 0; g < size_t(ngrids); ++g) {
         double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-        int d0 = S.N;
-        for (int c = cellpos[g]; c < cellpos[g + 1]; ++c)
-            for (int hf = hg.facepos[c]; hf < hg.facepos[c + 1]; ++hf) {
-                d0 = std::min(d0, S.cf[hf]);
-                const int sd = side[hf];
-                if (!hg.boundary(hf)) continue;
-                const int ax = (sd - 1) / 2;
-                const double x = grid->hf_centroid[3 * size_t(hf) + ax];
-                if (sd % 2 == 1) lo[ax] = std::min(lo[ax], x);
-                else {
-                    hi[ax] = std::max(hi[ax], x);
-                    A[3 * size_t(g) + ax] += grid->hf_area[hf];
-                }
+        for (const int end = hg.facepos[cellpos[g + 1]]; k < S.boundary_hf.size() && S.boundary_hf[k] < end; ++k) {
+            const int hf = S.boundary_hf[k], sd = side[hf], ax = (sd - 1) / 2;
+            const double x = grid->hf_centroid[3 * size_t(hf) + ax];
+            if (sd % 2 == 1) lo[ax] = std::min(lo[ax], x);
+            else {
+                hi[ax] = std::max(hi[ax], x);
+                A[3 * g + ax] += grid->hf_area[hf];
             }
+        }
         for (int ax = 0; ax < 3; ++ax) {
-            PORSOL_REQUIRE(hi[ax] > lo[ax] && A[3 * size_t(g) + ax] > 0.0, PORSOL_ERR_BAD_ARG,
+            PORSOL_REQUIRE(hi[ax] > lo[ax] && A[3 * g + ax] > 0.0, PORSOL_ERR_BAD_ARG,
                            "upscale: a sub-grid lacks boundary faces on some side");
-            L[3 * size_t(g) + ax] = hi[ax] - lo[ax];
+            L[3 * g + ax] = hi[ax] - lo[ax];
         }
-        dof0[g] = d0;
     }
-    reg_rows = dof0;
-    reg_rows_d.upload(reg_rows, stream);
-    // Unknowns of each sub-grid: its internal faces and its boundary faces are each numbered
-    // contiguously (faces are numbered in cell order, internal before boundary).
-    {
-        std::vector<int> rg(4 * size_t(ngrids));
-        for (int g = 0; g < ngrids; ++g) {
-            int lo[2] = {S.N, S.N}, hi[2] = {-1, -1};
-            long long cnt[2] = {0, 0};
-            for (int c = cellpos[g]; c < cellpos[g + 1]; ++c)
-                for (int hf = hg.facepos[c]; hf < hg.facepos[c + 1]; ++hf) {
-                    const int b = hg.boundary(hf) ? 1 : 0;
-                    lo[b] = std::min(lo[b], S.cf[hf]);
-                    hi[b] = std::max(hi[b], S.cf[hf]);
-                    cnt[b] += b ? 2 : 1;   // internal faces are seen from both cells
-                }
-            for (int b = 0; b < 2; ++b) {
-                if (hi[b] < 0) lo[b] = hi[b] = 0;
-                else
-                    PORSOL_REQUIRE(cnt[b] == 2LL * (hi[b] - lo[b] + 1), PORSOL_ERR_BAD_ARG,
-                                   "upscale: face unknowns of a sub-grid are not contiguous");
-                rg[4 * size_t(g) + 2 * b] = lo[b];
-                rg[4 * size_t(g) + 2 * b + 1] = hi[b] < 0 ? 0 : hi[b] + 1;
-            }
-        }
-        batch.build(rg, S.N, stream);
-    }
-    DBuf<int> cellpos_d, side_d;
-    cellpos_d.upload(cellpos, ngrids + 1, stream);
-    side_d.upload(side, nhf, stream);
-    DBuf<double> q_d;
-    q_d.alloc(3 * size_t(ngrids));
+    upscale_ranges(ngrids, cellpos);
+    up_cellpos_d.upload(cellpos, ngrids + 1, stream);
+    up_side_d.upload(side, nhf, stream);
+    up_q_d.alloc(3 * size_t(ngrids));
     // the solves' inputs on the device: unit mobility, zero sources, the boundary types once, and
     // each direction's pressure jumps written from the side tags (no host arrays per direction)
     std::vector<double> q(3 * size_t(ngrids));
@@ -849,7 +855,7 @@ void porsol_solver::upscale(const porsol_grid* grid, int ngrids, const int* cell
     launch_fill(stream, nc, 1.0, up_ones.p);
     up_zeros.zero(stream);
     in_bctype.upload(bct, stream);
-    auto jumps = [&](int d) { launch_jump_values(stream, nhf, side_d.p, d, up_bcv.p); };
+    auto jumps = [&](int d) { launch_jump_values(stream, nhf, up_side_d.p, d, up_bcv.p); };
     porsol_fluid fl{PORSOL_FLUID_CELLWISE, 1.0, 1.0, 0.0, 0.0};
     porsol_solve_opts o;
     porsol_solve_opts_default(&o);
@@ -863,8 +869,8 @@ void porsol_solver::upscale(const porsol_grid* grid, int ngrids, const int* cell
         batch.nblk = 0;
     };
     auto tensors = [&](int d) {   // column d of the effective tensors from the recovered fluxes
-        launch_side_fluxes(stream, ngrids, cellpos_d.p, facepos.p, side_d.p, outflux.p, q_d.p);
-        q_d.download(q.data(), q.size(), stream);
+        launch_side_fluxes(stream, ngrids, up_cellpos_d.p, facepos.p, up_side_d.p, outflux.p, up_q_d.p);
+        up_q_d.download(q.data(), q.size(), stream);
         PORSOL_CUDA(cudaStreamSynchronize(stream));
         for (int g = 0; g < ngrids; ++g)
             for (int i = 0; i < 3; ++i)

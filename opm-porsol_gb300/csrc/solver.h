@@ -91,6 +91,12 @@ struct porsol_solver {
     porsol::PersistentUpscale pup;
     porsol::DBuf<double> up_b3, up_x3;
     porsol::DBuf<double> up_ones, up_zeros, up_bcv;   // device inputs of the three upscaling solves
+    porsol::DBuf<int> up_cellpos_d, up_side_d;
+    porsol::DBuf<double> up_q_d;
+    // the sub-grids whose unknown ranges `batch` holds: their cells, their first unknowns, the topology
+    std::vector<int> up_cellpos, up_dof0;
+    long long topology_builds = 0, up_topology = -1;
+    void upscale_ranges(int ngrids, const int* cellpos);
     bool assemble_only = false;   // solve() stops after the assembly (and the pinned rows)
 
     // adjoint (permeability sensitivity) of the last solve

@@ -39,3 +39,32 @@ def test_stops_at_the_iteration_limit(pkg, gpulib, workloads):
                                   pkg.default_solve_opts(residual_tolerance=1e-12))
     assert np.isfinite(keff).all() and st.iterations > 9
     s.close()
+
+
+@pytest.mark.parametrize("schedule", ["batched", "persistent"])
+def test_other_groupings_of_one_union(pkg, gpulib, workloads, schedule):
+    """The unknown ranges stay from call to call: another grouping of the same union's cells, another union
+    and the first ones again give what a new solver gives."""
+    calls = []
+    for seed, sides in ((5, [4, 6, 5]), (7, [6, 4])):
+        union, _, K = workloads.periodic_subgrids(seed=seed, sides=sides)
+        calls.append((union, union.cellpos, K))
+        calls.append((union, np.ascontiguousarray(union.cellpos[[0, 1, -1]] if len(sides) > 2 else
+                                                  union.cellpos[[0, -1]]), K))
+    o = pkg.default_solve_opts(residual_tolerance=1e-11, precision=1)
+
+    def run(s, c):
+        if schedule == "persistent":
+            s.set_upscale_schedule(pkg.UPSCALE_PERSISTENT, 512, 0)
+        try:
+            return s.upscale_periodic(c[0], c[1], c[0].partner, c[0].side, c[2].ravel(), o)[0]
+        except pkg.PorsolError as e:
+            assert len(c[1]) < 3 or c[1] is not c[0].cellpos
+            return np.array([e.code])
+
+    s = pkg.PressureSolver()
+    for i in (0, 1, 1, 0, 2, 3, 0, 3):
+        fresh = pkg.PressureSolver()
+        assert np.array_equal(run(s, calls[i]), run(fresh, calls[i]))
+        fresh.close()
+    s.close()
