@@ -35,13 +35,14 @@ namespace {
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int UP_MAX_THREADS = 1024;
 constexpr int UP_MAX_WARPS = UP_MAX_THREADS / 32;
-constexpr int TUNE_ITERS = 8;   // CG iterations per sub-grid of one autotuner trial
+constexpr int TUNE_ITERS = 16;   // CG iterations of the largest sub-grid in one autotuner trial
 namespace cg = cooperative_groups;
 
 // The group of threads that solves one sub-grid: a warp, a CTA, or a cluster of CTAs.
 constexpr int G_WARP = 0, G_CTA = 1, G_CLUSTER = 2;
 
 struct UpArgs {
+    int trial;            // > 0: a trial; unknowns of the largest sub-grid
     int nitems, ncl, ntile, maxit, n;   // items [0, ncl): clusters; then ntile CTA items; then warp items
     double tol, delta;
     const int* order;     // sub-grid ids: tile items [0, ntile), then warp items
@@ -55,7 +56,7 @@ struct UpArgs {
     double* x3;           // solutions (FP64)
     double* r64;          // true residuals at replacements (FP64)
     float* r32;           // CG vectors (FP32, in units of the direction's sigma)
-    float* p32;
+    float4* p4;
     float* q32;
     float* dinv;          // 1 / a_ii
     int* iters;           // 3 per sub-grid: iteration at which the direction met its test, -1: never
@@ -87,60 +88,77 @@ __device__ __forceinline__ bool leader()
     return G == G_WARP || threadIdx.x < 32;
 }
 
-// Sums over the group, in its leader warp(s) (the first warp of every CTA).  FP32 partials (the CG's dot
-// products) are summed in FP32 within a warp and in FP64 across warps (a butterfly: every lane gets the
-// total) and CTAs (in CTA order), so every leader of the group holds the same sums.  One warp adds them: a
-// warp's FP64 instruction holds the SM's FP64 pipe for 16 cycles, and each of 32 warps adding all partials
-// and forming all scalars of the CG cost an iteration 10 to 20 us.  The batch of 192 sub-grids of 5 to 17 cells
-// a side went from 86 to 58.5 ms (10 us per iteration on 600 unknowns, 66 on 15,606 by two CTAs).
-template <int G, int NV, class T>
-__device__ __forceinline__ void group_sum(const T (&v)[NV], double (&out)[NV], UpShared* sh, int& rb)
+// double(v), exact, on the integer pipe for normal values: a conversion takes as long as an FP64 operation
+// (16 cycles of the SM for a warp).
+__device__ __forceinline__ double widen(float v)
 {
+    const unsigned u = __float_as_uint(v), e = u & 0x7f800000u;
+    if (e == 0u || e == 0x7f800000u) return (u << 1) == 0u ? __hiloint2double(int(u), 0) : double(v);
+    return __hiloint2double(int((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), int(u << 29));
+}
+__device__ __forceinline__ double widen(double v) { return v; }
+
+__device__ __forceinline__ bool finite_bits(double v)
+{
+    return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000;
+}
+
+// Sums over the group: lane l of its leader warp(s) (the first warp of every CTA) gets sum l % 8.  FP32
+// partials (the CG's dot products) are summed in FP32 within a warp and in FP64 across warps (eight lanes per
+// chunk of the warps, then the chunks) and CTAs (in CTA order), so every leader of the group holds the same
+// sums.  One warp adds them: a warp's FP64 instruction holds the SM's FP64 pipe for 16 cycles (a warp issues
+// one in 64), and each of 32 warps adding all partials and forming all scalars of the CG cost an iteration 10
+// to 20 us.
+template <int G, int NV, class T>
+__device__ __forceinline__ double group_sum(const T (&v)[NV], UpShared* sh, int& rb)
+{
+    const int lane = threadIdx.x & 31, i = lane & 7;
     T w[NV];
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-        w[i] = v[i];
+    for (int k = 0; k < NV; ++k) {
+        w[k] = v[k];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) w[i] += __shfl_xor_sync(FULL, w[i], o);
+        for (int o = 16; o > 0; o >>= 1) w[k] += __shfl_xor_sync(FULL, w[k], o);
     }
+    double s = 0.0;
     if constexpr (G == G_WARP) {
+        T mine = w[0];
 #pragma unroll
-        for (int i = 0; i < NV; ++i) out[i] = double(w[i]);
+        for (int k = 1; k < NV; ++k)
+            if (i == k) mine = w[k];
+        s = widen(mine);
         __syncwarp();
     } else {
         T* buf = reinterpret_cast<T*>(sh->part);
-        const int wi = threadIdx.x >> 5, nw = blockDim.x >> 5, lane = threadIdx.x & 31;
+        const int wi = threadIdx.x >> 5, nw = blockDim.x >> 5;
         if (lane == 0)
 #pragma unroll
-            for (int i = 0; i < NV; ++i) buf[i * UP_MAX_WARPS + wi] = w[i];
+            for (int k = 0; k < NV; ++k) buf[k * UP_MAX_WARPS + wi] = w[k];
         __syncthreads();
         if (wi == 0) {
-#pragma unroll
-            for (int i = 0; i < NV; ++i) {
-                out[i] = lane < nw ? double(buf[i * UP_MAX_WARPS + lane]) : 0.0;
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) out[i] += __shfl_xor_sync(FULL, out[i], o);
-            }
+            const int c0 = (lane >> 3) * (nw >> 2);   // 8, 16 or 32 warps
+            if (i < NV)
+                for (int c = c0; c < c0 + (nw >> 2); ++c) s += widen(buf[i * UP_MAX_WARPS + c]);
+            __syncwarp();
+            s += __shfl_xor_sync(FULL, s, 8);
+            s += __shfl_xor_sync(FULL, s, 16);
         }
         if constexpr (G == G_CLUSTER) {
             cg::cluster_group cl = cg::this_cluster();
             double* tot = sh->total[rb];
             rb ^= 1;
-            if (threadIdx.x == 0)
-#pragma unroll
-                for (int i = 0; i < NV; ++i) tot[i] = out[i];
+            if (threadIdx.x < NV) tot[threadIdx.x] = s;
             cl.sync();
             if (wi == 0) {
                 const int nc = int(cl.num_blocks());
-#pragma unroll
-                for (int i = 0; i < NV; ++i) {
-                    double t = 0.0;
-                    for (int c = 0; c < nc; ++c) t += cl.map_shared_rank(tot, c)[i];
-                    out[i] = t;
-                }
+                s = 0.0;
+                if (i < NV)
+                    for (int c = 0; c < nc; ++c) s += cl.map_shared_rank(tot, c)[i];
+                __syncwarp();
             }
         }
     }
+    return s;
 }
 
 // What the leader's lanes 0 .. 2 hold for the three directions, to all threads of the group: put() by the
@@ -173,13 +191,6 @@ __device__ __forceinline__ void bits(int m, bool (&b)[3])
 #pragma unroll
     for (int d = 0; d < 3; ++d) b[d] = (m >> d) & 1;
 }
-// the value of direction d = lane (lanes above: direction 2), values v[first + d]
-template <int FIRST, int NV>
-__device__ __forceinline__ double lane_pick(const double (&v)[NV], int d)
-{
-    return d == 0 ? v[FIRST] : d == 1 ? v[FIRST + 1] : v[FIRST + 2];
-}
-
 template <int G>
 __device__ __forceinline__ void group_sync()
 {
@@ -217,15 +228,38 @@ __device__ __forceinline__ void st3(T* v, int i, int n, const bool (&m)[3], cons
         if (m[d]) v[vix<L>(i, d, n)] = x[d];
 }
 
+// The direction p: four values side by side, the last one unused, so that a gather is one 16-byte load (three
+// 4-byte ones at a stride of 12 took twice the passes through the L1).
+__device__ __forceinline__ void ldp(const float4* p, int i, float (&o)[3])
+{
+    const float4 v = p[i];
+    o[0] = v.x;
+    o[1] = v.y;
+    o[2] = v.z;
+}
+__device__ __forceinline__ void stp(float4* p, int i, const float (&x)[3]) { p[i] = make_float4(x[0], x[1], x[2], 0.f); }
+
+// the three values of unknown i of a gathered vector
+template <int L>
+__device__ __forceinline__ void gather3(const float4* y, int i, int, float (&o)[3])
+{
+    ldp(y, i, o);
+}
+template <int L>
+__device__ __forceinline__ void gather3(const double* y, int i, int n, double (&o)[3])
+{
+    constexpr bool all[3] = {true, true, true};
+    ld3<L>(y, i, n, all, o);
+}
+
 // q = (A y)_r for the three directions (values TV, vector TX, sums TA): the row's SELL-32
 // entries read once, two entries' loads in flight before their gathers; products added in entry
 // order (padding adds exact zeros).
-template <int L, class TA, class TV, class TX>
+template <int L, class TA, class TV, class Y>
 __device__ __forceinline__ void row_apply3(const int* __restrict__ sp, const int* __restrict__ col,
-                                           const TV* __restrict__ val, const TX* y, int n, int r,
+                                           const TV* __restrict__ val, const Y* y, int n, int r,
                                            TA (&q)[3])
 {
-    constexpr bool all[3] = {true, true, true};
     const int s = r >> 5;
     const int b = sp[s], w = (sp[s + 1] - b) >> 5;
     TA a0 = TA(0), a1 = TA(0), a2 = TA(0);
@@ -233,9 +267,9 @@ __device__ __forceinline__ void row_apply3(const int* __restrict__ sp, const int
     for (; t + 2 <= w; t += 2, k += 64) {
         const int c0 = col[k], c1 = col[k + 32];
         const TA v0 = TA(val[k]), v1 = TA(val[k + 32]);
-        TX y0[3], y1[3];
-        ld3<L>(y, c0, n, all, y0);
-        ld3<L>(y, c1, n, all, y1);
+        TA y0[3], y1[3];
+        gather3<L>(y, c0, n, y0);
+        gather3<L>(y, c1, n, y1);
         a0 += v0 * TA(y0[0]);
         a1 += v0 * TA(y0[1]);
         a2 += v0 * TA(y0[2]);
@@ -246,8 +280,8 @@ __device__ __forceinline__ void row_apply3(const int* __restrict__ sp, const int
     if (t < w) {
         const int c0 = col[k];
         const TA v0 = TA(val[k]);
-        TX y0[3];
-        ld3<L>(y, c0, n, all, y0);
+        TA y0[3];
+        gather3<L>(y, c0, n, y0);
         a0 += v0 * TA(y0[0]);
         a1 += v0 * TA(y0[1]);
         a2 += v0 * TA(y0[2]);
@@ -255,6 +289,14 @@ __device__ __forceinline__ void row_apply3(const int* __restrict__ sp, const int
     q[0] = a0;
     q[1] = a1;
     q[2] = a2;
+}
+
+// The square of the residual norm, in units of sigma, below which the residual is replaced: dropped by delta,
+// or the tolerance reached.
+__device__ __forceinline__ double replace_below(const UpArgs& a, double sigma, double def0)
+{
+    const double l = fmax(a.delta, fmax(a.tol * def0, 1e-30) / sigma);
+    return l * l;
 }
 
 // The CG of one sub-grid, three directions at once, by a group of nthr threads (tid = rank), with
@@ -271,7 +313,14 @@ __device__ __forceinline__ void row_apply3(const int* __restrict__ sp, const int
 // one sub-grid of the 512-sub-grid batch stall at 3.3e-11 against a 1e-11 tolerance, its rounding
 // times the condition number bounding the residual each replacement can reach.
 // Each pass loads all of a row's values before it stores any, and frozen directions keep their
-// values.  Thread 0 keeps the per-direction iteration count and reduction in global memory.
+// values.  The leader's lanes 0 .. 2 keep the per-direction iteration count and reduction in global memory.
+// What bounds it (an iteration on 15,606 unknowns by a cluster of two CTAs, 60 us, in thousands of cycles): pass A 59,
+// streaming the matrix (the sub-grids at work together exceed the L2; twice as many loads in flight changed
+// nothing), pass B 30, the FP64 pipe, pass C 8, the sums, scalars and barriers 27 (53 before one warp did them).
+// 192 sub-grids of 5 to 17 cells a side: 86 ms with all threads adding all partials and converting p by FP64
+// instructions, 58.5 with one warp's sums, 48 with p as float4 and converted by integers, 44 to 50 with
+// clusters of four.  Measured and dropped: r and q in shared memory (64 ms, less L1 for the gathers), x brought up
+// to date every second iteration or under pass A (62), six entries a row in flight on 512 threads (65).
 template <int G, int L>
 __device__ void solve_one(const UpArgs& a, int g, int tid, int nthr, UpShared* sh)
 {
@@ -279,13 +328,15 @@ __device__ void solve_one(const UpArgs& a, int g, int tid, int nthr, UpShared* s
     const int* rg = a.ranges + 4 * g;
     const Rows R{rg[0], rg[1] - rg[0], rg[2], (rg[1] - rg[0]) + (rg[3] - rg[2])};
     const int n = a.n;
+    // the iterations of a solve grow like the side of its sub-grid: so do a trial's
+    const int maxit = a.trial > 0 ? max(1, int(float(a.maxit) * cbrtf(float(R.n) / float(a.trial)))) : a.maxit;
     const int dir = min(int(threadIdx.x & 31), 2);   // the direction whose scalars this lane of the leader keeps
     double* const dv0 = G == G_WARP ? nullptr : sh->dval;
     float *const fv0 = G == G_WARP ? nullptr : sh->fval, *const fv1 = G == G_WARP ? nullptr : sh->fval + 3;
     int* const mk = G == G_WARP ? nullptr : sh->mask;
     int rb = 0;
     bool bad = false;
-    double v[3] = {0.0, 0.0, 0.0}, sum[3];
+    double v[3] = {0.0, 0.0, 0.0}, sum;
     for (int k = tid; k < R.n; k += nthr) {
         const int r = R.row(k);
         double b[3];
@@ -299,16 +350,17 @@ __device__ void solve_one(const UpArgs& a, int g, int tid, int nthr, UpShared* s
         for (int d = 0; d < 3; ++d) v[d] += b[d] * b[d];
     }
     if (bad) atomicOr(a.status, ST_NONFINITE);
-    group_sum<G, 3>(v, sum, sh, rb);
-    // the leader's: sigma, ||b||, r.D^-1 r of direction dir
-    double sigma = 0.0, def0 = 0.0, rho = 0.0;
+    sum = group_sum<G, 3>(v, sh, rb);
+    // the leader's: sigma, ||b||, r.D^-1 r, r.r that asks for a replacement, of direction dir
+    double sigma = 0.0, def0 = 0.0, rho = 0.0, limit2 = 0.0;
     bool on = false, brk = false;
     int m = 0;   // directions still iterating
     if (leader<G>()) {
-        def0 = sigma = sqrt(lane_pick<0>(sum, dir));
+        def0 = sigma = sqrt(__shfl_sync(FULL, sum, dir));
         const bool fin = isfinite(def0);
         brk = !fin;
         on = fin && !(def0 < 1e-30);
+        limit2 = on ? replace_below(a, sigma, def0) : 0.0;
         if (tid < 3) {
             a.iters[3 * g + tid] = fin ? (on ? -1 : 0) : -1;
             a.red[3 * g + tid] = on ? 1.0 : 0.0;
@@ -337,14 +389,14 @@ __device__ void solve_one(const UpArgs& a, int g, int tid, int nthr, UpShared* s
                 u[d] += rr[d] * pp[d];
             }
             st3<L>(a.r32, r, n, all, rr);
-            st3<L>(a.p32, r, n, all, pp);
+            stp(a.p4, r, pp);
         }
-        group_sum<G, 3>(u, sum, sh, rb);
-        if (leader<G>()) rho = lane_pick<0>(sum, dir);
+        sum = group_sum<G, 3>(u, sh, rb);
+        if (leader<G>()) rho = __shfl_sync(FULL, sum, dir);
         publish<G>();   // the leader has read the partials
     }
     int it = 0;
-    while (m && it < a.maxit) {
+    while (m && it < maxit) {
         ++it;
         // pass A: q = A32 p, p.q
         {
@@ -352,18 +404,18 @@ __device__ void solve_one(const UpArgs& a, int g, int tid, int nthr, UpShared* s
             for (int k = tid; k < R.n; k += nthr) {
                 const int r = R.row(k);
                 float p[3], q[3];
-                ld3<L>(a.p32, r, n, all, p);
-                row_apply3<L, float>(a.sp, a.col, a.val32, a.p32, n, r, q);
+                ldp(a.p4, r, p);
+                row_apply3<L, float>(a.sp, a.col, a.val32, a.p4, n, r, q);
                 st3<L>(a.q32, r, n, all, q);
 #pragma unroll
                 for (int d = 0; d < 3; ++d) w[d] += p[d] * q[d];
             }
-            group_sum<G, 3>(w, sum, sh, rb);
+            sum = group_sum<G, 3>(w, sh, rb);
         }
         double alpha = 0.0;
         if (leader<G>()) {
-            const double c = lane_pick<0>(sum, dir);
-            if (on && !(c > 0.0 && isfinite(c))) {   // non-positive curvature: stop
+            const double c = __shfl_sync(FULL, sum, dir);
+            if (on && !(c > 0.0 && finite_bits(c))) {   // non-positive curvature: stop
                 on = false;
                 brk = true;
             }
@@ -393,14 +445,14 @@ __device__ void solve_one(const UpArgs& a, int g, int tid, int nthr, UpShared* s
                 double x[3];
                 float p[3], rr[3], q[3];
                 ld3<L>(a.x3, r, n, act, x);
-                ld3<L>(a.p32, r, n, act, p);
+                ldp(a.p4, r, p);
                 ld3<L>(a.r32, r, n, act, rr);
                 ld3<L>(a.q32, r, n, act, q);
 #pragma unroll
                 for (int d = 0; d < 3; ++d)
                     if (act[d]) {
                         const float rn = rr[d] - al[d] * q[d];
-                        x[d] += sa[d] * double(p[d]);
+                        x[d] += sa[d] * widen(p[d]);
                         rr[d] = rn;
                         part[d] += rn * (dv * rn);
                         part[3 + d] += rn * rn;
@@ -408,17 +460,15 @@ __device__ void solve_one(const UpArgs& a, int g, int tid, int nthr, UpShared* s
                 st3<L>(a.x3, r, n, act, x);
                 st3<L>(a.r32, r, n, act, rr);
             }
-            double tot[6];
-            group_sum<G, 6>(part, tot, sh, rb);
+            sum = group_sum<G, 6>(part, sh, rb);
             if (leader<G>()) {
                 // reliable update: which directions replace their residual
-                u = lane_pick<0>(tot, dir);
-                const double ratio = u / rho;
-                const double defs = sqrt(lane_pick<3>(tot, dir)), est = defs * sigma;
-                again = on && (defs < a.delta || est < a.tol * def0 || est < 1e-30 || !isfinite(defs) || it >= a.maxit);
+                u = __shfl_sync(FULL, sum, dir);
+                const double ratio = u / rho, rr2 = __shfl_sync(FULL, sum, 3 + dir);
+                again = on && (rr2 < limit2 || !finite_bits(rr2) || it >= maxit);
                 put_mask<G>(again, mrep, mk + 1);
                 if (mrep == 0) {
-                    if (on && !isfinite(u)) {
+                    if (on && !finite_bits(u)) {
                         on = false;
                         brk = true;
                     }
@@ -450,12 +500,12 @@ __device__ void solve_one(const UpArgs& a, int g, int tid, int nthr, UpShared* s
                     }
                 st3<L>(a.r64, r, n, rep, t);
             }
-            group_sum<G, 3>(t2, sum, sh, rb);
+            sum = group_sum<G, 3>(t2, sh, rb);
             float fac = 1.f;
             bool scaled = false;
             int mres = 0;
             if (leader<G>()) {
-                const double dd = sqrt(lane_pick<0>(sum, dir));
+                const double dd = sqrt(__shfl_sync(FULL, sum, dir));
                 if (again) {
                     if (tid < 3) a.red[3 * g + tid] = dd / def0;
                     if (!isfinite(dd)) {
@@ -464,13 +514,14 @@ __device__ void solve_one(const UpArgs& a, int g, int tid, int nthr, UpShared* s
                     } else if (dd < a.tol * def0 || dd < 1e-30) {
                         on = false;
                         if (tid < 3) a.iters[3 * g + tid] = it;
-                    } else if (it >= a.maxit) {
+                    } else if (it >= maxit) {
                         on = false;
                     } else {
                         const double f = sigma / dd;
                         fac = float(f);
                         rho *= f * f;
                         sigma = dd;
+                        limit2 = replace_below(a, sigma, def0);
                         scaled = true;
                     }
                 }
@@ -495,7 +546,7 @@ __device__ void solve_one(const UpArgs& a, int g, int tid, int nthr, UpShared* s
                     double t[3];
                     float p[3], rr[3];
                     ld3<L>(a.r64, r, n, resc, t);
-                    ld3<L>(a.p32, r, n, resc, p);
+                    ldp(a.p4, r, p);
                     ld3<L>(a.r32, r, n, resc, rr);
 #pragma unroll
                     for (int d = 0; d < 3; ++d)
@@ -505,13 +556,16 @@ __device__ void solve_one(const UpArgs& a, int g, int tid, int nthr, UpShared* s
                             uu[d] += rr[d] * (dv * rr[d]);
                         }
                     st3<L>(a.r32, r, n, resc, rr);
-                    st3<L>(a.p32, r, n, resc, p);
+                    stp(a.p4, r, p);
                 }
-                group_sum<G, 3>(uu, sum, sh, rb);
-                if (leader<G>() && scaled) u = lane_pick<0>(sum, dir);
+                sum = group_sum<G, 3>(uu, sh, rb);
+                if (leader<G>()) {
+                    const double un = __shfl_sync(FULL, sum, dir);
+                    if (scaled) u = un;
+                }
             }
             if (leader<G>()) {
-                if (on && !isfinite(u)) {
+                if (on && !finite_bits(u)) {
                     on = false;
                     brk = true;
                 }
@@ -533,12 +587,12 @@ __device__ void solve_one(const UpArgs& a, int g, int tid, int nthr, UpShared* s
             const int r = R.row(k);
             const float dv = a.dinv[r];
             float p[3], rr[3];
-            ld3<L>(a.p32, r, n, act, p);
+            ldp(a.p4, r, p);
             ld3<L>(a.r32, r, n, act, rr);
 #pragma unroll
             for (int d = 0; d < 3; ++d)
                 if (act[d]) p[d] = dv * rr[d] + be[d] * p[d];
-            st3<L>(a.p32, r, n, act, p);
+            stp(a.p4, r, p);
         }
         group_sync<G>();
     }
@@ -682,7 +736,7 @@ void PersistentUpscale::item_classes(const std::vector<int>& rg, const UpscaleSc
 
 void PersistentUpscale::launch(cudaStream_t s, const SellPattern& P, const double* val, const float* val32,
                                const int* ranges_d, const double* b3, double* x3, double tol, double delta, int maxit,
-                               const UpscaleSchedule& sc, bool graph)
+                               const UpscaleSchedule& sc, bool graph, int trial)
 {
     UpArgs a;
     std::memset(&a, 0, sizeof(a));
@@ -690,6 +744,7 @@ void PersistentUpscale::launch(cudaStream_t s, const SellPattern& P, const doubl
     item_classes(rg_h_, sc, a.ncl, a.ntile);
     a.n = n_;
     a.maxit = maxit;
+    a.trial = trial;
     a.tol = tol;
     a.delta = delta;
     a.order = order_.p;
@@ -703,7 +758,7 @@ void PersistentUpscale::launch(cudaStream_t s, const SellPattern& P, const doubl
     a.x3 = x3;
     a.r64 = r64_.p;
     a.r32 = r32_.p;
-    a.p32 = p32_.p;
+    a.p4 = reinterpret_cast<float4*>(p32_.p);
     a.q32 = q32_.p;
     a.dinv = dinv_.p;
     a.iters = iters_.p;
@@ -780,8 +835,10 @@ void PersistentUpscale::launch(cudaStream_t s, const SellPattern& P, const doubl
 // (256-thread CTAs and a 16384-unknown warp limit always measured slower on the 512-sub-grid
 // batch); sub-grids below 0 or 4096 unknowns (sides up to about 11 in the unit-cube batches) left
 // to single warps; and the sub-grids of at least half the largest one's unknowns solved by clusters
-// of 1 (none), 2 or 4 CTAs.  Each candidate runs TUNE_ITERS iterations of every sub-grid once, after
-// one warm-up launch; the fastest is kept for the batch shape.  A cluster shape that cannot be
+// of 1 (none), 2 or 4 CTAs.  Each candidate runs TUNE_ITERS iterations of the largest sub-grid, of the
+// others fewer in proportion to their sides, as whole solves do, after one warm-up launch; the fastest is kept
+// for the batch shape (192 sub-grids of 5 to 17 cells a side: clusters of 4, 44 ms; with eight iterations of
+// each, clusters of 2 won the trial and took 48).  A cluster shape that cannot be
 // resident on this GPU is skipped.
 UpscaleSchedule PersistentUpscale::tune(cudaStream_t s, const SellPattern& P, const double* val, const float* val32,
                                         const std::vector<int>& rg, const int* ranges_d, const double* b3, double* x3)
@@ -820,11 +877,11 @@ UpscaleSchedule PersistentUpscale::tune(cudaStream_t s, const SellPattern& P, co
                         c.tuned = true;
                         try {
                             if (!warmed) {
-                                launch(s, P, val, val32, ranges_d, b3, x3, 0.0, 0.0, TUNE_ITERS, c, false);
+                                launch(s, P, val, val32, ranges_d, b3, x3, 0.0, 0.0, TUNE_ITERS, c, false, int(largest));
                                 warmed = true;
                             }
                             PORSOL_CUDA(cudaEventRecord(e0, s));
-                            launch(s, P, val, val32, ranges_d, b3, x3, 0.0, 0.0, TUNE_ITERS, c, false);
+                            launch(s, P, val, val32, ranges_d, b3, x3, 0.0, 0.0, TUNE_ITERS, c, false, int(largest));
                         } catch (const Error& e) {
                             if (e.code != PORSOL_ERR_BAD_ARG) throw;
                             continue;   // cluster shape not resident here
@@ -871,7 +928,7 @@ UpscaleResult PersistentUpscale::solve(cudaStream_t s, const SellPattern& P, con
     nblk_ = int(rg.size() / 4);
     r64_.alloc(3 * size_t(n_));
     r32_.alloc(3 * size_t(n_));
-    p32_.alloc(3 * size_t(n_));
+    p32_.alloc(4 * size_t(n_));   // float4 per unknown
     q32_.alloc(3 * size_t(n_));
     dinv_.alloc(size_t(n_));
     red_.alloc(3 * size_t(nblk_));
@@ -893,7 +950,7 @@ UpscaleResult PersistentUpscale::solve(cudaStream_t s, const SellPattern& P, con
     sched_ = fixed.cta_threads ? fixed : tune(s, P, val, val32, rg, ranges_d, b3, x3);
     if (fixed.cta_threads) sched_.tuned = false;
     status_.zero(s);
-    launch(s, P, val, val32, ranges_d, b3, x3, tol, delta, maxit, sched_, true);
+    launch(s, P, val, val32, ranges_d, b3, x3, tol, delta, maxit, sched_, true, 0);
     std::vector<int> its(3 * size_t(nblk_));
     std::vector<double> red(3 * size_t(nblk_));
     int st = 0;

@@ -68,7 +68,7 @@ private:
     std::vector<unsigned char> exec_key_;
     void launch(cudaStream_t s, const SellPattern& P, const double* val, const float* val32, const int* ranges_d,
                 const double* b3, double* x3, double tol, double delta, int maxit, const UpscaleSchedule& sc,
-                bool graph);
+                bool graph, int trial);
     UpscaleSchedule tune(cudaStream_t s, const SellPattern& P, const double* val, const float* val32,
                          const std::vector<int>& ranges, const int* ranges_d, const double* b3, double* x3);
     // items solved by clusters and by single CTAs under a schedule (the rest go to warps)
