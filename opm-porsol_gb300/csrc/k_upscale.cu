@@ -35,7 +35,7 @@ namespace {
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int UP_MAX_THREADS = 1024;
 constexpr int UP_MAX_WARPS = UP_MAX_THREADS / 32;
-constexpr int TUNE_ITERS = 16;   // CG iterations of the largest sub-grid in one autotuner trial
+constexpr int TUNE_ITERS = 48;   // CG iterations of the largest sub-grid in one autotuner trial
 namespace cg = cooperative_groups;
 
 // The group of threads that solves one sub-grid: a warp, a CTA, or a cluster of CTAs.
@@ -89,7 +89,7 @@ __device__ __forceinline__ bool leader()
 }
 
 // double(v), exact, on the integer pipe for normal values: a conversion takes as long as an FP64 operation
-// (16 cycles of the SM for a warp).
+// (16 cycles of the SM for a warp): 192 sub-grids 49.3 -> 44.6 ms.
 __device__ __forceinline__ double widen(float v)
 {
     const unsigned u = __float_as_uint(v), e = u & 0x7f800000u;
@@ -837,8 +837,9 @@ void PersistentUpscale::launch(cudaStream_t s, const SellPattern& P, const doubl
 // to single warps; and the sub-grids of at least half the largest one's unknowns solved by clusters
 // of 1 (none), 2 or 4 CTAs.  Each candidate runs TUNE_ITERS iterations of the largest sub-grid, of the
 // others fewer in proportion to their sides, as whole solves do, after one warm-up launch; the fastest is kept
-// for the batch shape (192 sub-grids of 5 to 17 cells a side: clusters of 4, 44 ms; with eight iterations of
-// each, clusters of 2 won the trial and took 48).  A cluster shape that cannot be
+// for the batch shape (192 sub-grids of 5 to 17 cells a side: clusters of 4 and 1024 threads, 44.6 ms; trials of
+// eight iterations of each took clusters of 2, 49.7, and of 16 weighted ones 512 threads, 49.3).  Warp items are
+// not tried further once they took half as long again as the same schedule without them.  A cluster shape that cannot be
 // resident on this GPU is skipped.
 UpscaleSchedule PersistentUpscale::tune(cudaStream_t s, const SellPattern& P, const double* val, const float* val32,
                                         const std::vector<int>& rg, const int* ranges_d, const double* b3, double* x3)
@@ -861,13 +862,14 @@ UpscaleSchedule PersistentUpscale::tune(cudaStream_t s, const SellPattern& P, co
     PORSOL_CUDA(cudaEventCreate(&e0));
     PORSOL_CUDA(cudaEventCreate(&e1));
     UpscaleSchedule best;
-    float best_ms = 1e30f;
-    bool warmed = false;
+    float best_ms = 1e30f, cta_ms = 1e30f;
+    bool warmed = false, warps = true;
     try {
         for (int cluster : {1, 2, 4})
             for (int layout : {0, 1})
                 for (int threads : {512, 1024})
                     for (int wmax : {0, 4096}) {
+                        if (wmax > 0 && !warps) continue;
                         UpscaleSchedule c;
                         c.cta_threads = threads;
                         c.warp_max_unknowns = wmax;
@@ -897,6 +899,8 @@ UpscaleSchedule PersistentUpscale::tune(cudaStream_t s, const SellPattern& P, co
                             best_ms = ms;
                             best = c;
                         }
+                        if (wmax == 0) cta_ms = ms;
+                        else if (ms > 1.5f * cta_ms) warps = false;
                     }
     } catch (...) {
         cudaEventDestroy(e0);
