@@ -377,16 +377,18 @@ __global__ void __launch_bounds__(RED_THREADS, 2) k_rc_pq(int n, const int* __re
 {
     chain_wait();
     if (st->stop) return;
-    const int guard = st->guard;
-    float v = 0.0f, w = 0.0f;
+    float v = 0.0f;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float qi = sell_row(sp, col, val, p, i);
         q[i] = qi;
         v += p[i] * qi;
-        if (guard) w += p[i] * r[i];
     }
     block_partials<0>(v, pq);
-    if (guard) block_partials<1>(w, pr);
+    if (st->guard) {   // a pass of its own: a branch in the loop above costs 1.6 us of 51.4 at 3M rows
+        float w = 0.0f;
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) w += p[i] * r[i];
+        block_partials<1>(w, pr);
+    }
 }
 
 // alpha = rho / (p . q) (guarded: (p . r) / (p . q)); x += sigma alpha p (FP64); r -= alpha q; the
