@@ -435,9 +435,15 @@ long long porsol_launch_count(void);
  * Row i holds the values 1/4, 1/2, 3/4, 1 at columns i, i+1, i+5, i+17 (mod 64); d_j = 1 + j/64,
  * r = 2, x = 0, c1 = 1/2, c2 = 1/4, so r' = 2 - row_i . d, d' = d/2 + r'/4, x' = d + d' exactly.
  * expire != 0 makes every wait for the copies run out (about 40 ms): the step then writes nothing
- * and the call returns PORSOL_ERR_TIMEOUT with the context still usable.  Returns PORSOL_OK after a
- * normal step. */
+ * and the call returns PORSOL_ERR_TIMEOUT with the context still usable; expire = 2 + l does so for the
+ * wait of lane l of each warp alone, with the same result.  Returns PORSOL_OK after a normal step. */
 int porsol_selftest_bulk_wait(int expire, float* r, float* d, float* x);
+/* Factorises the 48-row tridiagonal matrix (-1, 2.5, -1) by ILU(0) (exact here) and applies the fused
+ * triangular sweeps to r_i = 1 + i/8 on the current device; z (48 doubles) receives the result.  shared:
+ * the sweep's form with the vector in shared memory, else the one with it in global memory.  thread >= 0:
+ * the wait of that thread of the sweep's block (0..287, 256 the one that copies) for the first step's record
+ * runs out (about 20 ms): the call returns PORSOL_ERR_TIMEOUT with the context still usable. */
+int porsol_selftest_ilu_wait(int thread, int shared, double* z);
 
 #ifdef __cplusplus
 }

@@ -183,6 +183,7 @@ EXPORTS = [
     ("porsol_stream", _vp, [_vp]),
     ("porsol_launch_count", C.c_longlong, []),
     ("porsol_selftest_bulk_wait", C.c_int, [C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]),
+    ("porsol_selftest_ilu_wait", C.c_int, [C.c_int, C.c_int, C.c_void_p]),
     ("porsol_transport_cfl_noalloc", _i, [_i, _vp, _vp, _vp, _vp, _d, C.POINTER(_d), _vp]),
 ]
 
@@ -206,13 +207,21 @@ def lib():
 
 def selftest_bulk_wait(expire: bool = False):
     """One run of the finest-level smoother step that stages its slices by bulk copy, on the fixed
-    64-row system of porsol_selftest_bulk_wait; expire makes every wait for the copies run out.
-    Returns (status code, r, d, x)."""
+    64-row system of porsol_selftest_bulk_wait; expire makes every wait for the copies run out (an
+    integer 2 + l: that of lane l of each warp alone).  Returns (status code, r, d, x)."""
     r = np.zeros(64, np.float32)
     d = np.zeros(64, np.float32)
     x = np.zeros(64, np.float32)
-    rc = lib().porsol_selftest_bulk_wait(1 if expire else 0, _p(r), _p(d), _p(x))
+    rc = lib().porsol_selftest_bulk_wait(int(expire), _p(r), _p(d), _p(x))
     return rc, r, d, x
+
+
+def selftest_ilu_wait(thread: int = -1, shared: bool = True):
+    """One application of the fused ILU(0) sweeps on the 48-row system of porsol_selftest_ilu_wait; the wait
+    of `thread` (>= 0) runs out.  Returns (status code, z)."""
+    z = np.zeros(48)
+    rc = lib().porsol_selftest_ilu_wait(int(thread), int(shared), _p(z))
+    return rc, z
 
 
 class PorsolError(RuntimeError):

@@ -50,9 +50,9 @@ struct AmgOpts {
                                    // (0: plain V-cycle)
 };
 
-// One finest-level bulk-staged Chebyshev step on a fixed 64-row system (expire: every wait for the
-// bulk copies runs out); returns the kernel's status bits and the 64 values of r, d and x.
-int bulk_step_selftest(bool expire, float* r, float* d, float* x);
+// One finest-level bulk-staged Chebyshev step on a fixed 64-row system (gated: the lanes of each warp, a bit
+// each, whose wait for the bulk copies runs out); returns the kernel's status bits and the 64 values of r, d and x.
+int bulk_step_selftest(unsigned gated, float* r, float* d, float* x);
 
 // Device aggregation result: agg (row -> aggregate or -1), members CSR (aggregate -> rows).
 struct Aggregates {

@@ -17,23 +17,30 @@ __device__ __forceinline__ unsigned long long global_ns()
     return t;
 }
 
-// wait for the barrier's phase of this parity; false when it has not completed within limit_ns
+__device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity)
+{
+    unsigned ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
+// Wait for the barrier's phase of this parity; false when it has not completed within limit_ns.  The last
+// look comes after the limit, so a thread that was not running while the time passed does not give up on a
+// copy that has landed.  Threads wait each for themselves: one may give up where another does not, so the
+// caller lets all threads that work together hear of it (a vote) before any of them leaves.
 __device__ __forceinline__ bool mbar_wait_bounded(unsigned bar, unsigned parity, unsigned long long limit_ns)
 {
-    unsigned long long t0 = 0;
+    if (mbar_try(bar, parity)) return true;   // apart from the loop (8.17 against 8.67 ms for ILU0-CG on 1000 cells)
+    const unsigned long long t0 = global_ns();
     for (long long it = 0; it < BULK_WAIT_TRIES; ++it) {
-        unsigned ok;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (ok) return true;
-        const unsigned long long t = global_ns();
-        if (it == 0) t0 = t;
-        else if (t - t0 > limit_ns) return false;
+        if (mbar_try(bar, parity)) return true;
+        if (global_ns() - t0 > limit_ns) break;
     }
-    return false;
+    return mbar_try(bar, parity);
 }
 
 __device__ __forceinline__ void mbar_init(unsigned bar)

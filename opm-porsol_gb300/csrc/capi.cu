@@ -1121,6 +1121,23 @@ int guarded(porsol_solver* h, F&& f)
 
 }  // namespace
 
+namespace {
+// runs f, which returns device status bits, as a C entry point
+template <class F>
+int selftest(F&& f)
+{
+    try {
+        const int st = f();
+        if (st & porsol::ST_TIMEOUT) return PORSOL_ERR_TIMEOUT;
+        return st ? PORSOL_ERR_BAD_ARG : PORSOL_OK;
+    } catch (const porsol::Error& e) {
+        return e.code;
+    } catch (...) {
+        return PORSOL_ERR_CUDA;
+    }
+}
+}  // namespace
+
 extern "C" {
 
 void porsol_solve_opts_default(porsol_solve_opts* o)
@@ -1517,15 +1534,14 @@ long long porsol_launch_count(void) { return porsol::g_launches.load(); }
 int porsol_selftest_bulk_wait(int expire, float* r, float* d, float* x)
 {
     if (!r || !d || !x) return PORSOL_ERR_BAD_ARG;
-    try {
-        const int st = porsol::bulk_step_selftest(expire != 0, r, d, x);
-        if (st & porsol::ST_TIMEOUT) return PORSOL_ERR_TIMEOUT;
-        return st ? PORSOL_ERR_BAD_ARG : PORSOL_OK;
-    } catch (const porsol::Error& e) {
-        return e.code;
-    } catch (...) {
-        return PORSOL_ERR_CUDA;
-    }
+    const unsigned gated = expire == 0 ? 0u : expire >= 2 && expire < 34 ? 1u << (expire - 2) : ~0u;
+    return selftest([&] { return porsol::bulk_step_selftest(gated, r, d, x); });
+}
+
+int porsol_selftest_ilu_wait(int thread, int shared, double* z)
+{
+    if (!z) return PORSOL_ERR_BAD_ARG;
+    return selftest([&] { return porsol::ilu_sweep_selftest(thread, shared != 0, z); });
 }
 
 }  // extern "C"

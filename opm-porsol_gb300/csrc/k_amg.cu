@@ -882,7 +882,7 @@ __global__ void k_cheb_step(int n, const int* __restrict__ sp, const CI* __restr
 // slice) has the TMA engine copy the slice's columns and FP16 values into the warp's part of
 // shared memory with two cp.async.bulk transfers completing on the warp's own mbarrier, so the
 // warp waits for one transfer instead of a column load per group before its gathers.  The sums are
-// those of k_cheb_step<T, 0, __half, true> in the same order.  Every wait is bounded: on a timeout
+// those of k_cheb_step<T, 0, __half, true> in the same order.  Every wait is bounded: when any lane's runs out
 // the warp sets ST_TIMEOUT, waits once more (bounded) for its copies and returns without writing.
 constexpr int BULK_SLICES = 8;
 
@@ -890,9 +890,9 @@ constexpr int BULK_SLICES = 8;
 // and one gate used only by the self-test), then BULK_SLICES column areas of cap entries
 // (sizeof(CI) B each: 4 for columns, 2 for 16-bit column offsets), then BULK_SLICES value areas
 // (2 B each).  cap and the slice offsets are multiples of 128 entries, so every copy starts and
-// ends on a 16-byte boundary.  extra_tx (0 in solves) makes the gate barrier wait for bytes that
-// no copy delivers: the self-test of the timeout path, whose copies still complete on their own
-// barrier, so the warp sees them land before it leaves.
+// ends on a 16-byte boundary.  gated (0 in solves): the lanes, a bit each, that first wait at the gate
+// barrier for bytes that no copy delivers: the self-test of the timeout path, whose copies still
+// complete on their own barrier, so the warp sees them land before it leaves.
 template <class CI>
 __device__ __forceinline__ int4 x4_columns(const CI* p, int row);
 template <>
@@ -912,7 +912,7 @@ __global__ void __launch_bounds__(BULK_SLICES * 32)
     k_cheb_step_bulk(int n, int nslices, const int* __restrict__ sp4, const CI* __restrict__ col4,
                      const __half* __restrict__ a4, const T* x_in, const T* __restrict__ d_in, T* __restrict__ r,
                      T* __restrict__ d_out, T* x_out, T c1, T c2, int final_step, const int* stop, int cap,
-                     int* status, unsigned extra_tx)
+                     int* status, unsigned gated)
 {
     constexpr unsigned CB = sizeof(CI);
     extern __shared__ __align__(128) unsigned char smem[];
@@ -932,15 +932,17 @@ __global__ void __launch_bounds__(BULK_SLICES * 32)
     __half* sval = reinterpret_cast<__half*>(smem + 128 + size_t(BULK_SLICES) * cap * CB) + size_t(w) * cap;
     if (lane == 0) {
         mbar_init(bar);
-        if (extra_tx) mbar_init(gate);
+        if (gated) mbar_init(gate);
         mbar_init_fence();
         mbar_expect(bar, unsigned(ne) * (CB + 2u));
-        if (extra_tx) mbar_expect(gate, extra_tx);
+        if (gated) mbar_expect(gate, 16);
         bulk_copy(smem_u32(scol), col4 + e0, unsigned(ne) * CB, bar);
         bulk_copy(smem_u32(sval), a4 + e0, unsigned(ne) * 2u, bar);
     }
     __syncwarp();
-    if (!((extra_tx == 0 || mbar_wait_bounded(gate, 0, BULK_WAIT_NS)) && mbar_wait_bounded(bar, 0, BULK_WAIT_NS))) {
+    const bool landed = (!(gated >> lane & 1u) || mbar_wait_bounded(gate, 0, BULK_WAIT_NS)) &&
+                        mbar_wait_bounded(bar, 0, BULK_WAIT_NS);
+    if (!__all_sync(0xffffffffu, landed)) {
         if (lane == 0) atomicOr(status, ST_TIMEOUT);
         mbar_wait_bounded(bar, 0, BULK_WAIT_NS);  // the copies themselves may still be in flight
         return;
@@ -2502,9 +2504,9 @@ template class Amg<float>;
 // Self-test of k_cheb_step_bulk and of its bounded wait: one step (c1 = 1/2, c2 = 1/4, from x = 0,
 // final) on a 64-row system of two slices with one group each; row i holds the FP16 values
 // 1/4, 1/2, 3/4, 1 at columns i, (i+1)%64, (i+5)%64, (i+17)%64 and d_j = 1 + j/64, r = 2 (every
-// product and sum exact in FP32).  expire adds 16 bytes to what each warp's barrier waits for, so
-// every wait runs out.  Returns the kernel's status bits; r, d, x receive the 64 outputs.
-int bulk_step_selftest(bool expire, float* r_host, float* d_host, float* x_host)
+// product and sum exact in FP32).  gated: the lanes of each warp (a bit each) whose wait runs out.
+// Returns the kernel's status bits; r, d, x receive the 64 outputs.
+int bulk_step_selftest(unsigned gated, float* r_host, float* d_host, float* x_host)
 {
     const int n = 64, ns = 2, cap = 128;
     std::vector<int> sp4 = {0, 128, 256}, col4(256);
@@ -2537,7 +2539,7 @@ int bulk_step_selftest(bool expire, float* r_host, float* d_host, float* x_host)
     const size_t shm = 128 + size_t(BULK_SLICES) * cap * 6;
     PORSOL_LAUNCH((k_cheb_step_bulk<float, int><<<1, BULK_SLICES * 32, shm, s>>>(
         n, ns, dsp.p, dcol.p, da.p, nullptr, dd.p, dr.p, ddn.p, dx.p, 0.5f, 0.25f, 1, dstop.p, cap, dstat.p,
-        expire ? 16u : 0u)));
+        gated)));
     PORSOL_CUDA(cudaGetLastError());
     const int st = read_int(s, dstat.p);
     dr.download(r_host, n, s);

@@ -653,7 +653,10 @@ __global__ void k_ilu_pack(int nval, const int* __restrict__ pos, const int* __r
 // vector.  10^3 cube (3300 rows, 84 + 84 levels): one application takes 99 us in one launch, and took 510 us in
 // 168 launches.  Measured and not kept: the records prefetched into registers (130 us), one of the row
 // threads issuing the copies (163 us), each row's operands loaded a step ahead by its own thread (117 us).
-// Every wait is bounded; on a timeout the block sets ST_TIMEOUT, waits (bounded) for its copies and returns.
+// Every wait is bounded.  A thread whose wait ran out skips its row and says so in shared memory; all threads
+// read that behind the step's barrier and leave together one step later, when the load is long done (a voting
+// barrier cost 7 us of the 99): the block sets ST_TIMEOUT and waits (bounded) for its copies.  GATED (the
+// self-test): thread `gate` also waits, in the first step, at a barrier for bytes that no copy delivers.
 constexpr int ILU_ROWS = 256;              // rows of a step at most: a thread each, and one warp that copies
 constexpr int ILU_TB = ILU_ROWS + 32;
 constexpr int ILU_AHEAD = 8;               // products of a row whose operands are loaded before the first sum
@@ -680,21 +683,24 @@ __device__ __forceinline__ double ilu_row(double acc, const double* v, const CI*
 // Step record: a header (rows, W, upper, -), W columns of cp doubles (cp: rows rounded up to 8), for the
 // upper triangle cp inverted pivots, cp row numbers, W columns of cp column numbers.
 // steps: (offset in the records / 16, bytes).
-template <class CI, bool SZ>
+template <class CI, bool SZ, bool GATED = false>
 __global__ void __launch_bounds__(ILU_TB) k_ilu_steps(int s0, int s1, const int2* __restrict__ steps,
                                                       const unsigned char* __restrict__ blob,
                                                       const double* __restrict__ r, double* z, int n, int nst,
-                                                      const int* stop, int* status)
+                                                      const int* stop, int* status, int gate)
 {
     chain_wait();
     if (*stop) return;
-    extern __shared__ __align__(128) unsigned char sm[];
+    extern __shared__ __align__(128) unsigned char sm[];   // the stages' barriers and the gate, the ring, the vector
     unsigned char* ring = sm + 128;
     double* zs = reinterpret_cast<double*>(ring + size_t(nst) * ILU_STAGE);
     const int i = threadIdx.x;
     const bool copier = i == ILU_ROWS;
-    const unsigned bars = smem_u32(sm);
+    const unsigned bars = smem_u32(sm), gate_bar = bars + 8 * ILU_STAGES;
+    volatile int* gave_up = reinterpret_cast<volatile int*>(sm + 8 * (ILU_STAGES + 1));   // by the step's parity
+    int issued = s0, seen = s0;   // steps whose copies were started and have landed (copier)
     auto issue = [&](const int2& t, int stage) {
+        ++issued;
         mbar_expect(bars + 8 * stage, unsigned(t.y));
         bulk_copy(smem_u32(ring + size_t(stage) * ILU_STAGE), blob + 16 * size_t(t.x), unsigned(t.y), bars + 8 * stage);
     };
@@ -702,7 +708,10 @@ __global__ void __launch_bounds__(ILU_TB) k_ilu_steps(int s0, int s1, const int2
     int2 next = none;
     if (copier) {
         for (int k = 0; k < nst; ++k) mbar_init(bars + 8 * k);
+        if (GATED) mbar_init(gate_bar);
         mbar_init_fence();
+        if (GATED) mbar_expect(gate_bar, 16);
+        gave_up[0] = gave_up[1] = 0;
         for (int k = 0; k < nst && s0 + k < s1; ++k) issue(steps[s0 + k], k);
         next = s0 + nst < s1 ? steps[s0 + nst] : none;
     }
@@ -711,23 +720,23 @@ __global__ void __launch_bounds__(ILU_TB) k_ilu_steps(int s0, int s1, const int2
         if (i == 0) zs[n] = 0.0;
     }
     auto value = [&](int j) { return SZ ? zs[j] : (j < n ? z[j] : 0.0); };
-    int stage = 0;
+    auto leave = [&] {
+        if (!copier) return;
+        atomicOr(status, ST_TIMEOUT);
+        for (int t = seen; t < issued; ++t)   // the copies still in flight
+            mbar_wait_bounded(bars + 8 * ((t - s0) % nst), unsigned((t - s0) / nst) & 1u, BULK_WAIT_NS);
+    };
+    int stage = 0, late = 0;
     unsigned parity = 0;
     __syncthreads();   // barriers initialised, vector in place
     for (int s = s0; s < s1; ++s) {
-        if (!mbar_wait_bounded(bars + 8 * stage, parity, BULK_WAIT_NS)) {
-            if (copier) {
-                atomicOr(status, ST_TIMEOUT);
-                for (int k = 0; k < nst && s + k < s1; ++k) {   // the copies still in flight
-                    const int g = stage + k;
-                    mbar_wait_bounded(bars + 8 * (g < nst ? g : g - nst), g < nst ? parity : parity ^ 1u, BULK_WAIT_NS);
-                }
-            }
-            return;
-        }
+        bool landed = mbar_wait_bounded(bars + 8 * stage, parity, BULK_WAIT_NS);
+        if (GATED && i == gate && s == s0) landed = mbar_wait_bounded(gate_bar, 0, BULK_WAIT_NS) && landed;
+        if (landed) seen = s + 1;
+        else gave_up[s & 1] = 1;
         const unsigned char* rec = ring + size_t(stage) * ILU_STAGE;
         const int4 h = *reinterpret_cast<const int4*>(rec);
-        if (i < h.x) {
+        if (landed && i < h.x) {
             const int W = h.y, up = h.z, cp = (h.x + 7) & ~7;
             const double* v = reinterpret_cast<const double*>(rec + 16) + i;
             const CI* rows = reinterpret_cast<const CI*>(rec + 16 + size_t(W + up) * cp * sizeof(double)) + i;
@@ -751,7 +760,9 @@ __global__ void __launch_bounds__(ILU_TB) k_ilu_steps(int s0, int s1, const int2
             else z[row] = acc;
         }
         __syncthreads();
-        if (copier && s + nst < s1) {   // every thread is done with this stage
+        if (late) return leave();
+        late = gave_up[s & 1];
+        if (copier && landed && s + nst < s1) {   // every thread is done with this stage
             issue(next, stage);
             next = s + nst + 1 < s1 ? steps[s + nst + 1] : none;
         }
@@ -760,6 +771,7 @@ __global__ void __launch_bounds__(ILU_TB) k_ilu_steps(int s0, int s1, const int2
             parity ^= 1u;
         }
     }
+    if (late) return leave();
     if (SZ)
         for (int k = i; k < n; k += ILU_TB) z[k] = zs[k];
 }
@@ -1143,7 +1155,7 @@ CgResult ReliableCg::solve(cudaStream_t s, const SellPattern& P, const double* v
 }
 
 // ---------------- ILU(0) host side ----------------
-void Ilu0::build_levels(const SellPattern& P, cudaStream_t s)
+void Ilu0::build_levels(const SellPattern& P, cudaStream_t s, bool shared)
 {
     P_ = &P;
     const int n = P.n;
@@ -1195,7 +1207,7 @@ void Ilu0::build_levels(const SellPattern& P, cudaStream_t s)
     for (const std::vector<int>* ptr : {&h_lptr_, &h_uptr_})
         for (size_t l = 0; l + 1 < ptr->size(); ++l) all = all && (*ptr)[l + 1] - (*ptr)[l] <= FUSE_ROWS;
     const size_t zbytes = (size_t(n) + 1) * sizeof(double);
-    shared_z_ = all && n < 65535 && 128 + zbytes + 2 * size_t(ILU_STAGE) <= ILU_SMEM;
+    shared_z_ = shared && all && n < 65535 && 128 + zbytes + 2 * size_t(ILU_STAGE) <= ILU_SMEM;
     stages_ = shared_z_ ? std::min<int>(ILU_STAGES, int((ILU_SMEM - 128 - zbytes) / ILU_STAGE)) : ILU_STAGES;
     const size_t ib = shared_z_ ? 2 : 4;
     std::vector<int2> steps;
@@ -1319,23 +1331,72 @@ int Ilu0::solve_status(cudaStream_t s) const
     return st;
 }
 
+size_t Ilu0::steps_shm() const
+{
+    return 128 + size_t(stages_) * ILU_STAGE + (shared_z_ ? (size_t(P_->n) + 1) * sizeof(double) : 0);
+}
+
+int ilu_sweep_selftest(int thread, bool shared, double* z_host)
+{
+    const int n = 48;
+    HVec<int> ptr(size_t(n) + 1, 0), col, slot;
+    std::vector<double> a, r(n);
+    for (int i = 0; i < n; ++i) {
+        for (int j = std::max(0, i - 1); j <= std::min(n - 1, i + 1); ++j) {
+            col.push_back(j);
+            a.push_back(j == i ? 2.5 : -1.0);
+        }
+        ptr[size_t(i) + 1] = int(col.size());
+        r[size_t(i)] = 1.0 + i / 8.0;
+    }
+    cudaStream_t s = nullptr;
+    SellPattern P;
+    build_sell(n, ptr, col, P, &slot);
+    P.upload(s);
+    std::vector<double> v(size_t(P.nent), 0.0);
+    for (size_t k = 0; k < a.size(); ++k) v[size_t(slot[k])] = a[k];
+    DBuf<double> val, rd, zd;
+    DBuf<int> stop;
+    val.upload(v, s);
+    rd.upload(r, s);
+    zd.alloc(n);
+    stop.alloc(1);
+    stop.zero(s);
+    Ilu0 ilu;
+    ilu.build_levels(P, s, shared);
+    ilu.factor(s, P, val.p);
+    if (thread < 0) {
+        ilu.apply(s, rd.p, zd.p, stop.p);
+    } else {
+        PORSOL_REQUIRE(thread < ILU_TB && ilu.runs_.size() == 1 && ilu.runs_[0].fused, PORSOL_ERR_BAD_ARG, "ILU0 self-test");
+        auto* f = ilu.shared_z_ ? k_ilu_steps<unsigned short, true, true> : k_ilu_steps<int, false, true>;
+        PORSOL_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ILU_SMEM)));
+        device_copy(s, zd.p, rd.p, n * sizeof(double));
+        chain(f, 1, ILU_TB, ilu.steps_shm(), s, ilu.runs_[0].a, ilu.runs_[0].b, ilu.steps_.p, ilu.blob_.p, rd.p,
+              zd.p, n, ilu.stages_, stop.p, ilu.status_.p, thread);
+    }
+    const int st = ilu.solve_status(s);
+    zd.download(z_host, n, s);
+    PORSOL_CUDA(cudaStreamSynchronize(s));
+    return st;
+}
+
 void Ilu0::apply(cudaStream_t s, const double* r, double* z, const int* stop)
 {
     const SellPattern& P = *P_;
-    const size_t zbytes = size_t(P.n) * sizeof(double);
-    const size_t shm = 128 + size_t(stages_) * ILU_STAGE + (shared_z_ ? zbytes + sizeof(double) : 0);
+    const size_t zbytes = size_t(P.n) * sizeof(double), shm = steps_shm();
     if (!shared_z_) PORSOL_CUDA(cudaMemcpyAsync(z, r, zbytes, cudaMemcpyDeviceToDevice, s));   // the fused steps start from z
     for (const Run& u : runs_) {
         if (u.fused && shared_z_) {
             PORSOL_CUDA(cudaFuncSetAttribute(k_ilu_steps<unsigned short, true>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, int(ILU_SMEM)));
             chain(k_ilu_steps<unsigned short, true>, 1, ILU_TB, shm, s, u.a, u.b, steps_.p, blob_.p, r, z, P.n, stages_,
-                  stop, status_.p);
+                  stop, status_.p, -1);
         } else if (u.fused) {
             PORSOL_CUDA(cudaFuncSetAttribute(k_ilu_steps<int, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              int(ILU_SMEM)));
             chain(k_ilu_steps<int, false>, 1, ILU_TB, shm, s, u.a, u.b, steps_.p, blob_.p, r, z, P.n, stages_, stop,
-                  status_.p);
+                  status_.p, -1);
         } else if (u.b == 0) {
             const int b = h_lptr_[u.a], cnt = h_lptr_[u.a + 1] - b;
             chain(k_ilu_lower_level, div_up(cnt, 128), 128, 0, s, cnt, lrows_.p + b, P.slice_ptr.p, P.col.p, P.diag.p,

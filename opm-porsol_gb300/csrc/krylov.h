@@ -160,7 +160,8 @@ private:
 // wider levels, which would wait for one SM's FP64 pipe, keep a launch of their own.
 class Ilu0 : public Precond<double> {
 public:
-    void build_levels(const SellPattern& P, cudaStream_t s);   // structure only
+    // structure only; shared: the sweep's vector may live in shared memory
+    void build_levels(const SellPattern& P, cudaStream_t s, bool shared = true);
     void factor(cudaStream_t s, const SellPattern& P, const double* val);
     void apply(cudaStream_t s, const double* r, double* z, const int* stop) override;
     // error bits set by apply() (ST_TIMEOUT: a bounded wait for a bulk copy gave up); synchronises the stream
@@ -188,7 +189,13 @@ private:
     DBuf<int> pos_, from_;         // value pos_[e] of the records is the factor's slot from_[e]
     bool shared_z_ = false;        // the sweep's vector lives in shared memory
     int stages_ = 2;
+    size_t steps_shm() const;      // dynamic shared memory of k_ilu_steps
+    friend int ilu_sweep_selftest(int thread, bool shared, double* z);
 };
+
+// The fused sweeps on a fixed 48-row system (thread >= 0: that thread's wait for a step record runs out); returns
+// the kernel's status bits and the 48 values of z.
+int ilu_sweep_selftest(int thread, bool shared, double* z);
 
 // Helpers used by the solver front end.
 void device_copy(cudaStream_t s, void* dst, const void* src, size_t bytes);
