@@ -444,6 +444,13 @@ int porsol_selftest_bulk_wait(int expire, float* r, float* d, float* x);
  * the wait of that thread of the sweep's block (0..287, 256 the one that copies) for the first step's record
  * runs out (about 20 ms): the call returns PORSOL_ERR_TIMEOUT with the context still usable. */
 int porsol_selftest_ilu_wait(int thread, int shared, double* z);
+/* Sets up the AMG hierarchy of a symmetric positive definite CSR matrix (host arrays, sorted columns) in the given
+ * precision (PORSOL_MIXED: FP32) on the current device, with clusters of at most `clusters` blocks (16 or 8; 0: a
+ * launch per step, as on a device that cannot hold the clusters) and three pairing rounds on coarse levels of
+ * fewer than round3_below rows.  levels; per level (24 at most) its rows and a hash of its matrix and aggregates;
+ * inverse: the coarsest level's, row by row (at most 160 x 160). */
+int porsol_selftest_amg_setup(int n, const int* rowptr, const int* col, const double* val, int precision, int clusters,
+                              int round3_below, int* levels, int* rows, unsigned long long* hash, double* inverse);
 
 #ifdef __cplusplus
 }

@@ -184,6 +184,7 @@ EXPORTS = [
     ("porsol_launch_count", C.c_longlong, []),
     ("porsol_selftest_bulk_wait", C.c_int, [C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]),
     ("porsol_selftest_ilu_wait", C.c_int, [C.c_int, C.c_int, C.c_void_p]),
+    ("porsol_selftest_amg_setup", C.c_int, [_i, _vp, _vp, _vp, _i, _i, _i, _vp, _vp, _vp, _vp]),
     ("porsol_transport_cfl_noalloc", _i, [_i, _vp, _vp, _vp, _vp, _d, C.POINTER(_d), _vp]),
 ]
 
@@ -222,6 +223,22 @@ def selftest_ilu_wait(thread: int = -1, shared: bool = True):
     z = np.zeros(48)
     rc = lib().porsol_selftest_ilu_wait(int(thread), int(shared), _p(z))
     return rc, z
+
+
+def selftest_amg_setup(matrix, precision=FP64, clusters=16, round3_below=0):
+    """The AMG hierarchy of a scipy CSR matrix (porsol_selftest_amg_setup): rows per level, a hash per level of
+    its matrix and aggregates, the coarsest level's inverse."""
+    ptr, col = (np.ascontiguousarray(a, np.int32) for a in (matrix.indptr, matrix.indices))
+    val = np.ascontiguousarray(matrix.data, np.float64)
+    levels, rows, hashes = np.zeros(1, np.int32), np.zeros(24, np.int32), np.zeros(24, np.uint64)
+    inverse = np.zeros(160 * 160)
+    rc = lib().porsol_selftest_amg_setup(len(ptr) - 1, _p(ptr), _p(col), _p(val), int(precision), int(clusters),
+                                         int(round3_below), _p(levels), _p(rows), _p(hashes), _p(inverse))
+    if rc:
+        raise PorsolError(rc, "AMG setup self-test")
+    n = int(levels[0])
+    nc = int(rows[n - 1])
+    return rows[:n].tolist(), hashes[:n].tolist(), inverse[:nc * nc].reshape(nc, nc)
 
 
 class PorsolError(RuntimeError):

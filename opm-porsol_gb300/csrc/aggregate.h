@@ -37,10 +37,13 @@ struct AggArgs {
     int* scratch;
 };
 
+// Both return false, with nothing launched, where the device holds no cluster of the size (of at most `limit`
+// blocks) that the level needs; the caller then takes a launch per step.
 template <class T>
-void agg_launch(cudaStream_t s, int lanes, const AggArgs<T>& a);
+bool agg_launch(cudaStream_t s, int lanes, const AggArgs<T>& a, int limit);
 
 // agg1 = agg2 o agg1 (n rows onto nc aggregates) with member lists
-void compose_launch(cudaStream_t s, int n, int nc, int* agg1, const int* agg2, int* cnt, int* ptr, int* idx, int* scratch);
+bool compose_launch(cudaStream_t s, int n, int nc, int* agg1, const int* agg2, int* cnt, int* ptr, int* idx, int* scratch,
+                    int limit);
 
 }  // namespace porsol

@@ -45,6 +45,7 @@ struct AmgOpts {
                                    // choice then depends on timing: off where runs must be
                                    // bitwise reproducible)
     bool three_vectors = false;    // work vectors of three right-hand sides (apply3; one with apply)
+    int setup_cluster = AGG_CTAS;  // blocks of a setup cluster at most: 16 or 8 (0: a launch per step)
     int kcycle_levels = 0;         // K-cycle: the coarse corrections of levels 1 .. kcycle_levels are
                                    // two flexible-CG steps preconditioned by the cycle of that level
                                    // (0: plain V-cycle)
@@ -53,6 +54,11 @@ struct AmgOpts {
 // One finest-level bulk-staged Chebyshev step on a fixed 64-row system (gated: the lanes of each warp, a bit
 // each, whose wait for the bulk copies runs out); returns the kernel's status bits and the 64 values of r, d and x.
 int bulk_step_selftest(unsigned gated, float* r, float* d, float* x);
+
+// Hierarchy of a symmetric CSR matrix (sorted columns), set up with clusters of at most `clusters` blocks: levels,
+// and per level its rows and its fingerprint hash (24 at most); the coarsest inverse (at most 160 x 160).
+int amg_setup_selftest(int n, const int* ptr, const int* col, const double* val, bool fp32, int clusters,
+                       int round3_below, int* levels, int* rows, unsigned long long* hash, double* inverse);
 
 // Device aggregation result: agg (row -> aggregate or -1), members CSR (aggregate -> rows).
 struct Aggregates {
@@ -74,6 +80,9 @@ public:
     // the same cycle for three right-hand sides at once (hierarchies set up with three_vectors)
     void apply3(cudaStream_t s, const V3<T>* r, V3<T>* z, const int* stop);
     int levels() const { return nlev_; }
+    // A hash per level of its matrix (entries, values, diagonal) and of its aggregates with their member lists,
+    // and the coarsest level's inverse: two setups made the same hierarchy.
+    void fingerprint(cudaStream_t s, std::vector<unsigned long long>& hash, std::vector<double>& inverse) const;
     void set_profiler(Profiler* p) { prof_ = p; }
     const std::vector<int>& level_sizes() const { return sizes_; }
     // Algorithmic bytes of one apply() (one V-cycle) of the current hierarchy, in total and per
@@ -134,7 +143,7 @@ private:
     void aggregate_round(cudaStream_t s, const SellPattern& P, const T* A, int n, bool neg_first, Aggregates& out);
     void pairwise(cudaStream_t s, const SellPattern& P, const T* A, int n, bool neg, double theta, bool join,
                   Aggregates& out);
-    void aggregate_small(cudaStream_t s, const SellPattern& P, const T* A, int n, bool neg_first, Aggregates& out);
+    bool aggregate_small(cudaStream_t s, const SellPattern& P, const T* A, int n, bool neg_first, Aggregates& out);
     void compose(cudaStream_t s, Aggregates& first, const Aggregates& second);
     void members(cudaStream_t s, Aggregates& a);
     void galerkin(cudaStream_t s, const SellPattern& P, const T* A, const Aggregates& a, SellPattern& Pc,

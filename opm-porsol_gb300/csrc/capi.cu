@@ -1538,6 +1538,16 @@ int porsol_selftest_bulk_wait(int expire, float* r, float* d, float* x)
     return selftest([&] { return porsol::bulk_step_selftest(gated, r, d, x); });
 }
 
+int porsol_selftest_amg_setup(int n, const int* rowptr, const int* col, const double* val, int precision, int clusters,
+                              int round3_below, int* levels, int* rows, unsigned long long* hash, double* inverse)
+{
+    if (n <= 0 || !rowptr || !col || !val || !levels || !rows || !hash || !inverse) return PORSOL_ERR_BAD_ARG;
+    return selftest([&] {
+        return porsol::amg_setup_selftest(n, rowptr, col, val, precision == PORSOL_MIXED, clusters, round3_below, levels,
+                                          rows, hash, inverse);
+    });
+}
+
 int porsol_selftest_ilu_wait(int thread, int shared, double* z)
 {
     if (!z) return PORSOL_ERR_BAD_ARG;

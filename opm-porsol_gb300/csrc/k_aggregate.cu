@@ -338,46 +338,58 @@ __global__ void __launch_bounds__(AGG_THREADS, 1) k_compose_members(int n, int n
 
 namespace {
 
+// Bytes of the two worklists of a block.
+size_t worklists(int rows, int blocks) { return 2 * sizeof(int) * size_t((rows + blocks - 1) / blocks); }
+
 // Blocks of the cluster: what a level's lanes need at one row (or lane) per thread and sweep, at most 16 (the
-// opt-in size; the grid is one cluster).
-int blocks_for(long long threads)
+// opt-in size; the grid is one cluster), 8 where 16 do not fit the device or the limit; 0: none does.  With fewer
+// than that a level of these sizes would be done sooner by a launch per step.
+template <class... KA>
+int blocks_for(void (*f)(KA...), long long threads, bool lists, int limit)
 {
     int b = 1;
     while (b < AGG_CTAS && threads > (long long)b * AGG_THREADS) b *= 2;
-    return b;
+    for (; b > 0; b = b > 8 ? 8 : 0) {
+        // the largest level that this many blocks may get: up to AGG_ROWS rows for 8 and 16 blocks
+        const int rows = b >= 8 ? AGG_ROWS : b * AGG_THREADS;
+        if (b <= limit && cluster_fits(f, b, AGG_THREADS, lists ? worklists(rows, b) : 0)) return b;
+    }
+    return 0;
 }
 
-template <class... KA, class... A>
-void go(void (*f)(KA...), int blocks, size_t shm, cudaStream_t s, A&&... args)
+template <class T, int K>
+bool agg_launch_lanes(cudaStream_t s, const AggArgs<T>& a, int limit)
 {
-    if (shm > 40 * 1024)   // static shared memory comes on top
-        PORSOL_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shm)));
-    if (blocks > 8) PORSOL_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    launch_cluster(f, blocks, AGG_THREADS, shm, s, false, std::forward<A>(args)...);
+    const int blocks = blocks_for(k_aggregate<T, K>, (long long)a.n * K, true, limit);
+    if (blocks)
+        launch_cluster(k_aggregate<T, K>, blocks, AGG_THREADS, worklists(a.n, blocks), s, false, a);
+    return blocks != 0;
 }
 
 }  // namespace
 
 template <class T>
-void agg_launch(cudaStream_t s, int lanes, const AggArgs<T>& a)
+bool agg_launch(cudaStream_t s, int lanes, const AggArgs<T>& a, int limit)
 {
-    const int blocks = blocks_for((long long)a.n * lanes);
-    const size_t shm = 2 * sizeof(int) * size_t((a.n + blocks - 1) / blocks);
     switch (lanes) {
-    case 1: go(k_aggregate<T, 1>, blocks, shm, s, a); break;
-    case 2: go(k_aggregate<T, 2>, blocks, shm, s, a); break;
-    case 4: go(k_aggregate<T, 4>, blocks, shm, s, a); break;
-    case 8: go(k_aggregate<T, 8>, blocks, shm, s, a); break;
-    default: go(k_aggregate<T, 16>, blocks, shm, s, a); break;
+    case 1: return agg_launch_lanes<T, 1>(s, a, limit);
+    case 2: return agg_launch_lanes<T, 2>(s, a, limit);
+    case 4: return agg_launch_lanes<T, 4>(s, a, limit);
+    case 8: return agg_launch_lanes<T, 8>(s, a, limit);
+    default: return agg_launch_lanes<T, 16>(s, a, limit);
     }
 }
 
-void compose_launch(cudaStream_t s, int n, int nc, int* agg1, const int* agg2, int* cnt, int* ptr, int* idx, int* scratch)
+bool compose_launch(cudaStream_t s, int n, int nc, int* agg1, const int* agg2, int* cnt, int* ptr, int* idx, int* scratch,
+                    int limit)
 {
-    go(k_compose_members, blocks_for(n), 0, s, n, nc, agg1, agg2, cnt, ptr, idx, scratch);
+    const int blocks = blocks_for(k_compose_members, n, false, limit);
+    if (blocks)
+        launch_cluster(k_compose_members, blocks, AGG_THREADS, 0, s, false, n, nc, agg1, agg2, cnt, ptr, idx, scratch);
+    return blocks != 0;
 }
 
-template void agg_launch<float>(cudaStream_t, int, const AggArgs<float>&);
-template void agg_launch<double>(cudaStream_t, int, const AggArgs<double>&);
+template bool agg_launch<float>(cudaStream_t, int, const AggArgs<float>&, int);
+template bool agg_launch<double>(cudaStream_t, int, const AggArgs<double>&, int);
 
 }  // namespace porsol

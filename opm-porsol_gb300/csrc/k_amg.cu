@@ -1613,24 +1613,21 @@ void Amg<T>::members(cudaStream_t s, Aggregates& a)
 }
 
 // One pairing round: the aggregates of a level with their member lists.  Levels of up to AGG_ROWS rows run
-// as one cluster launch (aggregate.h), larger ones as a launch per sweep and step.  Both make the same
+// as one cluster launch (aggregate.h) where the device holds the cluster, others as a launch per sweep and step.  Both make the same
 // decisions and write the same arrays.
 template <class T>
 void Amg<T>::aggregate_round(cudaStream_t s, const SellPattern& P, const T* A, int n, bool neg_first,
                              Aggregates& out)
 {
     out.offsets = false;
-    if (agg_small(n, P.nent)) {
-        aggregate_small(s, P, A, n, neg_first, out);
-        return;
-    }
+    if (agg_small(n, P.nent) && aggregate_small(s, P, A, n, neg_first, out)) return;
     if (neg_first) pairwise(s, P, A, n, true, o_.strength, false, out);
     if (!neg_first || out.nc > 0.8 * n) pairwise(s, P, A, n, false, 0.0, true, out);
     members(s, out);
 }
 
 template <class T>
-void Amg<T>::aggregate_small(cudaStream_t s, const SellPattern& P, const T* A, int n, bool neg_first, Aggregates& out)
+bool Amg<T>::aggregate_small(cudaStream_t s, const SellPattern& P, const T* A, int n, bool neg_first, Aggregates& out)
 {
     s_rs_.alloc(n);
     for (DBuf<int>* b : {&s_state_, &s_partner_, &s_join_, &s_best_, &s_cidx_, &s_cnt_}) b->alloc(size_t(n) + 1);
@@ -1663,7 +1660,7 @@ void Amg<T>::aggregate_small(cudaStream_t s, const SellPattern& P, const T* A, i
     a.goff = s_goff_.p;
     a.woff = s_woff_.p;
     a.scratch = iscratch_.p;
-    agg_launch<T>(s, pick_lanes(n, P.nent), a);
+    if (!agg_launch<T>(s, pick_lanes(n, P.nent), a, o_.setup_cluster)) return false;
     int r[3];
     PORSOL_CUDA(cudaMemcpyAsync(r, iscratch_.p, sizeof(r), cudaMemcpyDeviceToHost, s));
     PORSOL_CUDA(cudaStreamSynchronize(s));
@@ -1671,6 +1668,7 @@ void Amg<T>::aggregate_small(cudaStream_t s, const SellPattern& P, const T* A, i
     out.total = r[1];
     out.bound = r[2];
     out.offsets = true;   // s_goff_ and s_woff_ hold the candidate offsets of this round
+    return true;
 }
 
 // The aggregates of two rounds as one: `first` maps rows to those of the next round's aggregates, with
@@ -1685,8 +1683,9 @@ void Amg<T>::compose(cudaStream_t s, Aggregates& first, const Aggregates& second
         first.ptr.alloc(size_t(first.n) + 1);
         first.idx.alloc(first.n);
         iscratch_.alloc(AGG_SCRATCH);
-        compose_launch(s, first.n, first.nc, first.agg.p, second.agg.p, s_cnt_.p, first.ptr.p, first.idx.p, iscratch_.p);
-        return;
+        if (compose_launch(s, first.n, first.nc, first.agg.p, second.agg.p, s_cnt_.p, first.ptr.p, first.idx.p,
+                           iscratch_.p, o_.setup_cluster))
+            return;
     }
     PORSOL_LAUNCH(k_compose<<<div_up(first.n, TB), TB, 0, s>>>(first.n, first.agg.p, second.agg.p));
     members(s, first);
@@ -1919,8 +1918,10 @@ void Amg<T>::build_coarse_solver(cudaStream_t s, const SellPattern& P, const T* 
     DBuf<double>&D = s_D_, &Linv = s_Linv_;
     cinv_.alloc(std::max<size_t>((size_t)n * n, 1));
     if (n > 0) {
-        if (n <= DENSE_CLUSTER_N) {
-            const size_t shm = size_t(2 + div_up(n, DENSE_CTAS)) * n * sizeof(double);
+        auto bytes = [](int m) { return size_t(2 + div_up(m, DENSE_CTAS)) * m * sizeof(double); };
+        if (n <= DENSE_CLUSTER_N && DENSE_CTAS <= o_.setup_cluster &&
+            cluster_fits(k_dense_inverse<T>, DENSE_CTAS, 512, bytes(DENSE_CLUSTER_N))) {
+            const size_t shm = bytes(n);
             launch_cluster(k_dense_inverse<T>, DENSE_CTAS, 512, shm, s, false, n, (const int*)P.slice_ptr.p,
                            (const int*)P.col.p, (const int*)P.rowlen.p, A, cinv_.p, status_.p);
         } else {
@@ -2091,7 +2092,7 @@ void Amg<T>::choose_tail(cudaStream_t s)
     tail_ = tail_first_ = -1;
     const int last = nlev_ - 2;
     if (blk0_ || lv_[0]->n > TAIL_SYSTEM || o_.smooth_steps != 1 || o_.cheb_degree != 2 || last < 1 || lv_[nlev_ - 1]->n > TAIL_DENSE ||
-        lv_[nlev_ - 1]->n < 1 || !tail_fits<T>(lv_[last]->half, TAIL_SMEM))
+        lv_[nlev_ - 1]->n < 1 || !tail_fits<T>(lv_[last]->half))
         return;
     const long long most = sizeof(T) == 8 ? TAIL_ENTRIES_FP64 : TAIL_ENTRIES_FP16;
     int first = nlev_ - 1;
@@ -2159,6 +2160,70 @@ void Amg<T>::cheb_coefficients(const Level& L, T& inv_theta, T (&c1)[2], T (&c2)
         c2[k] = T(2.0 * rho1 / delta);
         rho = rho1;
     }
+}
+
+template <class T>
+void Amg<T>::fingerprint(cudaStream_t s, std::vector<unsigned long long>& hash, std::vector<double>& inverse) const
+{
+    hash.assign(size_t(nlev_), 14695981039346656037ULL);
+    for (int l = 0; l < nlev_; ++l) {
+        const Level& L = *lv_[size_t(l)];
+        auto add = [&](const auto* d, size_t n) {   // FNV-1a over the bytes
+            std::vector<unsigned char> b(n * sizeof(*d));
+            if (!n) return;
+            PORSOL_CUDA(cudaMemcpyAsync(b.data(), d, b.size(), cudaMemcpyDeviceToHost, s));
+            PORSOL_CUDA(cudaStreamSynchronize(s));
+            for (unsigned char c : b) hash[size_t(l)] = (hash[size_t(l)] ^ c) * 1099511628211ULL;
+        };
+        const SellPattern& P = *L.P;
+        add(P.slice_ptr.p, size_t(P.nslices) + 1);
+        add(P.col.p, size_t(P.nent));
+        add(L.A, size_t(P.nent));
+        add(P.rowlen.p, size_t(P.n));
+        add(P.diag.p, size_t(P.n));
+        if (l + 1 == nlev_) continue;
+        add(L.agg.agg.p, size_t(L.n));
+        add(L.agg.ptr.p, size_t(L.agg.nc) + 1);
+        add(L.agg.idx.p, size_t(read_int(s, L.agg.ptr.p + L.agg.nc)));
+    }
+    inverse.resize(size_t(nc_) * nc_);
+    cinv_.download(inverse.data(), inverse.size(), s);
+    PORSOL_CUDA(cudaStreamSynchronize(s));
+}
+
+int amg_setup_selftest(int n, const int* ptr, const int* col, const double* val, bool fp32, int clusters,
+                       int round3_below, int* levels, int* rows, unsigned long long* hash, double* inverse)
+{
+    cudaStream_t s = nullptr;
+    SellPattern P;
+    HVec<int> slot;
+    build_sell(n, HVec<int>(ptr, ptr + n + 1), HVec<int>(col, col + ptr[n]), P, &slot);
+    P.upload(s);
+    auto run = [&](auto zero) {
+        using T = decltype(zero);
+        std::vector<T> v(size_t(P.nent), T(0));
+        for (int k = 0; k < ptr[n]; ++k) v[size_t(slot[size_t(k)])] = T(val[k]);
+        DBuf<T> A;
+        A.upload(v, s);
+        Amg<T> amg;
+        AmgOpts o;
+        o.setup_cluster = clusters;
+        o.round3_below = round3_below;
+        amg.setup(s, P, A.p, o);
+        std::vector<unsigned long long> h;
+        std::vector<double> inv;
+        amg.fingerprint(s, h, inv);
+        *levels = amg.levels();
+        for (int l = 0; l < *levels; ++l) {
+            rows[l] = amg.level_sizes()[size_t(l)];
+            hash[l] = h[size_t(l)];
+        }
+        PORSOL_REQUIRE(inv.size() <= size_t(DENSE_CLUSTER_N) * DENSE_CLUSTER_N, PORSOL_ERR_BAD_ARG, "coarsest level too large");
+        std::copy(inv.begin(), inv.end(), inverse);
+    };
+    if (fp32) run(0.0f);
+    else run(0.0);
+    return 0;
 }
 
 template <class T>

@@ -2,7 +2,6 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
-#include <mutex>
 
 #include "bulk.cuh"
 #include "cluster.cuh"
@@ -317,12 +316,6 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) k_tail(const __grid_constant_
     }
 }
 
-template <class T>
-void* tail_kernel(bool half)
-{
-    return half ? (void*)k_tail<T, true> : (void*)k_tail<T, false>;
-}
-
 }  // namespace
 
 int tail_lanes(int n)
@@ -371,34 +364,10 @@ int tail_layout(TailArgs<T>& a)
 }
 
 template <class T>
-bool tail_fits(bool half, int shm)
+bool tail_fits(bool half)
 {
-    if (shm > TAIL_SMEM) return false;
-    // asked once per process: the answer does not depend on the data
-    static std::mutex m;
-    static int known[2] = {-1, -1};
-    std::lock_guard<std::mutex> lk(m);
-    int& k = known[half ? 1 : 0];
-    if (k < 0) {
-        void* f = tail_kernel<T>(half);
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = TAIL_CTAS;
-        cfg.blockDim = TAIL_THREADS;
-        cfg.dynamicSmemBytes = TAIL_SMEM;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = TAIL_CTAS;
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        int n = 0;
-        k = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, TAIL_SMEM) == cudaSuccess &&
-                    cudaOccupancyMaxActiveClusters(&n, f, &cfg) == cudaSuccess && n > 0
-                ? 1
-                : 0;
-        cudaGetLastError();
-    }
-    return k == 1;
+    return half ? cluster_fits(k_tail<T, true>, TAIL_CTAS, TAIL_THREADS, TAIL_SMEM)
+                : cluster_fits(k_tail<T, false>, TAIL_CTAS, TAIL_THREADS, TAIL_SMEM);
 }
 
 template <class T>
@@ -414,7 +383,7 @@ void tail_launch(cudaStream_t s, bool half, const TailArgs<T>& a, int shm)
                                const T*, const T*, const int*, int, const int*, const int*, bool, unsigned char*);   \
     template int tail_layout<T>(TailArgs<T>&);                                                                       \
     template void tail_launch<T>(cudaStream_t, bool, const TailArgs<T>&, int);                                       \
-    template bool tail_fits<T>(bool, int);
+    template bool tail_fits<T>(bool);
 PORSOL_TAIL(float)
 PORSOL_TAIL(double)
 #undef PORSOL_TAIL

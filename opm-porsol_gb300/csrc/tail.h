@@ -82,8 +82,8 @@ int tail_layout(TailArgs<T>& a);
 template <class T>
 void tail_launch(cudaStream_t s, bool half, const TailArgs<T>& a, int shm);
 
-// whether the device schedules such a cluster with this much shared memory
+// whether the device holds such a cluster
 template <class T>
-bool tail_fits(bool half, int shm);
+bool tail_fits(bool half);
 
 }  // namespace porsol
