@@ -1201,15 +1201,16 @@ void Ilu0::build_levels(const SellPattern& P, cudaStream_t s, bool shared)
     warp_rows_ = true;
     for (int i = 0; i < n; ++i) warp_rows_ = warp_rows_ && P.h_rowlen[i] <= 32;
     // The fused sweep: step records of at most ILU_ROWS rows of one level and ILU_STAGE bytes.  The vector
-    // goes to shared memory (16-bit row and column numbers) when all levels are fused and it fits beside
+    // goes to shared memory (16-bit row and column numbers) when all levels can be fused and it fits beside
     // two stages.
     bool all = true;
     for (const std::vector<int>* ptr : {&h_lptr_, &h_uptr_})
-        for (size_t l = 0; l + 1 < ptr->size(); ++l) all = all && (*ptr)[l + 1] - (*ptr)[l] <= FUSE_ROWS;
+        for (size_t l = 0; l + 1 < ptr->size(); ++l) all = all && (*ptr)[l + 1] - (*ptr)[l] <= SHARED_ROWS;
     const size_t zbytes = (size_t(n) + 1) * sizeof(double);
     shared_z_ = shared && all && n < 65535 && 128 + zbytes + 2 * size_t(ILU_STAGE) <= ILU_SMEM;
     stages_ = shared_z_ ? std::min<int>(ILU_STAGES, int((ILU_SMEM - 128 - zbytes) / ILU_STAGE)) : ILU_STAGES;
     const size_t ib = shared_z_ ? 2 : 4;
+    const int fused_rows = shared_z_ ? SHARED_ROWS : FUSE_ROWS;
     std::vector<int2> steps;
     std::vector<unsigned char> blob;
     std::vector<int> pos, from;
@@ -1226,7 +1227,7 @@ void Ilu0::build_levels(const SellPattern& P, cudaStream_t s, bool shared)
             return m;
         };
         for (int l = 0; l + 1 < int(ptr.size()); ++l) {
-            if (ptr[l + 1] - ptr[l] > FUSE_ROWS) {
+            if (ptr[l + 1] - ptr[l] > fused_rows) {
                 runs_.push_back({false, l, up});
                 continue;
             }

@@ -157,7 +157,10 @@ private:
 // The levels of a mid-size grid hold tens of rows and a sweep has a hundred levels, so a launch per
 // level costs a launch latency per handful of rows.  Runs of levels of at most FUSE_ROWS rows are swept
 // by one block in one launch (k_ilu_steps), from records of the two triangles in sweep order;
-// wider levels, which would wait for one SM's FP64 pipe, keep a launch of their own.
+// wider levels, which would wait for one SM's FP64 pipe, keep a launch of their own.  Per CG iteration, with
+// levels fused up to 0 / 384 / 512 / 768 / 1024 rows: 30^3 cells 1653 / 1184 / 1186 / 1195 / 1195 us, 40^3 2304 / 1883 /
+// 1876 / 2029 / 2682, 100 x 100 x 10 3539 / 2929 / 3012 / 3234 / 3855, 60^3 5216 / 4571 / 4511 / 4492 / 4638.  Small
+// systems without a level of more than SHARED_ROWS rows are swept in one launch, the vector in shared memory.
 class Ilu0 : public Precond<double> {
 public:
     // structure only; shared: the sweep's vector may live in shared memory
@@ -170,7 +173,7 @@ public:
     int num_levels_upper() const { return int(h_uptr_.size()) - 1; }
 
 private:
-    static constexpr int FUSE_ROWS = 1024;
+    static constexpr int FUSE_ROWS = 512, SHARED_ROWS = 1024;
     const SellPattern* P_ = nullptr;
     DBuf<double> lu_;
     std::vector<int> h_lptr_, h_uptr_;

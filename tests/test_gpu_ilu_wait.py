@@ -38,3 +38,26 @@ def test_any_lanes_timeout_is_reported(pkg, gpulib, lane):
     assert rc == TIMEOUT
     assert np.all(r == 2.0)   # the step wrote nothing
     assert pkg.selftest_bulk_wait(False)[0] == 0
+
+
+def launches_per_iteration(pkg, workloads, dims):
+    prob = workloads.layered_lognormal(dims=dims, seed=5, sat=np.full(int(np.prod(dims)), 0.3))
+    s = pkg.PressureSolver()
+    s.init(prob.grid, prob.perm.ravel(), (0.0, 0.0, 0.0), prob.bc_type)
+    n = []
+    for maxit in (2, 6):
+        before = pkg.lib().porsol_launch_count()
+        with pytest.raises(pkg.PorsolError) as e:
+            s.solve(pkg.Fluid(*prob.fluid), prob.sat, prob.bc_type, prob.bc_value, prob.src,
+                    opts=pkg.default_solve_opts(linsolver_type=0, residual_tolerance=1e-12, linsolver_maxit=maxit))
+        assert e.value.code == 1   # stopped at the iteration limit
+        n.append(pkg.lib().porsol_launch_count() - before)
+    s.close()
+    return (n[1] - n[0]) / 4
+
+
+def test_wide_levels_keep_their_own_launches(pkg, gpulib, workloads):
+    """One block takes longer over a level of more than 512 rows than a launch does: 10^3 cells are swept in one
+    launch (with the CG's four), 36^3, whose middle levels hold 600 to 1000 rows, in hundreds."""
+    assert launches_per_iteration(pkg, workloads, (10, 10, 10)) == 5
+    assert launches_per_iteration(pkg, workloads, (36, 36, 36)) > 100
