@@ -83,10 +83,10 @@ struct porsol_transport {
     porsol::DBuf<int> fe_c0, fe_c1, fe_hf, bc_cell;
     porsol::DBuf<double> fe_G, fe_capf, fe_nn, bc_sat;
     porsol::DBuf<porsol::CellState> cstate;
-    // the viscous-only sub-step: outflow coefficient and inflow list of each cell (written once per
-    // call), and two fractional-flow buffers (read one, write the other)
+    // the viscous-only sub-step: outflow (and what its rounding left), time step over pore volume and inflow
+    // list of each cell (written once per call), and two fractional-flow buffers (read one, write the other)
     porsol::DBuf<int> in_cnt, in_src;
-    porsol::DBuf<double> in_out, in_coef, frac, frac2;
+    porsol::DBuf<double> in_out, in_left, in_scale, in_coef, frac, frac2;
     bool any_gravity = false;   // some face entry has a non-zero gravity driving force
     porsol::DBuf<unsigned long long> red;
     porsol::DBuf<double> cfl_part;   // per-block minima of the CFL bounds
