@@ -444,6 +444,8 @@ int porsol_selftest_bulk_wait(int expire, float* r, float* d, float* x);
  * the wait of that thread of the sweep's block (0..287, 256 the one that copies) for the first step's record
  * runs out (about 20 ms): the call returns PORSOL_ERR_TIMEOUT with the context still usable. */
 int porsol_selftest_ilu_wait(int thread, int shared, double* z);
+/* q[i] = num[i] / den[i] and r[i] = 1 / den[i] as the kernels form them (host arrays), on the current device. */
+int porsol_selftest_quotients(int n, const double* num, const double* den, double* q, double* r);
 /* Sets up the AMG hierarchy of a symmetric positive definite CSR matrix (host arrays, sorted columns) in the given
  * precision (PORSOL_MIXED: FP32) on the current device, with clusters of at most `clusters` blocks (16 or 8; 0: a
  * launch per step, as on a device that cannot hold the clusters) and three pairing rounds on coarse levels of

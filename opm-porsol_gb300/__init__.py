@@ -184,6 +184,7 @@ EXPORTS = [
     ("porsol_launch_count", C.c_longlong, []),
     ("porsol_selftest_bulk_wait", C.c_int, [C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]),
     ("porsol_selftest_ilu_wait", C.c_int, [C.c_int, C.c_int, C.c_void_p]),
+    ("porsol_selftest_quotients", C.c_int, [_i, _vp, _vp, _vp, _vp]),
     ("porsol_selftest_amg_setup", C.c_int, [_i, _vp, _vp, _vp, _i, _i, _i, _vp, _vp, _vp, _vp]),
     ("porsol_transport_cfl_noalloc", _i, [_i, _vp, _vp, _vp, _vp, _d, C.POINTER(_d), _vp]),
 ]
@@ -223,6 +224,16 @@ def selftest_ilu_wait(thread: int = -1, shared: bool = True):
     z = np.zeros(48)
     rc = lib().porsol_selftest_ilu_wait(int(thread), int(shared), _p(z))
     return rc, z
+
+
+def selftest_quotients(num, den):
+    """num / den and 1 / den by the kernels' quotient() and reciprocal()."""
+    num, den = (np.ascontiguousarray(a, np.float64) for a in (num, den))
+    q, r = np.zeros(len(den)), np.zeros(len(den))
+    rc = lib().porsol_selftest_quotients(len(den), _p(num), _p(den), _p(q), _p(r))
+    if rc:
+        raise PorsolError(rc, "quotients self-test")
+    return q, r
 
 
 def selftest_amg_setup(matrix, precision=FP64, clusters=16, round3_below=0):

@@ -1548,6 +1548,12 @@ int porsol_selftest_amg_setup(int n, const int* rowptr, const int* col, const do
     });
 }
 
+int porsol_selftest_quotients(int n, const double* num, const double* den, double* q, double* r)
+{
+    if (n <= 0 || !num || !den || !q || !r) return PORSOL_ERR_BAD_ARG;
+    return selftest([&] { return porsol::quotients_selftest(n, num, den, q, r); });
+}
+
 int porsol_selftest_ilu_wait(int thread, int shared, double* z)
 {
     if (!z) return PORSOL_ERR_BAD_ARG;

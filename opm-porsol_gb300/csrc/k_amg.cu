@@ -16,6 +16,7 @@
 #include "bulk.cuh"
 #include "cluster.cuh"
 #include "match.cuh"
+#include "quotient.cuh"
 #include "sell.cuh"
 
 namespace porsol {
@@ -1343,15 +1344,6 @@ __global__ void k_dense_cholesky_inverse(int n, double* __restrict__ D, double* 
 // updates.  FP64-issue bound (two operations a clock and SM): eight SMs, one FMA per entry and pivot, one
 // division per pivot instead of one per warp and pivot; 108 rows take 219 us, one block with a division in
 // every thread took 718 us.  Non-positive or non-finite pivots set ST_NONFINITE.
-// 1 / x by two Newton steps from the hardware's estimate (within an ulp or two; x normal)
-__device__ __forceinline__ double reciprocal(double x)
-{
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    r = fma(r, fma(-x, r, 1.0), r);
-    return fma(r, fma(-x, r, 1.0), r);
-}
-
 constexpr int DENSE_CLUSTER_N = 160;
 constexpr int DENSE_CTAS = 8;
 template <class T>

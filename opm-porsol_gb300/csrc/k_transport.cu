@@ -481,9 +481,34 @@ void single_rock_cfl(double mu1, double mu2, const RockView* R, int rock, double
     out[2] = maxffg * mdpc;   // 0 without a rock table
 }
 
+__global__ void k_quotients(int n, const double* __restrict__ num, const double* __restrict__ den,
+                            double* __restrict__ q, double* __restrict__ r)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    q[i] = quotient(num[i], den[i]);
+    r[i] = reciprocal(den[i]);
+}
+
 }  // namespace
 
 namespace porsol {
+
+int quotients_selftest(int n, const double* num, const double* den, double* q, double* r)
+{
+    cudaStream_t s = nullptr;
+    DBuf<double> a, b, c, d;
+    a.upload(num, n, s);
+    b.upload(den, n, s);
+    c.alloc(n);
+    d.alloc(n);
+    PORSOL_LAUNCH(k_quotients<<<div_up(n, TB), TB, 0, s>>>(n, a.p, b.p, c.p, d.p));
+    PORSOL_CUDA(cudaGetLastError());
+    c.download(q, n, s);
+    d.download(r, n, s);
+    PORSOL_CUDA(cudaStreamSynchronize(s));
+    return 0;
+}
 
 void launch_cell_state(cudaStream_t s, const FaceTables& f, const double* sat, const TrParams& p, const RockTab& R,
                        CellState* cs)

@@ -154,4 +154,7 @@ int sum_scratch_size();
 int sum_result_index(int n);
 void launch_sum(cudaStream_t s, int n, const double* x, double* scratch);
 
+// q = num / den and r = 1 / den by the kernels' quotient() and reciprocal() (host arrays)
+int quotients_selftest(int n, const double* num, const double* den, double* q, double* r);
+
 }  // namespace porsol

@@ -12,6 +12,10 @@
 #include <cmath>
 #include <cstring>
 
+#ifdef __CUDACC__
+#include "quotient.cuh"
+#endif
+
 namespace porsol {
 
 struct RockView {
@@ -131,17 +135,6 @@ __device__ __forceinline__ const double* tab_row(const RockTab& R, int r, double
         dx = v - R.node[8 * size_t(lo)];
     }
     return R.node + 8 * size_t(lo);
-}
-
-// num / den in five FP64 operations: the hardware's reciprocal estimate, one Newton step, and the
-// quotient corrected once by its remainder (Markstein, IBM J. Res. Dev. 34, 1990).
-__device__ __forceinline__ double quotient(double num, double den)
-{
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(den));
-    r = fma(r, fma(-den, r, 1.0), r);
-    const double q = num * r;
-    return fma(fma(-den, q, num), r, q);
 }
 #endif
 
