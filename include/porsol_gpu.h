@@ -444,6 +444,12 @@ int porsol_selftest_bulk_wait(int expire, float* r, float* d, float* x);
  * the wait of that thread of the sweep's block (0..287, 256 the one that copies) for the first step's record
  * runs out (about 20 ms): the call returns PORSOL_ERR_TIMEOUT with the context still usable. */
 int porsol_selftest_ilu_wait(int thread, int shared, double* z);
+/* Solves A x = b (symmetric CSR matrix with sorted columns, host arrays) from x = 0 by the mixed-precision CG with
+ * residual replacements whenever the iterated residual has dropped by delta, and a Jacobi preconditioner whose
+ * applications skip .. skip + skips - 1 (0 the first) return zero.  guarded: the solve ended in the guarded form of
+ * the recurrence.  Returns PORSOL_OK, PORSOL_ERR_NOT_CONVERGED or PORSOL_ERR_NONFINITE (breakdown). */
+int porsol_selftest_mixed_cg(int n, const int* rowptr, const int* col, const double* val, const double* b, double* x,
+                             double tol, int maxit, double delta, int skip, int skips, int* iterations, int* guarded);
 /* q[i] = num[i] / den[i] and r[i] = 1 / den[i] as the kernels form them (host arrays), on the current device. */
 int porsol_selftest_quotients(int n, const double* num, const double* den, double* q, double* r);
 /* Sets up the AMG hierarchy of a symmetric positive definite CSR matrix (host arrays, sorted columns) in the given

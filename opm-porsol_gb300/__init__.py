@@ -184,6 +184,7 @@ EXPORTS = [
     ("porsol_launch_count", C.c_longlong, []),
     ("porsol_selftest_bulk_wait", C.c_int, [C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]),
     ("porsol_selftest_ilu_wait", C.c_int, [C.c_int, C.c_int, C.c_void_p]),
+    ("porsol_selftest_mixed_cg", C.c_int, [_i, _vp, _vp, _vp, _vp, _vp, _d, _i, _d, _i, _i, _vp, _vp]),
     ("porsol_selftest_quotients", C.c_int, [_i, _vp, _vp, _vp, _vp]),
     ("porsol_selftest_amg_setup", C.c_int, [_i, _vp, _vp, _vp, _i, _i, _i, _vp, _vp, _vp, _vp]),
     ("porsol_transport_cfl_noalloc", _i, [_i, _vp, _vp, _vp, _vp, _d, C.POINTER(_d), _vp]),
@@ -224,6 +225,17 @@ def selftest_ilu_wait(thread: int = -1, shared: bool = True):
     z = np.zeros(48)
     rc = lib().porsol_selftest_ilu_wait(int(thread), int(shared), _p(z))
     return rc, z
+
+
+def selftest_mixed_cg(matrix, b, tol, maxit, delta, skip=-1, skips=0):
+    """The mixed-precision CG on a scipy CSR matrix (porsol_selftest_mixed_cg): status code, x, iterations, whether
+    it ended guarded."""
+    ptr, col = (np.ascontiguousarray(a, np.int32) for a in (matrix.indptr, matrix.indices))
+    val, b = np.ascontiguousarray(matrix.data, np.float64), np.ascontiguousarray(b, np.float64)
+    x, its, guarded = np.zeros(len(b)), np.zeros(1, np.int32), np.zeros(1, np.int32)
+    rc = lib().porsol_selftest_mixed_cg(len(b), _p(ptr), _p(col), _p(val), _p(b), _p(x), float(tol), int(maxit),
+                                        float(delta), int(skip), int(skips), _p(its), _p(guarded))
+    return rc, x, int(its[0]), bool(guarded[0])
 
 
 def selftest_quotients(num, den):

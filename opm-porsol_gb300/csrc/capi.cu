@@ -1548,6 +1548,15 @@ int porsol_selftest_amg_setup(int n, const int* rowptr, const int* col, const do
     });
 }
 
+int porsol_selftest_mixed_cg(int n, const int* rowptr, const int* col, const double* val, const double* b, double* x,
+                             double tol, int maxit, double delta, int skip, int skips, int* iterations, int* guarded)
+{
+    if (n <= 0 || !rowptr || !col || !val || !b || !x || !iterations || !guarded) return PORSOL_ERR_BAD_ARG;
+    return selftest([&] {
+        return porsol::mixed_cg_selftest(n, rowptr, col, val, b, x, tol, maxit, delta, skip, skips, iterations, guarded);
+    });
+}
+
 int porsol_selftest_quotients(int n, const double* num, const double* den, double* q, double* r)
 {
     if (n <= 0 || !num || !den || !q || !r) return PORSOL_ERR_BAD_ARG;

@@ -348,11 +348,16 @@ __global__ void __launch_bounds__(RED_THREADS, 2) k_rc_init(int n, const int* __
 }
 
 // at the start and after a replacement: r = r64 / sigma in FP32, p in the new units, the preconditioner's
-// start from r
+// start from r.  A breakdown found by k_rc_update stops the solve here: threads that still read the flag do
+// the same work either way.
 __global__ void k_rc_rescale(int n, const double* __restrict__ r64, float* __restrict__ r, float* __restrict__ p,
-                             const RcDev* st, Precond<float>::Start start, int init)
+                             RcDev* st, Precond<float>::Start start, int init, CgHostView* hv)
 {
     chain_wait();
+    if (blockIdx.x == 0 && threadIdx.x == 0 && st->breakdown && !st->stop) {
+        st->stop = 1;
+        rc_publish(st, hv);
+    }
     if (st->stop || !(init || st->replaced)) return;
     const double is = st->isig;
     const float f = st->factor;
@@ -393,12 +398,14 @@ __global__ void __launch_bounds__(RED_THREADS, 2) k_rc_pq(int n, const int* __re
 
 // alpha = rho / (p . q) (guarded: (p . r) / (p . q)); x += sigma alpha p (FP64); r -= alpha q; the
 // preconditioner's start from r; partial sums of r . r.  Where the curvature is not positive nothing changes
-// (alpha = 0): the direction starts anew from z, guarded; the solve stops if it had just done so.
+// (alpha = 0): the direction starts anew from z, guarded.  That happens once: in a direction just started anew, or
+// in the guarded form, which keeps the directions conjugate, the matrix itself is not positive definite and the
+// solve stops (restarting on and on, indefinite systems ran up to 3000 iterations into an overflow).
 __global__ void __launch_bounds__(RED_THREADS, 2) k_rc_update(int n, double* __restrict__ x, float* __restrict__ r,
                                                   const float* __restrict__ p, const float* __restrict__ q,
                                                   RcDev* st, const double* __restrict__ pq,
                                                   const double* __restrict__ pr, Precond<float>::Start start,
-                                                  double* __restrict__ part, CgHostView* hv)
+                                                  double* __restrict__ part)
 {
     chain_wait();
     if (st->stop) return;
@@ -415,11 +422,7 @@ __global__ void __launch_bounds__(RED_THREADS, 2) k_rc_update(int n, double* __r
         if (blockIdx.x == 0) {
             st->pq = curv;
             st->restart = !ok;
-            if (!ok && (st->fresh || !isfinite(curv))) {
-                st->breakdown = 1;
-                st->stop = 1;
-                rc_publish(st, hv);
-            }
+            if (!ok && (st->fresh || guard || !isfinite(curv))) st->breakdown = 1;   // k_rc_rescale stops the solve
         }
     }
     __syncthreads();
@@ -1048,14 +1051,14 @@ void ReliableCg::iteration(cudaStream_t s, const SellPattern& P, const double* v
         if (pf) prof->end(s, PK_SPMV32, bytes, ev);
     }
     const Precond<float>::Start start = M.start();
-    chain(k_rc_update, nr, tb, 0, s, n, x, r_.p, p_.p, q_.p, st_.p, pq_.p, pr_.p, start, rr_.p, dview_);
+    chain(k_rc_update, nr, tb, 0, s, n, x, r_.p, p_.p, q_.p, st_.p, pq_.p, pr_.p, start, rr_.p);
     if (P.has_off16())
         chain(k_rc_true<short>, nr, tb, 0, s, n, P.slice_ptr.p, P.off16.p, val64, x, b, r64_.p, st_.p, rr_.p,
               red_.partial.p, red_.counter.p, dview_);
     else
         chain(k_rc_true<int>, nr, tb, 0, s, n, P.slice_ptr.p, P.col.p, val64, x, b, r64_.p, st_.p, rr_.p,
               red_.partial.p, red_.counter.p, dview_);
-    chain(k_rc_rescale, nr, tb, 0, s, n, r64_.p, r_.p, p_.p, st_.p, start, 0);
+    chain(k_rc_rescale, nr, tb, 0, s, n, r64_.p, r_.p, p_.p, st_.p, start, 0, dview_);
     if (start.dinv) M.apply_started(s, r_.p, z_.p, stop);
     else M.apply(s, r_.p, z_.p, stop);
     chain(k_rc_zr, nr, tb, 0, s, n, z_.p, r_.p, q_.p, st_.p, zr_.p, 0);
@@ -1088,7 +1091,7 @@ CgResult ReliableCg::solve(cudaStream_t s, const SellPattern& P, const double* v
         chain(k_rc_init<int>, nr, tb, 0, s, n, P.slice_ptr.p, P.col.p, val64, x, b, r64_.p, st_.p, red_.partial.p,
             red_.counter.p, dview_);
     const Precond<float>::Start start = M.start();
-    chain(k_rc_rescale, nr, tb, 0, s, n, r64_.p, r_.p, p_.p, st_.p, start, 1);
+    chain(k_rc_rescale, nr, tb, 0, s, n, r64_.p, r_.p, p_.p, st_.p, start, 1, dview_);
     const int* stop = &st_.p->stop;
     if (start.dinv) M.apply_started(s, r_.p, z_.p, stop);
     else M.apply(s, r_.p, z_.p, stop);
@@ -1145,6 +1148,7 @@ CgResult ReliableCg::solve(cudaStream_t s, const SellPattern& P, const double* v
     PORSOL_CUDA(cudaMemcpyAsync(&fin, st_.p, sizeof(RcDev), cudaMemcpyDeviceToHost, s));
     PORSOL_CUDA(cudaStreamSynchronize(s));
     nrep_ = fin.nrep;
+    guarded_ = fin.guard != 0;
     res.iterations = fin.iter;
     res.def0 = fin.def0;
     res.def = fin.true_def;
@@ -1152,6 +1156,79 @@ CgResult ReliableCg::solve(cudaStream_t s, const SellPattern& P, const double* v
     res.breakdown = fin.breakdown != 0;
     res.reduction = fin.def0 > 0 ? fin.true_def / fin.def0 : 0.0;
     return res;
+}
+
+namespace {
+// z = D^-1 r, zero in the applications [skip, skip + skips) (counted on the device, so in graphs too)
+__global__ void k_test_precond(int n, const float* __restrict__ dinv, const float* __restrict__ r,
+                               float* __restrict__ z, const int* __restrict__ count, int skip, int skips,
+                               const int* stop)
+{
+    if (*stop) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool zero = *count >= skip && *count < skip + skips;
+    if (i < n) z[i] = zero ? 0.0f : dinv[i] * r[i];
+}
+__global__ void k_test_count(int* count, const int* stop)
+{
+    if (!*stop) ++*count;
+}
+struct TestPrecond : Precond<float> {
+    int n = 0, skip = 0, skips = 0;
+    DBuf<float> dinv;
+    DBuf<int> count;
+    void apply(cudaStream_t s, const float* r, float* z, const int* stop) override
+    {
+        PORSOL_LAUNCH(k_test_precond<<<div_up(n, RB), RB, 0, s>>>(n, dinv.p, r, z, count.p, skip, skips, stop));
+        PORSOL_LAUNCH(k_test_count<<<1, 1, 0, s>>>(count.p, stop));
+    }
+};
+}  // namespace
+
+int mixed_cg_selftest(int n, const int* ptr, const int* col, const double* val, const double* b, double* x, double tol,
+                      int maxit, double delta, int skip, int skips, int* iterations, int* guarded)
+{
+    struct Stream {   // the default stream cannot be captured
+        cudaStream_t s = nullptr;
+        Stream() { PORSOL_CUDA(cudaStreamCreate(&s)); }
+        ~Stream() { cudaStreamDestroy(s); }
+    } own;
+    const cudaStream_t s = own.s;
+    SellPattern P;
+    HVec<int> slot;
+    build_sell(n, HVec<int>(ptr, ptr + n + 1), HVec<int>(col, col + ptr[n]), P, &slot);
+    P.upload(s);
+    std::vector<double> v(size_t(P.nent), 0.0);
+    std::vector<float> v32(v.size(), 0.0f), d(n, 0.0f);
+    for (int i = 0; i < n; ++i)
+        for (int k = ptr[i]; k < ptr[i + 1]; ++k) {
+            v[size_t(slot[size_t(k)])] = val[k];
+            v32[size_t(slot[size_t(k)])] = float(val[k]);
+            if (col[k] == i) d[size_t(i)] = float(1.0 / val[k]);
+        }
+    DBuf<double> a, bd, xd;
+    DBuf<float> a32;
+    a.upload(v, s);
+    a32.upload(v32, s);
+    bd.upload(b, n, s);
+    xd.alloc(n);
+    xd.zero(s);
+    TestPrecond M;
+    M.n = n;
+    M.skip = skip;
+    M.skips = skips;
+    M.dinv.upload(d, s);
+    M.count.alloc(1);
+    M.count.zero(s);
+    ReliableCg cg;
+    const CgResult r = cg.solve(s, P, a.p, a32.p, M, bd.p, xd.p, tol, maxit, delta);
+    xd.download(x, n, s);
+    PORSOL_CUDA(cudaStreamSynchronize(s));
+    *iterations = r.iterations;
+    *guarded = cg.guarded() ? 1 : 0;
+    if (r.breakdown) throw Error(PORSOL_ERR_NONFINITE, "CG breakdown");
+    if (!r.converged) throw Error(PORSOL_ERR_NOT_CONVERGED, "not converged");
+    return 0;
 }
 
 // ---------------- ILU(0) host side ----------------

@@ -114,7 +114,7 @@ private:
 // thousands or broke down, the others 40 to 80).  A stage between replacements that lasts RC_STAGE iterations
 // (10 to 15 are usual), or a curvature that is not positive, switches to the guarded form, alpha = p.r / p.q
 // and beta = -z.q / p.q, which minimise along the direction at hand whatever came before: a solve of 5874
-// iterations then takes 180.
+// iterations then takes 180.  A curvature that is not positive in the guarded form ends the solve.
 struct RcDev {
     double rho[2], pq, sigma, isig, def0, tol, delta, true_def;
     float factor;
@@ -129,10 +129,12 @@ public:
                    Precond<float>& M, const double* b, double* x, double tol, int maxit, double delta,
                    Profiler* prof = nullptr);
     int replacements() const { return nrep_; }
+    bool guarded() const { return guarded_; }   // the last solve ended in the guarded form
     ~ReliableCg();
 
 private:
     int n_ = 0, nrep_ = 0;
+    bool guarded_ = false;
     DBuf<float> r_, z_, p_, q_;
     DBuf<double> r64_;       // the true residual at a replacement
     DBuf<RcDev> st_;
@@ -149,6 +151,11 @@ private:
     void iteration(cudaStream_t s, const SellPattern& P, const double* val64, const float* val32, Precond<float>& M,
                    const double* b, double* x, Profiler* prof);
 };
+
+// Mixed CG from x = 0 on a symmetric CSR matrix (host arrays) with a Jacobi preconditioner whose applications
+// [skip, skip + skips) return zero (a direction of zero curvature); throws what a solve does.
+int mixed_cg_selftest(int n, const int* ptr, const int* col, const double* val, const double* b, double* x, double tol,
+                      int maxit, double delta, int skip, int skips, int* iterations, int* guarded);
 
 // ILU(0) with the pivots stored inverted, factor and triangular solves level-scheduled
 // (rows of one level are independent).  The algorithm of dune-istl's SeqILU0 with
