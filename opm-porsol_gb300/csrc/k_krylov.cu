@@ -354,11 +354,14 @@ __global__ void k_rc_rescale(int n, const double* __restrict__ r64, float* __res
                              RcDev* st, Precond<float>::Start start, int init, CgHostView* hv)
 {
     chain_wait();
-    if (blockIdx.x == 0 && threadIdx.x == 0 && st->breakdown && !st->stop) {
-        st->stop = 1;
-        rc_publish(st, hv);
+    const int stop = st->stop, broken = st->breakdown, replaced = st->replaced;
+    if (stop || broken || !(init || replaced)) {
+        if (broken && !stop && blockIdx.x == 0 && threadIdx.x == 0) {
+            st->stop = 1;
+            rc_publish(st, hv);
+        }
+        return;
     }
-    if (st->stop || !(init || st->replaced)) return;
     const double is = st->isig;
     const float f = st->factor;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
