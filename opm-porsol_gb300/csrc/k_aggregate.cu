@@ -258,7 +258,7 @@ __device__ void member_lists(const Part& rows, int rank, int nc, const int* agg,
 }
 
 // Latency bound: about 30 cluster barriers and as many dependent L2 accesses; the level's entries are
-// read by eight SMs once for the isolated rows, once per full sweep and for the rows still free after it.
+// read by the cluster's SMs once for the isolated rows, once per full sweep and for the rows still free after it.
 template <class T, int K>
 __global__ void __launch_bounds__(AGG_THREADS, 1) k_aggregate(const AggArgs<T> a)
 {

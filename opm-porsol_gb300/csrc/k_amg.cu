@@ -1838,8 +1838,8 @@ void Amg<T>::smoother_setup(cudaStream_t s, Level& L, int level)
     }
 }
 
-// Lane schedule autotuner: for a level shape not seen before, time one smoother step with 1, 2,
-// 4, 8 and 16 lanes per row and keep the fastest.  Shapes are bucketed by value width, log2 of
+// Lane schedule autotuner: for a level shape not seen before, time one smoother step (of one vector, also where
+// the cycle then runs on three) with 1, 2, 4, 8 and 16 lanes per row and keep the fastest.  Shapes are bucketed by value width, log2 of
 // the row count and the mean padded row length, so nearby hierarchies (the next solve of an
 // IMPES run, the next batch of sub-grids) reuse the choice without timing again.
 template <class T>

@@ -549,47 +549,7 @@ __global__ void __launch_bounds__(RED_THREADS, 2) k_rc_direction(int n, const fl
 // ---------------- ILU(0) ----------------
 __device__ __forceinline__ int sell_slot(const int* sp, int r, int t) { return sp[r >> 5] + t * 32 + (r & 31); }
 
-__global__ void k_ilu_factor_level(int nrows, const int* __restrict__ rows, const int* __restrict__ sp,
-                                   const int* __restrict__ col, const int* __restrict__ rowlen,
-                                   const int* __restrict__ diag, double* __restrict__ lu, int* status)
-{
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= nrows) return;
-    const int i = rows[q];
-    const int li = rowlen[i];
-    for (int t = 0; t < li; ++t) {
-        const int ij = sell_slot(sp, i, t);
-        const int j = col[ij];
-        if (j >= i) break;
-        const int jj = diag[j];
-        lu[ij] *= lu[jj];                     // L_ij = a_ij * inv(a_jj)
-        const double lij = lu[ij];
-        // a_ik -= L_ij a_jk for k > j present in both rows
-        const int lj = rowlen[j];
-        int tj = 0;
-        while (tj < lj && col[sell_slot(sp, j, tj)] <= j) ++tj;
-        int ti = t + 1;
-        while (ti < li && tj < lj) {
-            const int ik = sell_slot(sp, i, ti), jk = sell_slot(sp, j, tj);
-            const int ci = col[ik], cj = col[jk];
-            if (ci == cj) {
-                lu[ik] -= lij * lu[jk];
-                ++ti;
-                ++tj;
-            } else if (ci < cj) {
-                ++ti;
-            } else {
-                ++tj;
-            }
-        }
-    }
-    const int d = diag[i];
-    const double piv = lu[d];
-    if (!(fabs(piv) > 0.0) || !isfinite(piv)) atomicOr(status, ST_NONFINITE);
-    lu[d] = 1.0 / piv;
-}
-
-// The same factorisation of one level with a warp per row (every row at most 32 entries): lane t holds
+// Factorisation of one level with a warp per row (rows of at most 32 entries): lane t holds
 // entry t of row i.  The finished rows j < i it needs are read lane by entry, two at a time ahead of
 // their use, and lane t finds its column in row j among the lanes.  Each entry takes the updates of the
 // serial walk in its order.  A level of the 10^3 cube takes about a launch latency instead of the 27 us
@@ -1278,8 +1238,8 @@ void Ilu0::build_levels(const SellPattern& P, cudaStream_t s, bool shared)
     bucket(ulev, nu, h_uptr_, urows, true);
     lrows_.upload(lrows, s);
     urows_.upload(urows, s);
-    warp_rows_ = true;
-    for (int i = 0; i < n; ++i) warp_rows_ = warp_rows_ && P.h_rowlen[i] <= 32;
+    // two cells of at most 12 faces share a face: 23 entries at most
+    for (int i = 0; i < n; ++i) PORSOL_REQUIRE(P.h_rowlen[i] <= 32, PORSOL_ERR_BAD_ARG, "ILU0: row too long");
     // The fused sweep: step records of at most ILU_ROWS rows of one level and ILU_STAGE bytes.  The vector
     // goes to shared memory (16-bit row and column numbers) when all levels can be fused and it fits beside
     // two stages.
@@ -1385,13 +1345,8 @@ void Ilu0::factor(cudaStream_t s, const SellPattern& P, const double* val)
     DBuf<int>& status = status_;
     for (size_t l = 0; l + 1 < h_lptr_.size(); ++l) {
         const int cnt = h_lptr_[l + 1] - h_lptr_[l];
-        if (warp_rows_)
-            chain(k_ilu_factor_warp, div_up(cnt, 4), 128, 0, s, cnt, lrows_.p + h_lptr_[l], P.slice_ptr.p, P.col.p,
-                  P.rowlen.p, P.diag.p, lu_.p, status.p);
-        else
-            PORSOL_LAUNCH(k_ilu_factor_level<<<div_up(cnt, 128), 128, 0, s>>>(cnt, lrows_.p + h_lptr_[l],
-                                                                              P.slice_ptr.p, P.col.p, P.rowlen.p,
-                                                                              P.diag.p, lu_.p, status.p));
+        chain(k_ilu_factor_warp, div_up(cnt, 4), 128, 0, s, cnt, lrows_.p + h_lptr_[l], P.slice_ptr.p, P.col.p,
+              P.rowlen.p, P.diag.p, lu_.p, status.p);
     }
     PORSOL_CUDA(cudaGetLastError());
     if (pos_.n)

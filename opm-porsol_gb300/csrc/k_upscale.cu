@@ -202,8 +202,8 @@ __device__ __forceinline__ void group_sync()
 // Position of direction d of unknown i in the three-direction vectors: side by side (L = 0,
 // 3 i + d: one run per gathered column) or direction-major (L = 1, d n + i: every streamed access
 // of a warp is one contiguous run).  The autotuner tries both; they measured within a few per cent
-// of each other, either ahead.  A third layout, side by side padded to four values and accessed as
-// 16-byte vectors (fewer memory instructions), measured no faster and was removed.
+// of each other, either ahead.  Padding all of them to four values measured no faster; the direction p, which
+// is gathered, has that layout of its own (ldp).
 template <int L>
 __device__ __forceinline__ size_t vix(int i, int d, int n)
 {
@@ -984,7 +984,7 @@ UpscaleResult PersistentUpscale::solve(cudaStream_t s, const SellPattern& P, con
         // start: diagonal and b twice, x, r, p; per iteration: stored entries (column 4 + FP32 value
         // 4), p gathered once, its own value read and q written (3 x 4 each), pass B (D^-1 4; x read
         // and written 16, p 4, r read and written 8, q 4 per direction) and pass C (D^-1 4; r 4, p
-        // read and written 8 per direction); replacements are not counted
+        // read and written 8 per direction); p's fourth, unused value and replacements are not counted
         const double n = nrow[size_t(g)];
         bytes_ += n * (12.0 + 48.0 + 3 * (8.0 + 4.0 + 4.0)) +
                   gi * n * (8.0 * avg_entries + 36.0 + 4.0 + 3 * 32.0 + 4.0 + 3 * 12.0);

@@ -186,7 +186,6 @@ private:
     std::vector<int> h_lptr_, h_uptr_;
     DBuf<int> lrows_, urows_;
     DBuf<int> status_;
-    bool warp_rows_ = false;   // every row fits a warp (the factorisation then takes one warp per row)
     // a launch of apply(): steps [a, b) of the fused sweep, or (fused false) level a of the lower (b = 0)
     // or upper (b = 1) triangle
     struct Run {

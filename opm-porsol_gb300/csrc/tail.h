@@ -21,10 +21,11 @@ constexpr int TAIL_ROWS = 4096;                    // rows of its first level at
 constexpr int TAIL_BLOB = 160 * 1024;              // bytes of one level's part of one block at most
 constexpr int TAIL_SMEM = 224 * 1024;
 constexpr int TAIL_DENSE = 160;                    // rows of the dense level at most
-// Unknowns of the system at most.  Above, the per-level kernels keep their order of sums: the launches
-// saved are 1 to 3 % of a cycle there (3M unknowns: 20 us of 800), and what a solve to the tightest
-// tolerances leaves in single fluxes of a strongly heterogeneous system (1e-7 of their mean) follows every
-// rounding of the cycle.
+// Unknowns of the system at most.  The tail adds a row's entries in another order than the per-level kernels,
+// and what a solve to the tightest tolerances leaves in single fluxes of a strongly heterogeneous system follows
+// every rounding of the cycle: at 3M unknowns in mixed precision by 1e-7 of their mean, for 1 to 3 % of a cycle
+// saved (20 us of 800).  Measured on systems of 3M (not taken) and of up to 1.5M unknowns (taken: 5 to 13 % of an
+// iteration); the limit lies between the two.
 constexpr int TAIL_SYSTEM = 2 << 20;
 
 // Part of one level that one block owns, as k_tail_pack writes it (offsets in bytes from its start; the
