@@ -35,7 +35,8 @@ namespace {
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int UP_MAX_THREADS = 1024;
 constexpr int UP_MAX_WARPS = UP_MAX_THREADS / 32;
-constexpr int TUNE_ITERS = 48;   // CG iterations of the largest sub-grid in one autotuner trial
+constexpr int TUNE_ITERS = 48, TUNE_ITERS_MIN = 12;   // CG iterations of the largest sub-grid in one autotuner trial
+constexpr double TUNE_WORK = 750e3;                   // ... times its unknowns, between those
 namespace cg = cooperative_groups;
 
 // The group of threads that solves one sub-grid: a warp, a CTA, or a cluster of CTAs.
@@ -835,12 +836,15 @@ void PersistentUpscale::launch(cudaStream_t s, const SellPattern& P, const doubl
 // (256-thread CTAs and a 16384-unknown warp limit always measured slower on the 512-sub-grid
 // batch); sub-grids below 0 or 4096 unknowns (sides up to about 11 in the unit-cube batches) left
 // to single warps; and the sub-grids of at least half the largest one's unknowns solved by clusters
-// of 1 (none), 2 or 4 CTAs.  Each candidate runs TUNE_ITERS iterations of the largest sub-grid, of the
+// of 1 (none), 2 or 4 CTAs.  Each candidate runs some iterations of the largest sub-grid, of the
 // others fewer in proportion to their sides, as whole solves do, after one warm-up launch; the fastest is kept
-// for the batch shape (192 sub-grids of 5 to 17 cells a side: clusters of 4 and 1024 threads, 44.6 ms; trials of
-// eight iterations of each took clusters of 2, 49.7, and of 16 weighted ones 512 threads, 49.3).  Warp items are
-// not tried further once they took half as long again as the same schedule without them.  A cluster shape that cannot be
-// resident on this GPU is skipped.
+// for the batch shape (192 sub-grids of 5 to 17 cells a side, 48 iterations: clusters of 4 and 1024 threads,
+// 44.6 ms; trials of eight iterations of each took clusters of 2, 49.7, and of 16 weighted ones 512 threads,
+// 49.3).  Large sub-grids, whose iterations take longer, get fewer (TUNE_WORK), so that a batch solved once does
+// not pay more for the trials than they can give (128 sub-grids of 8 to 32 cells a side: trials 227 ms of a first
+// call of 1.14 s, with 48 iterations 700 ms of 1.65 s, for 0.46 s a call either way).
+// Warp items are not tried further once they took half as long again as the same schedule without them.  A
+// cluster shape that cannot be resident on this GPU is skipped.
 UpscaleSchedule PersistentUpscale::tune(cudaStream_t s, const SellPattern& P, const double* val, const float* val32,
                                         const std::vector<int>& rg, const int* ranges_d, const double* b3, double* x3)
 {
@@ -857,6 +861,7 @@ UpscaleSchedule PersistentUpscale::tune(cudaStream_t s, const SellPattern& P, co
         auto it = tune_cache().find(key);
         if (it != tune_cache().end()) return it->second;
     }
+    const int iters = std::clamp(int(TUNE_WORK / double(std::max(largest, 1LL))), TUNE_ITERS_MIN, TUNE_ITERS);
     static const bool debug = std::getenv("PORSOL_DEBUG_UPSCALE") != nullptr;
     cudaEvent_t e0, e1;
     PORSOL_CUDA(cudaEventCreate(&e0));
@@ -879,11 +884,11 @@ UpscaleSchedule PersistentUpscale::tune(cudaStream_t s, const SellPattern& P, co
                         c.tuned = true;
                         try {
                             if (!warmed) {
-                                launch(s, P, val, val32, ranges_d, b3, x3, 0.0, 0.0, TUNE_ITERS, c, false, int(largest));
+                                launch(s, P, val, val32, ranges_d, b3, x3, 0.0, 0.0, iters, c, false, int(largest));
                                 warmed = true;
                             }
                             PORSOL_CUDA(cudaEventRecord(e0, s));
-                            launch(s, P, val, val32, ranges_d, b3, x3, 0.0, 0.0, TUNE_ITERS, c, false, int(largest));
+                            launch(s, P, val, val32, ranges_d, b3, x3, 0.0, 0.0, iters, c, false, int(largest));
                         } catch (const Error& e) {
                             if (e.code != PORSOL_ERR_BAD_ARG) throw;
                             continue;   // cluster shape not resident here
