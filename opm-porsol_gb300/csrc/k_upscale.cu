@@ -35,8 +35,7 @@ namespace {
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int UP_MAX_THREADS = 1024;
 constexpr int UP_MAX_WARPS = UP_MAX_THREADS / 32;
-constexpr int TUNE_ITERS = 48, TUNE_ITERS_MIN = 12;   // CG iterations of the largest sub-grid in one autotuner trial
-constexpr double TUNE_WORK = 750e3;                   // ... times its unknowns, between those
+constexpr int TUNE_ITERS = 48;   // CG iterations of the largest sub-grid in one autotuner trial
 namespace cg = cooperative_groups;
 
 // The group of threads that solves one sub-grid: a warp, a CTA, or a cluster of CTAs.
@@ -832,19 +831,18 @@ void PersistentUpscale::launch(cudaStream_t s, const SellPattern& P, const doubl
     PORSOL_COUNT_LAUNCH();
 }
 
-// Candidate schedules: both vector layouts; CTAs of 512 or 1024 threads for the CTA items
-// (256-thread CTAs and a 16384-unknown warp limit always measured slower on the 512-sub-grid
-// batch); sub-grids below 0 or 4096 unknowns (sides up to about 11 in the unit-cube batches) left
-// to single warps; and the sub-grids of at least half the largest one's unknowns solved by clusters
-// of 1 (none), 2 or 4 CTAs.  Each candidate runs some iterations of the largest sub-grid, of the
-// others fewer in proportion to their sides, as whole solves do, after one warm-up launch; the fastest is kept
-// for the batch shape (192 sub-grids of 5 to 17 cells a side, 48 iterations: clusters of 4 and 1024 threads,
-// 44.6 ms; trials of eight iterations of each took clusters of 2, 49.7, and of 16 weighted ones 512 threads,
-// 49.3).  Large sub-grids, whose iterations take longer, get fewer (TUNE_WORK), so that a batch solved once does
-// not pay more for the trials than they can give (128 sub-grids of 8 to 32 cells a side: trials 227 ms of a first
-// call of 1.14 s, with 48 iterations 700 ms of 1.65 s, for 0.46 s a call either way).
-// Warp items are not tried further once they took half as long again as the same schedule without them.  A
-// cluster shape that cannot be resident on this GPU is skipped.
+// Candidate schedules: CTAs of 512 or 1024 threads for the CTA items (256-thread CTAs always measured slower on
+// the 512-sub-grid batch) and the sub-grids of at least half the largest one's unknowns solved by clusters of 1
+// (none), 2 or 4 CTAs; then, with the fastest of these, sub-grids below 4096 unknowns (sides up to about 11 in the
+// unit-cube batches) left to single warps, and the other vector layout.  Each runs TUNE_ITERS iterations of the
+// largest sub-grid, of the others fewer in proportion to their sides, as whole solves do, after one warm-up launch;
+// the fastest is kept for the batch shape.  A cluster shape that cannot be resident on this GPU is skipped.
+// Trials of few iterations misjudge: their start and last replacement weigh more than in a solve, most for the
+// small sub-grids.  192 sub-grids of 5 to 17 cells a side: 48 weighted iterations take clusters of 4 and 1024
+// threads, 44.6 ms, 16 take 512 threads, 49.3, eight of each took clusters of 2, 49.7; 512 of 8 to 32: 48 take
+// clusters of 2, 922 ms, or none, 1035 (a tie in the trials), 12 to 32 always none.  All combinations of the four
+// choices, 14 to 24 trials, picked none faster, and a batch solved once paid for them: first call on 128
+// sub-grids of 8 to 32 cells a side 1.65 s, with these eight 1.13.
 UpscaleSchedule PersistentUpscale::tune(cudaStream_t s, const SellPattern& P, const double* val, const float* val32,
                                         const std::vector<int>& rg, const int* ranges_d, const double* b3, double* x3)
 {
@@ -861,52 +859,52 @@ UpscaleSchedule PersistentUpscale::tune(cudaStream_t s, const SellPattern& P, co
         auto it = tune_cache().find(key);
         if (it != tune_cache().end()) return it->second;
     }
-    const int iters = std::clamp(int(TUNE_WORK / double(std::max(largest, 1LL))), TUNE_ITERS_MIN, TUNE_ITERS);
     static const bool debug = std::getenv("PORSOL_DEBUG_UPSCALE") != nullptr;
     cudaEvent_t e0, e1;
     PORSOL_CUDA(cudaEventCreate(&e0));
     PORSOL_CUDA(cudaEventCreate(&e1));
     UpscaleSchedule best;
-    float best_ms = 1e30f, cta_ms = 1e30f;
-    bool warmed = false, warps = true;
+    float best_ms = 1e30f;
+    bool warmed = false;
+    auto trial = [&](const UpscaleSchedule& c) {
+        auto run = [&] { launch(s, P, val, val32, ranges_d, b3, x3, 0.0, 0.0, TUNE_ITERS, c, false, int(largest)); };
+        try {
+            if (!warmed) run();
+            warmed = true;
+            PORSOL_CUDA(cudaEventRecord(e0, s));
+            run();
+        } catch (const Error& e) {
+            if (e.code != PORSOL_ERR_BAD_ARG) throw;
+            return;   // cluster shape not resident here
+        }
+        PORSOL_CUDA(cudaEventRecord(e1, s));
+        PORSOL_CUDA(cudaEventSynchronize(e1));
+        float ms = 0.f;
+        PORSOL_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+        if (debug)
+            std::fprintf(stderr, "[upscale] trial cluster=%d layout=%d cta=%d warp_below=%d: %.3f ms\n", c.cluster, c.layout,
+                         c.cta_threads, c.warp_max_unknowns, ms);
+        if (ms < best_ms) {
+            best_ms = ms;
+            best = c;
+        }
+    };
     try {
         for (int cluster : {1, 2, 4})
-            for (int layout : {0, 1})
-                for (int threads : {512, 1024})
-                    for (int wmax : {0, 4096}) {
-                        if (wmax > 0 && !warps) continue;
-                        UpscaleSchedule c;
-                        c.cta_threads = threads;
-                        c.warp_max_unknowns = wmax;
-                        c.layout = layout;
-                        c.cluster = cluster;
-                        c.cluster_min_unknowns = cluster > 1 ? int(largest / 2) : 0;
-                        c.tuned = true;
-                        try {
-                            if (!warmed) {
-                                launch(s, P, val, val32, ranges_d, b3, x3, 0.0, 0.0, iters, c, false, int(largest));
-                                warmed = true;
-                            }
-                            PORSOL_CUDA(cudaEventRecord(e0, s));
-                            launch(s, P, val, val32, ranges_d, b3, x3, 0.0, 0.0, iters, c, false, int(largest));
-                        } catch (const Error& e) {
-                            if (e.code != PORSOL_ERR_BAD_ARG) throw;
-                            continue;   // cluster shape not resident here
-                        }
-                        PORSOL_CUDA(cudaEventRecord(e1, s));
-                        PORSOL_CUDA(cudaEventSynchronize(e1));
-                        float ms = 0.f;
-                        PORSOL_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-                        if (debug)
-                            std::fprintf(stderr, "[upscale] trial cluster=%d layout=%d cta=%d warp_below=%d: %.3f ms\n",
-                                         cluster, layout, threads, wmax, ms);
-                        if (ms < best_ms) {
-                            best_ms = ms;
-                            best = c;
-                        }
-                        if (wmax == 0) cta_ms = ms;
-                        else if (ms > 1.5f * cta_ms) warps = false;
-                    }
+            for (int threads : {512, 1024}) {
+                UpscaleSchedule c;
+                c.cta_threads = threads;
+                c.cluster = cluster;
+                c.cluster_min_unknowns = cluster > 1 ? int(largest / 2) : 0;
+                c.tuned = true;
+                trial(c);
+            }
+        UpscaleSchedule c = best;
+        c.warp_max_unknowns = 4096;
+        trial(c);
+        c = best;
+        c.layout = 0;
+        trial(c);
     } catch (...) {
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
